@@ -11,6 +11,7 @@
 
 #include "common.cuh"
 #include "product.cuh"
+#include "series.cuh"
 
 namespace rpyb {
 
@@ -490,11 +491,22 @@ RPYB_API int rpyb_ft_exp(int dtype, int32_t width, int32_t depth, int64_t batch,
         rows.batch = batch;
         return launch_product(dtype, g, sp, rows, s);
     }
+    // the workspace is asked for also where the series runs in one launch, so
+    // that its documented size and failures do not depend on the shape
     Scratch scratch(workspace, workspace_bytes, s);
     void* tmp = nullptr;
     if (M > 1 &&
         (rc = scratch.get((size_t)(batch * g.size()) * elem_size(dtype), &tmp)))
         return rc;
+    if (series_available(g, M)) {
+        SeriesRows r;
+        r.out = out;
+        r.ld_out = ld_out;
+        r.arg = arg;
+        r.ld_arg = ld_arg;
+        r.batch = batch;
+        return launch_series(dtype, kSeriesExp, g, M, M, r, s);
+    }
     return horner_exp_like(dtype, g, M, batch, out, ld_out, out, ld_out, arg, ld_arg, nullptr,
                            0, tmp, s);
 }
@@ -525,6 +537,17 @@ RPYB_API int rpyb_ft_fmexp(int dtype, int32_t width, int32_t depth, int64_t batc
     Scratch scratch(workspace, workspace_bytes, s);
     void* tmp = nullptr;
     if (M > 1 && (rc = scratch.get((size_t)(batch * g.size()) * es, &tmp))) return rc;
+    if (series_available(g, M)) {
+        SeriesRows r;
+        r.out = out;
+        r.ld_out = ld_out;
+        r.arg = exponent;
+        r.ld_arg = ld_exp;
+        r.mult = multiplier;
+        r.ld_mult = ld_mul;
+        r.batch = batch;
+        return launch_series(dtype, kSeriesFmexp, g, M, M, r, s);
+    }
     return horner_exp_like(dtype, g, M, batch, out, ld_out, multiplier, ld_mul, exponent, ld_exp,
                            multiplier, ld_mul, tmp, s);
 }
@@ -551,6 +574,15 @@ RPYB_API int rpyb_ft_log(int dtype, int32_t width, int32_t depth, int64_t batch,
     void* base = nullptr;
     const int nbuf = (dtype == RPYB_F64) ? 1 : 3;
     if ((rc = scratch.get((size_t)(nbuf * batch * T) * 8, &base))) return rc;
+    if (M >= 1 && series_available(g, M)) {
+        SeriesRows r;
+        r.out = out;
+        r.ld_out = ld_out;
+        r.arg = arg;
+        r.ld_arg = ld_arg;
+        r.batch = batch;
+        return launch_series(dtype, kSeriesLog, g, M, Ma, r, s);
+    }
     double* tmp = static_cast<double*>(base);
     double* out64 = static_cast<double*>(out);
     const double* arg64 = static_cast<const double*>(arg);
@@ -560,7 +592,9 @@ RPYB_API int rpyb_ft_log(int dtype, int32_t width, int32_t depth, int64_t batch,
         double* o64 = tmp + 2 * batch * T;
         if ((rc = launch_convert_rows(RPYB_F64, a64, T, RPYB_F32, arg, ld_arg, T, batch, s)))
             return rc;
-        if ((rc = launch_convert_rows(RPYB_F64, o64, T, RPYB_F32, out, ld_out, T, batch, s)))
+        // of out's rows only the scalar is read, and what lies above level M kept
+        const int64_t keep = M < depth ? T : 1;
+        if ((rc = launch_convert_rows(RPYB_F64, o64, T, RPYB_F32, out, ld_out, keep, batch, s)))
             return rc;
         arg64 = a64;
         out64 = o64;
