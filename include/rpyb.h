@@ -372,6 +372,28 @@ RPYB_API int rpyb_sparse_map(int dtype, int64_t n_rows, int64_t n_cols, int64_t 
                              int64_t ld_y, int64_t ld_x, double scale, void* stream);
 
 /*
+ * Packs a CSR matrix (host arrays) for rpyb_sparse_map_packed: returns the
+ * block's size in bytes, writes the block when `block` is not null (of at
+ * least that many bytes), and its three counts to layout.  Entries whose
+ * column lies outside [0, n_cols) are left out.  RPYB_E_UNSUPPORTED when the
+ * matrix has over 2^20 columns or over 4096 distinct values.  The caller
+ * copies the block to the device.
+ */
+RPYB_API int64_t rpyb_sparse_pack(int64_t n_rows, int64_t n_cols, const int64_t* indptr,
+                                  const int64_t* indices, const double* values, void* block,
+                                  int64_t block_bytes, int64_t* layout);
+
+/*
+ * y[b] = scale * M x[b], or y[b] += with accumulate, for a packed matrix
+ * (block on the device, layout on the host); otherwise as rpyb_sparse_map,
+ * whose terms and order it keeps.
+ */
+RPYB_API int rpyb_sparse_map_packed(int dtype, int64_t n_rows, int64_t n_cols, int64_t batch,
+                                    const void* block, const int64_t* layout, void* y,
+                                    const void* x, int64_t ld_y, int64_t ld_x, double scale,
+                                    int accumulate, void* stream);
+
+/*
  * Batched tensor -> Lie (Hall coordinates, rbracketing / degree) and
  * Lie -> tensor maps with the maps kept on the device (uploaded once per
  * device and shape).  Both assign their output rows.

@@ -100,6 +100,26 @@ class SparseMatrix:
             )
         return self._dev[key]
 
+    def device_packed(self, device):
+        """(block, layout) of ``rpyb_sparse_pack`` on the device, or None where the matrix
+        cannot be packed; made once, like ``device_arrays``."""
+        key = ("packed", str(device))
+        if key not in self._dev:
+            data = np.ascontiguousarray(self.data, dtype=np.float64)
+            layout = (ctypes.c_int64 * 3)()
+            args = (*self.shape, self.indptr.ctypes.data, self.indices.ctypes.data,
+                    data.ctypes.data)
+            size = int(_lib.lib.rpyb_sparse_pack(*args, None, 0, layout))
+            if size == _lib.E_UNSUPPORTED:
+                self._dev[key] = None
+            else:
+                _lib.check(min(size, 0))
+                block = np.empty(max(size, 1), dtype=np.uint8)
+                _lib.check(min(0, int(_lib.lib.rpyb_sparse_pack(*args, block.ctypes.data, size,
+                                                                layout))))
+                self._dev[key] = (torch.from_numpy(block).to(device), layout)
+        return self._dev[key]
+
 
 class LieBasis:
     """Hall basis with RoughPy's greedy construction.
@@ -386,12 +406,21 @@ def dense_ft_adjoint_left_mul(out, operator, argument, basis, out_depth=-1, lhs_
 
 
 # ------------------------------------------------------------------ Lie maps
-def _apply_csr(o: _Arg, a: _Arg, matrix: SparseMatrix, scale):
-    ptr, idx, val = matrix.device_arrays(o.t.device)
+def _apply_csr(o: _Arg, a: _Arg, matrix: SparseMatrix, scale, accumulate=True):
     rows, cols = matrix.shape
     if o.n < rows or a.n < cols:
         raise ValueError("array sizes do not match the map")
     s = 1.0 if scale is None else float(scale)
+    packed = matrix.device_packed(o.t.device)
+    if packed is not None:
+        block, layout = packed
+        _lib.check(_lib.lib.rpyb_sparse_map_packed(
+            o.dtype_code, rows, cols, o.batch, block.data_ptr(), layout, o.ptr(), a.ptr(), o.n,
+            a.n, s, int(accumulate), _stream_ptr(o.t)))
+        return
+    if not accumulate:
+        o.rows[:, :rows].zero_()
+    ptr, idx, val = matrix.device_arrays(o.t.device)
     _lib.check(_lib.lib.rpyb_sparse_map(o.dtype_code, rows, cols, o.batch, ptr.data_ptr(),
                                         idx.data_ptr(), val.data_ptr(), o.ptr(), a.ptr(), o.n,
                                         a.n, s, _stream_ptr(o.t)))
@@ -412,4 +441,14 @@ def dense_tensor_to_lie(out, arg, t2l_matrix, lie_basis, tensor_basis, scale_fac
     a = _Arg(arg, "arg", 1, False, o.t.device)
     _check_same(o, a)
     _apply_csr(o, a, t2l_matrix, scale_factor)
+    o.finish()
+
+
+def lie_map_into(out, arg, matrix: SparseMatrix, scale_factor=None):
+    """out <- scale * matrix(arg): the maps above without reading ``out``, whose columns
+    past the matrix's rows are left alone."""
+    o = _Arg(out, "out", 1, True)
+    a = _Arg(arg, "arg", 1, False, o.t.device)
+    _check_same(o, a)
+    _apply_csr(o, a, matrix, scale_factor, accumulate=False)
     o.finish()

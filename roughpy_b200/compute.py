@@ -66,6 +66,14 @@ def _zeros_like(data, n=None):
     return np.zeros(shape, dtype=data.dtype)
 
 
+def _empty_like(data, n=None):
+    """An uninitialised result for a call that writes all of it."""
+    shape = data.shape if n is None else (*data.shape[:-1], n)
+    if isinstance(data, torch.Tensor):
+        return torch.empty(shape, dtype=data.dtype, device=data.device)
+    return np.empty(shape, dtype=data.dtype)
+
+
 def _float_dtype(data):
     dt = data.dtype
     if dt in (np.float32, np.float64, torch.float32, torch.float64):
@@ -145,9 +153,9 @@ def lie_to_tensor(arg: Lie, tensor_basis: TensorBasis | None = None,
     """Embed a Lie element (Hall basis coordinates) in the tensor algebra."""
     l2t = arg.basis.get_l2t_matrix(np.float64)
     tensor_basis = tensor_basis or TensorBasis(arg.basis.width, arg.basis.depth)
-    result = _zeros_like(arg.data, tensor_basis.size())
-    _internals.dense_lie_to_tensor(result, arg.data, l2t, arg.basis, tensor_basis,
-                                   scale_factor=scale_factor)
+    n = tensor_basis.size()
+    result = (_empty_like if n == l2t.shape[0] else _zeros_like)(arg.data, n)
+    _internals.lie_map_into(result, arg.data, l2t, scale_factor)
     return FreeTensor(result, tensor_basis)
 
 
@@ -156,7 +164,7 @@ def tensor_to_lie(arg: FreeTensor, lie_basis: LieBasis | None = None,
     """Project a free tensor onto the Lie algebra (Dynkin map in the Hall basis)."""
     lie_basis = lie_basis or LieBasis(arg.basis.width, arg.basis.depth)
     t2l = lie_basis.get_t2l_matrix(np.float64)
-    result = _zeros_like(arg.data, lie_basis.size())
-    _internals.dense_tensor_to_lie(result, arg.data, t2l, lie_basis, arg.basis,
-                                   scale_factor=scale_factor)
+    n = lie_basis.size()
+    result = (_empty_like if n == t2l.shape[0] else _zeros_like)(arg.data, n)
+    _internals.lie_map_into(result, arg.data, t2l, scale_factor)
     return Lie(result, lie_basis)

@@ -100,10 +100,8 @@ RPYB_API int rpyb_cbh(int32_t width, int32_t depth, int64_t n_lists, const int64
         if (!chain && (rc = unit_rows(RPYB_F64, acc, T, T, nullptr, m, s))) return rc;
         if (nf > 0) {
             // exp(l2t(x)) for every item of the chunk
-            RPYB_CUDA(cudaMemsetAsync(emb, 0, (size_t)(nf * T * 8), s));
-            if ((rc = rpyb_sparse_map(RPYB_F64, T, L, nf, maps->l2t_ptr, maps->l2t_idx,
-                                      maps->l2t_val, emb, lies + f0 * ld_lies, T, ld_lies, 1.0,
-                                      s)) ||
+            if ((rc = lie_embed(RPYB_F64, g, *maps, nf, emb, T, lies + f0 * ld_lies, ld_lies,
+                                s)) ||
                 (rc = rpyb_ft_exp(RPYB_F64, width, depth, nf, ex, emb, T, T, -1, exp_mem, exp_b,
                                   s)))
                 return rc;

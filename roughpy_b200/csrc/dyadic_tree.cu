@@ -404,11 +404,7 @@ RPYB_API int rpyb_dyadic_build(int mode, int32_t width, int32_t depth, int32_t r
         void* emb = mem;
         void* ex = static_cast<char*>(mem) + emb_bytes;
         void* wsp = static_cast<char*>(mem) + 2 * emb_bytes;
-        // the sparse map accumulates: clear its output first
-        if (cudaMemsetAsync(emb, 0, (size_t)(n_events * T * es), s) != cudaSuccess)
-            return fail_release(cuda_fail(cudaGetLastError(), "cudaMemsetAsync"));
-        if ((rc = rpyb_sparse_map(mode, T, lie_dim, n_events, maps->l2t_ptr, maps->l2t_idx,
-                                  maps->l2t_val, emb, rows, T, lie_dim, 1.0, s)) ||
+        if ((rc = lie_embed(mode, g, *maps, n_events, emb, T, rows, lie_dim, s)) ||
             (rc = rpyb_ft_exp(mode, width, depth, n_events, ex, emb, T, T, -1, wsp,
                               (size_t)std::max<int64_t>(ws, 1), s)) ||
             (rc = unit_rows(mode, t->nodes, T, T, nullptr, n_leaves, s)))

@@ -154,10 +154,7 @@ RPYB_API int rpyb_piecewise_query(int32_t width, int32_t depth, int64_t n_pieces
             scaled_rows_kernel<<<blocks, 256, 0, s>>>(lrows, piece_lies, ld_lies, d_piece, d_mult, L,
                                                       nf);
             RPYB_CUDA(cudaGetLastError());
-            // the sparse map accumulates: clear its output first
-            RPYB_CUDA(cudaMemsetAsync(emb, 0, (size_t)(nf * T * 8), s));
-            if ((rc = rpyb_sparse_map(RPYB_F64, T, L, nf, maps->l2t_ptr, maps->l2t_idx,
-                                      maps->l2t_val, emb, lrows, T, L, 1.0, s)) ||
+            if ((rc = lie_embed(RPYB_F64, g, *maps, nf, emb, T, lrows, L, s)) ||
                 (rc = rpyb_ft_exp(RPYB_F64, width, depth, nf, ex, emb, T, T, -1, exp_mem, exp_b,
                                   s)))
                 return rc;

@@ -63,7 +63,7 @@ int upload(const std::vector<E>& h, const E** out)
     return RPYB_OK;
 }
 
-// The packed form of a CSR map for lie_project_kernel: rows sorted by entry
+// The packed form of the t2l map for the chain kernel's projection: rows sorted by entry
 // count (most first, stably) in groups of 32, each group padded to its
 // longest row with zero entries and stored lane-interleaved (entry j of lane
 // l at 32 j + l from the group's offset); an entry is 8 * column | value id
@@ -129,7 +129,8 @@ bool pack_csr(const std::vector<int64_t>& hp, const std::vector<int64_t>& hi,
 }
 
 int upload_csr(const Geometry& g, int which, int64_t n_rows, const int64_t** ptr,
-               const int64_t** idx, const double** val, LieMapsDev* packed_into = nullptr)
+               const int64_t** idx, const double** val, PackedMap* packed,
+               LieMapsDev* packed_into = nullptr)
 {
     const int64_t nnz = rpyb_lie_map_csr(g.width, g.depth, which, nullptr, nullptr, nullptr);
     if (nnz < 0) return (int)nnz;
@@ -137,6 +138,14 @@ int upload_csr(const Geometry& g, int which, int64_t n_rows, const int64_t** ptr
     std::vector<double> hv(std::max<int64_t>(nnz, 1));
     const int64_t got = rpyb_lie_map_csr(g.width, g.depth, which, hp.data(), hi.data(), hv.data());
     if (got < 0) return (int)got;
+    std::vector<unsigned char> block;
+    if (pack_map(n_rows, which == 0 ? rpyb_lie_basis_size(g.width, g.depth) : g.size(), hp.data(),
+                 hi.data(), hv.data(), *packed, block)) {
+        const unsigned char* d_block = nullptr;
+        const int rc = upload(block, &d_block);
+        if (rc) return rc;
+        packed->block = d_block;
+    }
     if (packed_into) {
         std::vector<uint32_t> goff, ent, perm;
         std::vector<double> tab;
@@ -203,107 +212,6 @@ int upload_async(void* dst, const void* src, size_t bytes, cudaStream_t s)
     return RPYB_OK;
 }
 
-
-// ------------------------------------------------------------------------
-// Tensor -> Lie projection with the packed map held in shared memory.  One
-// persistent block per SM loads the map (column and value id per entry, the
-// distinct values, the group offsets) once; for each of its rows of x it
-// copies the row into shared memory with coalesced loads, and every warp
-// computes groups of 32 Lie coordinates from shared memory, one per lane.
-// The compact entries are what makes this pay: as (int64, float64) pairs the
-// map is larger than a row of x and its gathers go to L2 for every row.  The
-// lane-interleaved groups make a warp's entry reads consecutive words and
-// give its lanes equal trip counts.
-constexpr int kProjThreads = 1024;
-constexpr int64_t kProjSmemLimit = 220 * 1024;
-
-struct ProjArgs {
-    int64_t n_cols = 0, slots = 0, groups = 0, ntab = 0, batch = 0;
-    int64_t ld_y = 0, ld_x = 0;
-    const uint32_t* goff = nullptr;
-    const uint32_t* ent = nullptr;
-    const uint32_t* perm = nullptr;
-    const double* tab = nullptr;
-};
-
-template <typename T>
-size_t proj_smem_bytes(const ProjArgs& a)
-{
-    const int64_t xs_bytes = (a.n_cols * (int64_t)sizeof(T) + 15) / 16 * 16;
-    return (size_t)(xs_bytes + a.ntab * 8 + (a.groups + 1) * 4 + a.slots * 4);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kProjThreads, 1)
-lie_project_kernel(const ProjArgs a, T* __restrict__ y, const T* __restrict__ x)
-{
-    // the row first, so an entry's byte offset addresses its word directly
-    extern __shared__ __align__(16) unsigned char proj_smem[];
-    T* xs = reinterpret_cast<T*>(proj_smem);
-    double* tab = reinterpret_cast<double*>(proj_smem + (a.n_cols * (int64_t)sizeof(T) + 15) / 16 * 16);
-    uint32_t* goff = reinterpret_cast<uint32_t*>(tab + a.ntab);
-    uint32_t* ent = goff + a.groups + 1;
-    const int tid = (int)threadIdx.x;
-    const int lane = tid & 31, warp = tid >> 5, nwarps = (int)blockDim.x >> 5;
-    for (int64_t i = tid; i < a.ntab; i += blockDim.x) tab[i] = a.tab[i];
-    for (int64_t i = tid; i <= a.groups; i += blockDim.x) goff[i] = a.goff[i];
-    for (int64_t i = tid; i < a.slots; i += blockDim.x) ent[i] = a.ent[i];
-    constexpr int kU = 8;
-    for (int64_t b = blockIdx.x; b < a.batch; b += gridDim.x) {
-        __syncthreads();   // the map is loaded; the previous row's gathers are done
-        const T* xr = x + b * a.ld_x;
-        // eight independent loads in flight per thread
-        for (int64_t c0 = tid; c0 < a.n_cols; c0 += kU * blockDim.x) {
-            T v[kU];
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int64_t c = c0 + (int64_t)u * blockDim.x;
-                v[u] = c < a.n_cols ? __ldg(xr + c) : T(0);
-            }
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int64_t c = c0 + (int64_t)u * blockDim.x;
-                if (c < a.n_cols) xs[c] = v[u];
-            }
-        }
-        __syncthreads();
-        if (b + gridDim.x < a.batch) {
-            // the block's next row into L2 while this one is computed
-            const char* nx = reinterpret_cast<const char*>(x + (b + gridDim.x) * a.ld_x);
-            const int64_t bytes = a.n_cols * (int64_t)sizeof(T);
-            for (int64_t l = (int64_t)tid * 128; l < bytes; l += (int64_t)blockDim.x * 128)
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + l));
-        }
-        T* yr = y + b * a.ld_y;
-        for (int64_t g = warp; g < a.groups; g += nwarps) {
-            double acc = 0.0;
-            const uint32_t e1 = goff[g + 1];
-#pragma unroll 4
-            for (uint32_t k = goff[g] + lane; k < e1; k += 32) {
-                const uint32_t w = ent[k];
-                const uint32_t off = w & 0x7ffffu;   // 8 * column
-                const T xv = *reinterpret_cast<const T*>(
-                    proj_smem + (sizeof(T) == 8 ? off : off >> 1));
-                acc = fma(tab[w >> 19], (double)xv, acc);
-            }
-            const uint32_t row = __ldg(a.perm + g * 32 + lane);
-            if (row != 0xffffffffu) yr[row] = (T)acc;
-        }
-    }
-}
-
-template <typename T>
-int launch_lie_project(const ProjArgs& a, void* y, const void* x, cudaStream_t s)
-{
-    const size_t smem = proj_smem_bytes<T>(a);
-    RPYB_CUDA(cudaFuncSetAttribute(lie_project_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem));
-    const unsigned blocks = (unsigned)std::min<int64_t>(a.batch, 148);
-    lie_project_kernel<T><<<blocks, kProjThreads, smem, s>>>(a, static_cast<T*>(y),
-                                                             static_cast<const T*>(x));
-    RPYB_CUDA(cudaGetLastError());
-    return RPYB_OK;
-}
 
 // ------------------------------------------------------------------------
 // Fused chain products: acc[q] <- src[r_0] * src[r_1] * ... (the unit for an
@@ -824,8 +732,8 @@ int lie_maps_device(const Geometry& g, const LieMapsDev** out)
     e.depth = g.depth;
     e.lie_dim = lie_dim;
     int rc;
-    if ((rc = upload_csr(g, 0, g.size(), &e.l2t_ptr, &e.l2t_idx, &e.l2t_val)) ||
-        (rc = upload_csr(g, 1, lie_dim, &e.t2l_ptr, &e.t2l_idx, &e.t2l_val, &e)))
+    if ((rc = upload_csr(g, 0, g.size(), &e.l2t_ptr, &e.l2t_idx, &e.l2t_val, &e.l2t)) ||
+        (rc = upload_csr(g, 1, lie_dim, &e.t2l_ptr, &e.t2l_idx, &e.t2l_val, &e.t2l, &e)))
         return rc;
     entries[n_entries] = e;
     *out = &entries[n_entries++];
@@ -926,29 +834,26 @@ int lie_project(int dtype, const Geometry& g, const LieMapsDev& maps, int64_t m,
 {
     if (m <= 0) return RPYB_OK;
     const int64_t T = g.size(), L = maps.lie_dim;
-    ProjArgs a;
-    a.n_cols = T;
-    a.slots = maps.t2l_slots;
-    a.groups = maps.t2l_groups;
-    a.ntab = maps.t2l_ntab;
-    a.batch = m;
-    a.ld_y = ld_lie;
-    a.ld_x = ld_x;
-    a.goff = maps.t2l_goff;
-    a.ent = maps.t2l_ent;
-    a.perm = maps.t2l_perm;
-    a.tab = maps.t2l_tab;
-    if (maps.t2l_ent) {
-        if (dtype == RPYB_F64 && proj_smem_bytes<double>(a) <= (size_t)kProjSmemLimit)
-            return launch_lie_project<double>(a, lie, x, s);
-        if (dtype == RPYB_F32 && proj_smem_bytes<float>(a) <= (size_t)kProjSmemLimit)
-            return launch_lie_project<float>(a, lie, x, s);
-    }
+    if (maps.t2l.block)
+        return launch_packed_map(dtype, maps.t2l, m, lie, ld_lie, x, ld_x, 1.0, false, s);
     // the sparse map accumulates: clear its outputs first
     const size_t es = dtype == RPYB_F64 ? 8 : 4;
     RPYB_CUDA(cudaMemset2DAsync(lie, (size_t)ld_lie * es, 0, (size_t)L * es, (size_t)m, s));
     return rpyb_sparse_map(dtype, L, T, m, maps.t2l_ptr, maps.t2l_idx, maps.t2l_val, lie, x, ld_lie,
                            ld_x, 1.0, s);
+}
+
+int lie_embed(int dtype, const Geometry& g, const LieMapsDev& maps, int64_t m, void* x,
+              int64_t ld_x, const void* lie, int64_t ld_lie, cudaStream_t s)
+{
+    if (m <= 0) return RPYB_OK;
+    const int64_t T = g.size(), L = maps.lie_dim;
+    if (maps.l2t.block)
+        return launch_packed_map(dtype, maps.l2t, m, x, ld_x, lie, ld_lie, 1.0, false, s);
+    const size_t es = dtype == RPYB_F64 ? 8 : 4;
+    RPYB_CUDA(cudaMemset2DAsync(x, (size_t)ld_x * es, 0, (size_t)T * es, (size_t)m, s));
+    return rpyb_sparse_map(dtype, T, L, m, maps.l2t_ptr, maps.l2t_idx, maps.l2t_val, x, lie, ld_x,
+                           ld_lie, 1.0, s);
 }
 
 size_t finish_scratch_bytes(const Geometry& g, int64_t lie_dim, int64_t n)
@@ -1001,9 +906,7 @@ int finish_queries(const Geometry& g, const LieMapsDev& maps, int64_t m, double*
     }
     if (out_sig) {
         // algebra/src/context.cpp:156-159: exp(lie_to_tensor(log_signature))
-        RPYB_CUDA(cudaMemsetAsync(tmp, 0, (size_t)(m * T * 8), s));
-        if ((rc = rpyb_sparse_map(RPYB_F64, T, L, m, maps.l2t_ptr, maps.l2t_idx, maps.l2t_val, tmp,
-                                  lie, T, ld_lie, 1.0, s)) ||
+        if ((rc = lie_embed(RPYB_F64, g, maps, m, tmp, T, lie, ld_lie, s)) ||
             (rc = rpyb_ft_exp(RPYB_F64, g.width, g.depth, m, out_sig, tmp, ld_sig, T, -1, ws, wsb,
                               s)))
             return rc;
@@ -1088,12 +991,8 @@ RPYB_API int rpyb_lie_to_tensor(int dtype, int32_t width, int32_t depth, int64_t
     if (ld_out < g.size() || ld_arg < L) return fail(RPYB_E_INVALID, "row stride too small");
     const LieMapsDev* maps = nullptr;
     if ((rc = lie_maps_device(g, &maps))) return rc;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const size_t es = dtype == RPYB_F64 ? 8 : 4;
-    RPYB_CUDA(cudaMemset2DAsync(out, (size_t)ld_out * es, 0, (size_t)g.size() * es, (size_t)batch,
-                                s));
-    return rpyb_sparse_map(dtype, g.size(), L, batch, maps->l2t_ptr, maps->l2t_idx, maps->l2t_val,
-                           out, arg, ld_out, ld_arg, 1.0, s);
+    return lie_embed(dtype, g, *maps, batch, out, ld_out, arg, ld_arg,
+                     static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "sparse_map.cuh"
 
 namespace rpyb {
 
@@ -22,7 +23,7 @@ struct LieMapsDev {
     const int64_t* t2l_ptr = nullptr;   // lie_dim rows x tensor_size
     const int64_t* t2l_idx = nullptr;
     const double* t2l_val = nullptr;
-    // t2l packed for the shared-memory projection kernel (null when a column
+    // t2l packed for the projection inside the chain kernel (null when a column
     // does not fit 16 bits or the number of distinct values 13 bits).  Rows sorted by
     // entry count, in groups of 32 (one per warp lane), each group padded to
     // its longest row; entry j of lane l of group g is t2l_ent[t2l_goff[g] +
@@ -34,6 +35,7 @@ struct LieMapsDev {
     const uint32_t* t2l_perm = nullptr;   // 32 * groups
     const double* t2l_tab = nullptr;
     int64_t t2l_slots = 0, t2l_groups = 0, t2l_ntab = 0;
+    PackedMap l2t, t2l;   // for launch_packed_map (block null: not packable)
 };
 int lie_maps_device(const Geometry& g, const LieMapsDev** out);
 
@@ -41,6 +43,10 @@ int lie_maps_device(const Geometry& g, const LieMapsDev** out);
 // both, float64 arithmetic)
 int lie_project(int dtype, const Geometry& g, const LieMapsDev& maps, int64_t m, void* lie,
                 int64_t ld_lie, const void* x, int64_t ld_x, cudaStream_t s);
+
+// x[b] <- l2t(lie[b]) for m rows (assigning, as above)
+int lie_embed(int dtype, const Geometry& g, const LieMapsDev& maps, int64_t m, void* x,
+              int64_t ld_x, const void* lie, int64_t ld_lie, cudaStream_t s);
 
 // rows idx[i] (or i) of `out` (stride ld) <- the unit tensor
 int unit_rows(int mode, void* out, int64_t ld, int64_t cols, const int64_t* idx, int64_t n,
