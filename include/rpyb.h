@@ -89,6 +89,14 @@ RPYB_API int rpyb_ft_fma(int dtype, int32_t width, int32_t depth, int64_t batch,
                          const int32_t* deg_bounds, void* stream);
 
 /*
+ * out[b] = lhs[b] (x) rhs[b]: rpyb_ft_fma without reading out.  Every level
+ * from out_min to out_max is written (zero where the bounds leave no term).
+ */
+RPYB_API int rpyb_ft_mul(int dtype, int32_t width, int32_t depth, int64_t batch, void* out,
+                         const void* lhs, const void* rhs, int64_t ld_out, int64_t ld_lhs,
+                         int64_t ld_rhs, const int32_t* deg_bounds, void* stream);
+
+/*
  * Row-gathered variant used by tree reductions: for i < n,
  *   out[out_idx[i]] (+)= lhs[lhs_idx[i]] (x) rhs[rhs_idx[i]]
  * with accumulate != 0 selecting += and 0 selecting =.  Index arrays are
@@ -190,6 +198,15 @@ RPYB_API int rpyb_ft_log(int dtype, int32_t width, int32_t depth, int64_t batch,
                          size_t workspace_bytes, void* stream);
 
 /*
+ * rpyb_ft_log of rows whose incoming scalar is zero, without reading out: the
+ * plain logarithm into a fresh array.
+ */
+RPYB_API int rpyb_ft_log_fresh(int dtype, int32_t width, int32_t depth, int64_t batch, void* out,
+                               const void* arg, int64_t ld_out, int64_t ld_arg,
+                               int32_t out_depth, int32_t arg_depth, void* workspace,
+                               size_t workspace_bytes, void* stream);
+
+/*
  * out[b] <- antipode(arg[b]): word reversal with sign (-1)^degree.
  * Replaces: roughpy_compute/dense/basic/free_tensor_antipode.hpp:50-100 via
  *           roughpy/compute/_src/dense_basic.cpp:244-330.
@@ -209,6 +226,12 @@ RPYB_API int rpyb_ft_adjoint_left_mul(int dtype, int32_t width, int32_t depth,
                                       const void* arg, int64_t ld_out, int64_t ld_op,
                                       int64_t ld_arg, const int32_t* deg,
                                       void* stream);
+
+/* out[b] = L*_{op[b]}(arg[b]) up to out_depth, without reading out. */
+RPYB_API int rpyb_ft_adjoint_left_mul_fresh(int dtype, int32_t width, int32_t depth,
+                                            int64_t batch, void* out, const void* op,
+                                            const void* arg, int64_t ld_out, int64_t ld_op,
+                                            int64_t ld_arg, const int32_t* deg, void* stream);
 
 /*
  * Batched path signatures: for each stream s, with increments rows

@@ -239,11 +239,17 @@ def _basis_wd(basis):
 class _Arg:
     """One array argument: a CUDA tensor view of shape (batch, n) plus writeback."""
 
-    def __init__(self, obj, name: str, need: int, writable: bool, device=None):
+    def __init__(self, obj, name: str, need: int, writable: bool, device=None, fresh=False):
         self.name = name
         self.obj = obj
         self.is_numpy = isinstance(obj, np.ndarray)
-        if self.is_numpy:
+        if self.is_numpy and fresh:
+            # wholly written by the call: nothing to copy to the device
+            if obj.dtype not in (np.float32, np.float64):
+                raise TypeError(f"{name}: unsupported dtype")
+            self.t = torch.empty(obj.shape, device=device or "cuda",
+                                 dtype=torch.float64 if obj.dtype == np.float64 else torch.float32)
+        elif self.is_numpy:
             if obj.dtype not in (np.float32, np.float64):
                 raise TypeError(f"{name}: unsupported dtype")
             host = np.ascontiguousarray(obj)
@@ -444,10 +450,54 @@ def dense_tensor_to_lie(out, arg, t2l_matrix, lie_basis, tensor_basis, scale_fac
     o.finish()
 
 
+# ----------------------------------------------------- into fresh results
+# The operations above on an ``out`` that they wholly write (its last axis has exactly
+# the tensor's size) and do not read.
+def ft_mul_into(out, lhs, rhs, basis, rhs_depth=-1):
+    """out <- lhs (x) rhs."""
+    w, d = _basis_wd(basis)
+    size = int(_lib.lib.rpyb_tensor_size(w, d))
+    o = _Arg(out, "out", size, True, fresh=True)
+    lh = _Arg(lhs, "lhs", size, False, o.t.device)
+    rh = _Arg(rhs, "rhs", size, False, o.t.device)
+    _check_same(o, lh, rh)
+    b = _lib.bounds(0, -1, 0, -1, 0, rhs_depth)
+    _lib.check(_lib.lib.rpyb_ft_mul(o.dtype_code, w, d, o.batch, o.ptr(), lh.ptr(), rh.ptr(),
+                                    o.n, lh.n, rh.n, b, _stream_ptr(o.t)))
+    o.finish()
+
+
+def ft_log_into(out, arg, basis):
+    """out <- log(arg), its scalar taken as zero."""
+    w, d = _basis_wd(basis)
+    size = int(_lib.lib.rpyb_tensor_size(w, d))
+    o = _Arg(out, "out", size, True, fresh=True)
+    a = _Arg(arg, "arg", size, False, o.t.device)
+    _check_same(o, a)
+    ws = _workspace(_lib.lib.rpyb_ft_log_workspace_size(o.dtype_code, w, d, o.batch), o.t.device)
+    _lib.check(_lib.lib.rpyb_ft_log_fresh(o.dtype_code, w, d, o.batch, o.ptr(), a.ptr(), o.n, a.n,
+                                          -1, -1, ws.data_ptr(), ws.numel(), _stream_ptr(o.t)))
+    o.finish()
+
+
+def ft_adjoint_left_mul_into(out, operator, argument, basis):
+    """out <- L*_operator(argument)."""
+    w, d = _basis_wd(basis)
+    size = int(_lib.lib.rpyb_tensor_size(w, d))
+    o = _Arg(out, "out", size, True, fresh=True)
+    op = _Arg(operator, "operator", size, False, o.t.device)
+    ar = _Arg(argument, "argument", size, False, o.t.device)
+    _check_same(o, op, ar)
+    _lib.check(_lib.lib.rpyb_ft_adjoint_left_mul_fresh(
+        o.dtype_code, w, d, o.batch, o.ptr(), op.ptr(), ar.ptr(), o.n, op.n, ar.n, None,
+        _stream_ptr(o.t)))
+    o.finish()
+
+
 def lie_map_into(out, arg, matrix: SparseMatrix, scale_factor=None):
     """out <- scale * matrix(arg): the maps above without reading ``out``, whose columns
     past the matrix's rows are left alone."""
-    o = _Arg(out, "out", 1, True)
+    o = _Arg(out, "out", 1, True, fresh=int(np.shape(out)[-1]) == matrix.shape[0])
     a = _Arg(arg, "arg", 1, False, o.t.device)
     _check_same(o, a)
     _apply_csr(o, a, matrix, scale_factor, accumulate=False)

@@ -48,6 +48,7 @@ SIGNATURES = {
     "rpyb_scratch_pool_usage": (_int, [_vp, _vp]),
     "rpyb_tensor_size": (_i64, [_i32, _i32]),
     "rpyb_ft_fma": (_int, [_int, _i32, _i32, _i64, _vp, _vp, _vp, _i64, _i64, _i64, _pi32, _vp]),
+    "rpyb_ft_mul": (_int, [_int, _i32, _i32, _i64, _vp, _vp, _vp, _i64, _i64, _i64, _pi32, _vp]),
     "rpyb_ft_mul_gather": (_int, [_int, _i32, _i32, _i64, _vp, _vp, _vp, _i64, _vp, _vp, _vp,
                                   _int, _vp]),
     "rpyb_ft_mul_gather_mixed": (_int, [_i32, _i32, _i64, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _int,
@@ -65,9 +66,13 @@ SIGNATURES = {
     "rpyb_ft_log_workspace_size": (_i64, [_int, _i32, _i32, _i64]),
     "rpyb_ft_log": (_int, [_int, _i32, _i32, _i64, _vp, _vp, _i64, _i64, _i32, _i32, _vp, _sz,
                            _vp]),
+    "rpyb_ft_log_fresh": (_int, [_int, _i32, _i32, _i64, _vp, _vp, _i64, _i64, _i32, _i32, _vp,
+                                 _sz, _vp]),
     "rpyb_ft_antipode": (_int, [_int, _i32, _i32, _i64, _vp, _vp, _i64, _i64, _vp]),
     "rpyb_ft_adjoint_left_mul": (_int, [_int, _i32, _i32, _i64, _vp, _vp, _vp, _i64, _i64, _i64,
                                         _pi32, _vp]),
+    "rpyb_ft_adjoint_left_mul_fresh": (_int, [_int, _i32, _i32, _i64, _vp, _vp, _vp, _i64, _i64,
+                                              _i64, _pi32, _vp]),
     "rpyb_signature_workspace_size": (_i64, [_int, _i32, _i32, _i64]),
     "rpyb_signature": (_int, [_int, _i32, _i32, _i64, _vp, _vp, _vp, _i64, _vp, _vp, _sz, _vp]),
     "rpyb_signature_batched_workspace_size": (_i64, [_int, _i32, _i32, _i64, _i64, _int]),

@@ -90,8 +90,12 @@ def ft_fma(a: FreeTensor, b: FreeTensor, c: FreeTensor, **kwargs):
 def ft_mul(a: FreeTensor, b: FreeTensor, **kwargs) -> FreeTensor:
     """Free tensor product a * b."""
     _check_basis_compat(a.basis, b.basis)
-    result = _zeros_like(a.data)
-    _internals.dense_ft_fma(result, a.data, b.data, a.basis, rhs_depth=b.basis.depth)
+    if a.data.shape[-1] == a.basis.size():
+        result = _empty_like(a.data)
+        _internals.ft_mul_into(result, a.data, b.data, a.basis, b.basis.depth)
+    else:
+        result = _zeros_like(a.data)
+        _internals.dense_ft_fma(result, a.data, b.data, a.basis, rhs_depth=b.basis.depth)
     return DenseFreeTensor(result, a.basis)
 
 
@@ -103,7 +107,7 @@ def ft_inplace_mul(a: FreeTensor, b: FreeTensor, **kwargs):
 
 def antipode(a: FreeTensor, **kwargs) -> FreeTensor:
     """Antipode (signed word reversal) of a free tensor."""
-    result = _zeros_like(a.data)
+    result = (_empty_like if a.data.shape[-1] == a.basis.size() else _zeros_like)(a.data)
     _internals.dense_ft_antipode(result, a.data, a.basis)
     return FreeTensor(result, a.basis)
 
@@ -113,7 +117,7 @@ def ft_exp(x: FreeTensor, out_basis: TensorBasis | None = None) -> FreeTensor:
     out_basis = out_basis or x.basis
     _check_basis_compat(out_basis, x.basis)
     _float_dtype(x.data)
-    result = _zeros_like(x.data, out_basis.size())
+    result = _empty_like(x.data, out_basis.size())
     _internals.dense_ft_exp(result, x.data, out_basis)
     return FreeTensor(result, out_basis)
 
@@ -123,8 +127,8 @@ def ft_log(x: FreeTensor, out_basis: TensorBasis | None = None) -> FreeTensor:
     out_basis = out_basis or x.basis
     _check_basis_compat(out_basis, x.basis)
     _float_dtype(x.data)
-    result = _zeros_like(x.data, out_basis.size())
-    _internals.dense_ft_log(result, x.data, out_basis)
+    result = _empty_like(x.data, out_basis.size())
+    _internals.ft_log_into(result, x.data, out_basis)
     return FreeTensor(result, out_basis)
 
 
@@ -134,7 +138,7 @@ def ft_fmexp(multiplier: FreeTensor, exponent: FreeTensor,
     out_basis = out_basis or multiplier.basis
     _check_basis_compat(out_basis, multiplier.basis, exponent.basis)
     _float_dtype(multiplier.data)
-    result = _zeros_like(multiplier.data, out_basis.size())
+    result = _empty_like(multiplier.data, out_basis.size())
     _internals.dense_ft_fmexp(result, multiplier.data, exponent.data, out_basis)
     return FreeTensor(result, out_basis)
 
@@ -142,6 +146,10 @@ def ft_fmexp(multiplier: FreeTensor, exponent: FreeTensor,
 def ft_adjoint_left_mul(op: FreeTensor, arg: ShuffleTensor) -> ShuffleTensor:
     """Adjoint of left multiplication by op, applied to the shuffle tensor arg."""
     _check_basis_compat(op.basis, arg.basis)
+    if arg.data.shape[-1] == op.basis.size() and arg.basis.depth >= op.basis.depth:
+        result = _empty_like(arg.data)
+        _internals.ft_adjoint_left_mul_into(result, op.data, arg.data, op.basis)
+        return ShuffleTensor(result, arg.basis)
     result = _zeros_like(arg.data)
     _internals.dense_ft_adjoint_left_mul(result, op.data, arg.data, op.basis, arg.basis.depth,
                                          op.basis.depth, arg.basis.depth)

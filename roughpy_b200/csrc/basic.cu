@@ -75,6 +75,7 @@ struct AdjointArgs {
     int64_t ld_out, ld_op, ld_arg, batch;
     int64_t op_words, arg_words;     // words read of each row (staged form)
     int out_max;
+    bool accumulate;                 // out += (else out =)
     int tiles_per_task;
     int heavy;                       // tiles of more than 64 terms a word (the lowest levels')
 };
@@ -134,9 +135,10 @@ __device__ __forceinline__ void adjoint_tile(const AdjointArgs& a, T* __restrict
         }
         __syncthreads();   // part is free for the next tile
     }
-    if (slice == 0 && E > 0) {
+    if (slice == 0) {
         T* o = out + a.db[k] + i;
-        *o = (T)((double)*o + sum);
+        if (!a.accumulate) *o = (T)sum;
+        else if (E > 0) *o = (T)((double)*o + sum);
     }
 }
 
@@ -285,10 +287,9 @@ RPYB_API int rpyb_ft_antipode(int dtype, int32_t width, int32_t depth, int64_t b
     return RPYB_OK;
 }
 
-RPYB_API int rpyb_ft_adjoint_left_mul(int dtype, int32_t width, int32_t depth, int64_t batch,
-                                      void* out, const void* op, const void* arg, int64_t ld_out,
-                                      int64_t ld_op, int64_t ld_arg, const int32_t* deg,
-                                      void* stream)
+static int adjoint_left_mul(int dtype, int32_t width, int32_t depth, int64_t batch, void* out,
+                            const void* op, const void* arg, int64_t ld_out, int64_t ld_op,
+                            int64_t ld_arg, const int32_t* deg, bool accumulate, void* stream)
 {
     int rc;
     if (dtype != RPYB_F32 && dtype != RPYB_F64) return fail(RPYB_E_INVALID, "unsupported dtype");
@@ -316,6 +317,7 @@ RPYB_API int rpyb_ft_adjoint_left_mul(int dtype, int32_t width, int32_t depth, i
     a.ld_op = ld_op;
     a.ld_arg = ld_arg;
     a.out_max = out_max;
+    a.accumulate = accumulate;
     a.batch = batch;
     // op's words up to its highest degree used (never more than arg's), arg's
     // up to arg_hi
@@ -364,6 +366,24 @@ RPYB_API int rpyb_ft_adjoint_left_mul(int dtype, int32_t width, int32_t depth, i
         return RPYB_OK;
     };
     return dtype == RPYB_F64 ? go(double{}) : go(float{});
+}
+
+RPYB_API int rpyb_ft_adjoint_left_mul(int dtype, int32_t width, int32_t depth, int64_t batch,
+                                      void* out, const void* op, const void* arg, int64_t ld_out,
+                                      int64_t ld_op, int64_t ld_arg, const int32_t* deg,
+                                      void* stream)
+{
+    return adjoint_left_mul(dtype, width, depth, batch, out, op, arg, ld_out, ld_op, ld_arg, deg,
+                            true, stream);
+}
+
+RPYB_API int rpyb_ft_adjoint_left_mul_fresh(int dtype, int32_t width, int32_t depth,
+                                            int64_t batch, void* out, const void* op,
+                                            const void* arg, int64_t ld_out, int64_t ld_op,
+                                            int64_t ld_arg, const int32_t* deg, void* stream)
+{
+    return adjoint_left_mul(dtype, width, depth, batch, out, op, arg, ld_out, ld_op, ld_arg, deg,
+                            false, stream);
 }
 
 RPYB_API int rpyb_sparse_map(int dtype, int64_t n_rows, int64_t n_cols, int64_t batch,

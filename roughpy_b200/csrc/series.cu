@@ -38,6 +38,7 @@ constexpr int64_t kSeriesSmem = 226 * 1024;
 
 struct SeriesArgs {
     int width, top, arg_max;
+    bool fresh;                    // log: out[0] counts as zero
     double coeff[kMaxDepth + 1];   // 1 / deg, or log's series coefficient
     int64_t db[kMaxDepth + 2];
     int64_t pw[kMaxDepth + 1];
@@ -201,7 +202,7 @@ series_kernel(const SeriesArgs a)
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(p + l));
         }
         const double c_fm = MULT ? (double)__ldg(mult) : 1.0;
-        const double c_in = KIND == kSeriesLog ? (double)out[0] : 0.0;
+        const double c_in = KIND == kSeriesLog && !a.fresh ? (double)out[0] : 0.0;
         __syncthreads();
 
         for (int s = 1; s <= N; ++s) {
@@ -399,6 +400,7 @@ int launch_series(int dtype, SeriesKind kind, const Geometry& g, int top, int ar
     a.width = g.width;
     a.top = top;
     a.arg_max = std::min(arg_max, top);
+    a.fresh = rows.fresh;
     for (int deg = 1; deg <= top; ++deg)
         a.coeff[deg] = (kind == kSeriesLog && deg % 2 == 0) ? -(1.0 / deg) : 1.0 / deg;
     for (int k = 0; k <= kMaxDepth + 1; ++k) a.db[k] = g.db[k];
@@ -422,10 +424,10 @@ int launch_series(int dtype, SeriesKind kind, const Geometry& g, int top, int ar
     int64_t threads = std::min<int64_t>({(units + 31) / 32 * 32, std::max<int64_t>(64, 1024 / per_sm / 32 * 32), 512});
     threads = std::max<int64_t>(threads, 32);
     // fewer rows than SMs: blocks of one row share its top level (each
-    // computes the lower levels for itself).  Not for log, whose incoming
+    // computes the lower levels for itself).  Not for a log whose incoming
     // out[0] every block would have to read before one of them writes it.
     int64_t slices = 1;
-    if (kind != kSeriesLog && rows.batch < 148)
+    if ((kind != kSeriesLog || rows.fresh) && rows.batch < 148)
         slices = std::max<int64_t>(1, std::min<int64_t>({16, 296 / rows.batch, units / (2 * threads)}));
     const dim3 grid((unsigned)slices, (unsigned)std::min<int64_t>(rows.batch, 65535), 1);
     if (smem > 48 * 1024)

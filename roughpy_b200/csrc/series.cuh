@@ -14,6 +14,7 @@ struct SeriesRows {
     const void* mult = nullptr;   // fmexp only
     int64_t ld_out = 0, ld_arg = 0, ld_mult = 0;
     int64_t batch = 0;
+    bool fresh = false;           // log: take out[0] as zero
 };
 
 // Whether series of `top` levels of this shape run in the row-resident kernel.

@@ -190,9 +190,10 @@ RPYB_API int64_t rpyb_tensor_size(int32_t width, int32_t depth)
     return g.size();
 }
 
-RPYB_API int rpyb_ft_fma(int dtype, int32_t width, int32_t depth, int64_t batch, void* out,
-                         const void* lhs, const void* rhs, int64_t ld_out, int64_t ld_lhs,
-                         int64_t ld_rhs, const int32_t* deg_bounds, void* stream)
+// out (+)= lhs (x) rhs within the degree bounds
+static int product(int dtype, int32_t width, int32_t depth, int64_t batch, void* out,
+                   const void* lhs, const void* rhs, int64_t ld_out, int64_t ld_lhs,
+                   int64_t ld_rhs, const int32_t* deg_bounds, bool accumulate, void* stream)
 {
     int rc;
     if ((rc = check_dtype(dtype))) return rc;
@@ -219,11 +220,12 @@ RPYB_API int rpyb_ft_fma(int dtype, int32_t width, int32_t depth, int64_t batch,
         sp.pmin[k] = std::max(lmin, k - rmax);
         sp.scale[k] = 1.0;
     }
-    sp.accumulate = true;
-    if (out_min == 0 && lmin == 0 && rmin == 0) {
+    sp.accumulate = accumulate;
+    const bool l0_prod = out_min == 0 && lmin == 0 && rmin == 0;
+    if (l0_prod || (!accumulate && out_min == 0)) {
         sp.l0_write = true;
-        sp.l0_base = 1;
-        sp.l0_prod = true;
+        sp.l0_base = accumulate ? 1 : 0;
+        sp.l0_prod = l0_prod;
         sp.scale0 = 1.0;
     }
     ProductRows rows;
@@ -235,6 +237,22 @@ RPYB_API int rpyb_ft_fma(int dtype, int32_t width, int32_t depth, int64_t batch,
     rows.ld_rhs = ld_rhs;
     rows.batch = batch;
     return launch_product(dtype, g, sp, rows, static_cast<cudaStream_t>(stream));
+}
+
+RPYB_API int rpyb_ft_fma(int dtype, int32_t width, int32_t depth, int64_t batch, void* out,
+                         const void* lhs, const void* rhs, int64_t ld_out, int64_t ld_lhs,
+                         int64_t ld_rhs, const int32_t* deg_bounds, void* stream)
+{
+    return product(dtype, width, depth, batch, out, lhs, rhs, ld_out, ld_lhs, ld_rhs, deg_bounds,
+                   true, stream);
+}
+
+RPYB_API int rpyb_ft_mul(int dtype, int32_t width, int32_t depth, int64_t batch, void* out,
+                         const void* lhs, const void* rhs, int64_t ld_out, int64_t ld_lhs,
+                         int64_t ld_rhs, const int32_t* deg_bounds, void* stream)
+{
+    return product(dtype, width, depth, batch, out, lhs, rhs, ld_out, ld_lhs, ld_rhs, deg_bounds,
+                   false, stream);
 }
 
 RPYB_API int rpyb_ft_mul_gather(int dtype, int32_t width, int32_t depth, int64_t n, void* out,
@@ -552,9 +570,11 @@ RPYB_API int rpyb_ft_fmexp(int dtype, int32_t width, int32_t depth, int64_t batc
                            multiplier, ld_mul, tmp, s);
 }
 
-RPYB_API int rpyb_ft_log(int dtype, int32_t width, int32_t depth, int64_t batch, void* out,
-                         const void* arg, int64_t ld_out, int64_t ld_arg, int32_t out_depth,
-                         int32_t arg_depth, void* workspace, size_t workspace_bytes, void* stream)
+// out <- log(arg); fresh: out's incoming scalar counts as zero and is not read
+static int log_series(int dtype, int32_t width, int32_t depth, int64_t batch, void* out,
+                      const void* arg, int64_t ld_out, int64_t ld_arg, int32_t out_depth,
+                      int32_t arg_depth, bool fresh, void* workspace, size_t workspace_bytes,
+                      void* stream)
 {
     int rc;
     if ((rc = check_dtype(dtype))) return rc;
@@ -581,7 +601,12 @@ RPYB_API int rpyb_ft_log(int dtype, int32_t width, int32_t depth, int64_t batch,
         r.arg = arg;
         r.ld_arg = ld_arg;
         r.batch = batch;
+        r.fresh = fresh;
         return launch_series(dtype, kSeriesLog, g, M, Ma, r, s);
+    }
+    if (fresh) {
+        const size_t es = elem_size(dtype);
+        RPYB_CUDA(cudaMemset2DAsync(out, (size_t)ld_out * es, 0, es, (size_t)batch, s));
     }
     double* tmp = static_cast<double*>(base);
     double* out64 = static_cast<double*>(out);
@@ -647,6 +672,23 @@ RPYB_API int rpyb_ft_log(int dtype, int32_t width, int32_t depth, int64_t batch,
             return rc;
     }
     return RPYB_OK;
+}
+
+RPYB_API int rpyb_ft_log(int dtype, int32_t width, int32_t depth, int64_t batch, void* out,
+                         const void* arg, int64_t ld_out, int64_t ld_arg, int32_t out_depth,
+                         int32_t arg_depth, void* workspace, size_t workspace_bytes, void* stream)
+{
+    return log_series(dtype, width, depth, batch, out, arg, ld_out, ld_arg, out_depth, arg_depth,
+                      false, workspace, workspace_bytes, stream);
+}
+
+RPYB_API int rpyb_ft_log_fresh(int dtype, int32_t width, int32_t depth, int64_t batch, void* out,
+                               const void* arg, int64_t ld_out, int64_t ld_arg,
+                               int32_t out_depth, int32_t arg_depth, void* workspace,
+                               size_t workspace_bytes, void* stream)
+{
+    return log_series(dtype, width, depth, batch, out, arg, ld_out, ld_arg, out_depth, arg_depth,
+                      true, workspace, workspace_bytes, stream);
 }
 
 }  // extern "C"
