@@ -938,10 +938,33 @@ enum LaunchMode { kSuffix = 0, kBlocked = 1, kW2 = 2 };
 static int launch_levels(int dtype, const Geometry& g, const ProductSpec& spec,
                          const ProductRows& rows, cudaStream_t stream, int mode);
 
+// The environment switches name kernels of this file, and the row-resident
+// kernel accumulates float32 rows in float64 only.
+bool product_rows_enabled(int dtype)
+{
+    return blocked_enabled() && w2_kernel_enabled() && (dtype != RPYB_F32 || f32_acc_mode() == 1);
+}
+
+// Accumulating products of long rows at widths 6 and 8: with at most three
+// rows an SM the row-resident kernel does not keep HBM as busy as the blocked
+// one, whose tiles of a row are independent.  Measured on B200, row-resident /
+// blocked: (8,5) float64 x 700 167 / 151 us, (6,6) float64 x 300 111 / 105 us,
+// float32 74 / 72 us; shorter rows, assigning products ((8,5) float64 117 / 130
+// us, (6,6) 86 / 93 us) and float32 (8,5) (97 / 111 us) are faster row-resident.
+static bool blocked_accumulates_faster(int dtype, const Geometry& g, const ProductSpec& spec)
+{
+    if (!spec.accumulate || (g.width != 6 && g.width != 8)) return false;
+    const int64_t staged = 2 * g.db[spec.khi] * 8;
+    return staged > (dtype == RPYB_F32 ? 128 : 72) * 1024;
+}
+
 int launch_product(int dtype, const Geometry& g, const ProductSpec& spec,
                    const ProductRows& rows, cudaStream_t stream)
 {
     if (rows.batch <= 0) return RPYB_OK;
+    if (product_rows_enabled(dtype) && product_rows_available(g, spec, rows) &&
+        !blocked_accumulates_faster(dtype, g, spec))
+        return launch_product_rows(dtype, g, spec, rows, false, stream);
     // float64 rows of width 2 up to level kW2MinTop or higher: the
     // lane-letter kernel
     if (dtype == RPYB_F64 && blocked_enabled() && g.width == 2 && w2_kernel_enabled() &&

@@ -48,6 +48,14 @@ constexpr int kMixedF64F32 = 2;
 int launch_product(int dtype, const Geometry& g, const ProductSpec& spec,
                    const ProductRows& rows, cudaStream_t stream);
 
+// The row-resident product (product_rows.cu): whole truncated products of rows
+// whose lower levels fit in shared memory.  With in_place, out may be lhs.
+// product_rows_enabled: no environment switch asks for another product kernel.
+bool product_rows_enabled(int dtype);
+bool product_rows_available(const Geometry& g, const ProductSpec& spec, const ProductRows& rows);
+int launch_product_rows(int dtype, const Geometry& g, const ProductSpec& spec,
+                        const ProductRows& rows, bool in_place, cudaStream_t stream);
+
 // Elementwise helpers used by the Horner drivers.
 int launch_convert_rows(int dst_dtype, void* dst, int64_t ld_dst, int src_dtype,
                         const void* src, int64_t ld_src, int64_t cols, int64_t batch,

@@ -1,0 +1,356 @@
+// Row-resident product: out (+)= lhs (x) rhs with a row's lower levels in
+// shared memory (sm_100a).
+//
+// The top level holds most of a row's words, and each of its words needs the
+// two top-level words L_N, R_N (and the old out_N), read once, and products of
+// lower-level words.  One block stages the lower levels of both factors as
+// float64 (a float32 word is converted once, not once a use), computes the
+// lower output levels from them and streams the top level: coalesced reads and
+// writes, all other operands from shared memory (split_unit).  The terms of a
+// word are added in the same order as in the product kernels that read their
+// operands through L1, so results are the same bits.
+//
+// Measured on B200 against the kernels that read lower levels through L1 (in
+// product.cu, kept for shapes that do not fit and for bounded products): out =
+// lhs (x) rhs, (5,6) float64 x 700 107 -> 61 us (5.4 TB/s), (7,5) float32 x 700
+// 80 -> 41 us, (8,5) float32 107 -> 74 us, (8,3) float64 x 20000 145 -> 45 us
+// (6.3 TB/s); accumulating, (2,12) float32 x 1024 57.5 -> 49.5 us, (4,7)
+// float64 x 1000 130 -> 118 us.  What bounds it is HBM for float64 and short
+// rows; for narrow float32 rows the shared-memory requests of the splits.
+//
+// out may be lhs (in place): the lower levels are staged before a word is
+// written, and a top-level word of a factor is read only by the thread that
+// then writes the same word.
+#include <algorithm>
+
+#include "product.cuh"
+#include "row_units.cuh"
+
+namespace rpyb {
+namespace {
+
+// dynamic shared memory a block may take (227 KB less the static part)
+constexpr int64_t kRowSmem = 226 * 1024;
+constexpr int kRowThreads = 1024;   // most threads a block
+
+struct RowArgs {
+    int width, top;
+    int64_t db[kMaxDepth + 2];
+    int64_t pw[kMaxDepth + 1];
+    void* out;
+    const void* lhs;
+    const void* rhs;
+    int64_t ld_out, ld_lhs, ld_rhs, batch;
+    const int64_t* out_idx;
+    const int64_t* lhs_idx;
+    const int64_t* rhs_idx;
+};
+
+// The deepest top level of width D whose lower levels fit, both factors'.
+template <int D>
+constexpr int row_max_top()
+{
+    int64_t words = 0, pw = 1;
+    for (int k = 0; k <= kMaxDepth; ++k) {   // words: below level k
+        if (2 * words * 8 > kRowSmem) return k - 1;
+        words += pw;
+        pw *= D;
+    }
+    return kMaxDepth;
+}
+
+// Starts the lines of `runs` (at most 16) runs of `left` words (32 at most are
+// wanted), `run` words apart from p, towards L2: one line a lane.
+template <typename T>
+__device__ __forceinline__ void prefetch_runs(const T* p, int64_t run, int runs, int64_t left,
+                                              int lane)
+{
+    constexpr int kLines = sizeof(T) == 8 ? 2 : 1;   // of 128 bytes, a run
+    if (lane < runs * kLines && (lane % kLines) * 16 < left)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(p + (lane / kLines) * run + (lane % kLines) * 16));
+}
+
+// Room for n words staged by stage_words, in float64 words (16-byte multiple).
+__host__ __device__ constexpr int stage_room(int n) { return (n + 3) & ~1; }
+
+// n words of a row into shared memory as float64, at the returned place in
+// `room` (16-byte aligned, stage_room(n) words).  Float64: asynchronous copies
+// of 16 bytes, with a word before the first aligned piece and after the last
+// where the row starts or ends between two (8-byte copies throughout kept the
+// load/store queue full: mio_throttle 16.7 cycles an issue, (8,5) 173 -> 167
+// us).  Float32: words, eight of a thread's in flight (16-byte loads, whose
+// odd words wait for a latency of their own, were slower: (2,12) 43 -> 58 us).
+template <typename T>
+__device__ __forceinline__ double* stage_words(double* room, const T* src, int n, int tid, int B)
+{
+    if constexpr (sizeof(T) == 8) {
+        const int head = (int)((reinterpret_cast<uintptr_t>(src) >> 3) & 1);
+        double* dst = room + head;
+        const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst);
+        const int pieces = (n - head) / 2;
+        for (int i = tid; i < pieces; i += B)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + (head + 2 * i) * 8),
+                         "l"(src + head + 2 * i)
+                         : "memory");
+        const int odd = tid == 0 && head ? 0 : tid == 1 && head + 2 * pieces < n ? n - 1 : -1;
+        if (odd >= 0)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(to + odd * 8), "l"(src + odd)
+                         : "memory");
+        return dst;
+    } else {
+        constexpr int kLoads = 8;
+        for (int i0 = tid; i0 < n; i0 += kLoads * B) {
+            T v[kLoads];
+#pragma unroll
+            for (int j = 0; j < kLoads; ++j) v[j] = i0 + j * B < n ? src[i0 + j * B] : T(0);
+#pragma unroll
+            for (int j = 0; j < kLoads; ++j)
+                if (i0 + j * B < n) room[i0 + j * B] = (double)v[j];
+        }
+        return room;
+    }
+}
+
+template <typename T, typename TR, bool ACCUM, int D, int F>
+__global__ void __launch_bounds__(kRowThreads, 1)
+product_rows_kernel(const RowArgs a)
+{
+    constexpr int DD = D > 0 ? D : 1;
+    constexpr int U = D > 0 ? Power<DD, F>::value : 16;
+    extern __shared__ __align__(16) unsigned char row_smem[];
+    const int N = a.top;
+    const int d = D > 0 ? D : a.width;
+    const int uu = D > 0 ? U : d;   // words a unit has
+    const int TL = (int)a.db[N];
+    double* const l_room = reinterpret_cast<double*>(row_smem);
+    double* const r_room = l_room + stage_room(TL);
+    const int tid = (int)threadIdx.x, B = (int)blockDim.x;
+    const int lane = tid & 31, warp = tid >> 5, nwarps = B >> 5;
+
+    for (int64_t b = blockIdx.y; b < a.batch; b += gridDim.y) {
+        // not restrict: out may be lhs
+        T* out = static_cast<T*>(a.out) + (a.out_idx ? a.out_idx[b] : b) * a.ld_out;
+        const T* lhs = static_cast<const T*>(a.lhs) + (a.lhs_idx ? a.lhs_idx[b] : b) * a.ld_lhs;
+        const TR* rhs = static_cast<const TR*>(a.rhs) + (a.rhs_idx ? a.rhs_idx[b] : b) * a.ld_rhs;
+        __syncthreads();   // the previous row is done with the buffers
+        const double* L = stage_words(l_room, lhs, TL, tid, B);
+        const double* R = stage_words(r_room, rhs, TL, tid, B);
+        // The top-level words of a warp's next task start towards L2 while it
+        // works on one.  (The whole top level at once would be more than L2
+        // holds over all resident rows: (6,5) float64 ran at 3.1 TB/s so.)
+        const int top_tasks = N >= F ? (int)((a.pw[N - F] + 31) >> 5) : 0;
+        const int tstep = nwarps * (int)gridDim.x;
+        auto prefetch_task = [&](int t) {
+            if (t >= top_tasks) return;
+            const int64_t run = a.pw[N - F];
+            const int64_t o = a.db[N] + t * 32;
+            const int64_t left = run - t * 32;
+            prefetch_runs(lhs + o, run, uu, left, lane);
+            prefetch_runs(rhs + o, run, uu, left, lane);
+            if (ACCUM) prefetch_runs(static_cast<const T*>(out) + o, run, uu, left, lane);
+        };
+        prefetch_task(warp + nwarps * (int)blockIdx.x);
+        T out0 = T(0);
+        if (ACCUM && tid == 0 && blockIdx.x == 0) out0 = out[0];
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        const double l0 = L[0], r0 = R[0];
+
+        // unit r of the top level (streamed) or of a lower one (in shared memory)
+        auto unit = [&](auto kc, auto topc, uint32_t r) {
+            constexpr int K = decltype(kc)::value;
+            constexpr bool TOP = decltype(topc)::value;
+            constexpr int run = Power<DD, K - F>::value, begin = LevelStart<DD, K>::value;
+            if (run % 32 != 0 && r >= (uint32_t)run) return;
+            double acc[U];
+            T* op = out + begin + r;
+#pragma unroll
+            for (int u = 0; u < U; ++u) acc[u] = ACCUM ? (double)op[u * run] : 0.0;
+            if constexpr (TOP) {
+                const T* lp = lhs + begin + r;
+                T lv[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) lv[u] = lp[u * run];
+#pragma unroll
+                for (int u = 0; u < U; ++u) acc[u] = fma((double)lv[u], r0, acc[u]);
+            } else {
+                const double* lp = L + begin + r;
+#pragma unroll
+                for (int u = 0; u < U; ++u) acc[u] = fma(lp[u * run], r0, acc[u]);
+            }
+            if constexpr (TOP) {
+                const TR* rp = rhs + begin + r;
+                TR rv[U];   // in flight during the splits
+#pragma unroll
+                for (int u = 0; u < U; ++u) rv[u] = rp[u * run];
+                split_unit<DD, F, K, U>(acc, L, R, r);
+#pragma unroll
+                for (int u = 0; u < U; ++u) acc[u] = fma(l0, (double)rv[u], acc[u]);
+            } else {
+                split_unit<DD, F, K, U>(acc, L, R, r);
+                const double* rp = R + begin + r;
+#pragma unroll
+                for (int u = 0; u < U; ++u) acc[u] = fma(l0, rp[u * run], acc[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) op[u * run] = (T)acc[u];
+        };
+        auto any_unit = [&](int k, uint32_t r) {
+            const uint32_t run = (uint32_t)a.pw[k - 1];
+            if (r >= run) return;
+            const int o = (int)a.db[k] + (int)r;
+            double acc[16];
+#pragma unroll
+            for (int u = 0; u < 16; ++u) {
+                if (u >= d) break;
+                acc[u] = ACCUM ? (double)out[o + u * run] : 0.0;
+                acc[u] = fma(k < N ? L[o + u * run] : (double)lhs[o + u * run], r0, acc[u]);
+            }
+            split_unit_any(acc, L, R, a.db, a.pw, (uint32_t)d, k, r);
+#pragma unroll
+            for (int u = 0; u < 16; ++u) {
+                if (u >= d) break;
+                const double rv = k < N ? R[o + u * run] : (double)rhs[o + u * run];
+                out[o + u * run] = (T)fma(l0, rv, acc[u]);
+            }
+        };
+        // levels 0 and below the owned letters, word by word
+        auto short_levels = [&]() {
+            for (int k = 1; k < F && k <= N; ++k) {
+                for (int w = lane; w < (int)a.pw[k]; w += 32) {
+                    const int o = (int)a.db[k] + w;
+                    double v = ACCUM ? (double)out[o] : 0.0;
+                    v = fma(k < N ? L[o] : (double)lhs[o], r0, v);
+                    int ds = 1;
+                    for (int s = 1; s < k; ++s) {
+                        ds *= d;
+                        v = fma(L[a.db[k - s] + w / ds], R[a.db[s] + w % ds], v);
+                    }
+                    out[o] = (T)fma(l0, k < N ? R[o] : (double)rhs[o], v);
+                }
+            }
+        };
+
+        int t = warp;
+        const int step = nwarps;
+        if (N >= F) {
+            for (t += nwarps * (int)blockIdx.x; t < top_tasks; t += tstep) {
+                prefetch_task(t + tstep);
+                const uint32_t r = (uint32_t)(t * 32 + lane);
+                if constexpr (D > 0) {
+                    with_level<F, row_max_top<DD>()>(N, [&](auto kc) {
+                        unit(kc, std::integral_constant<bool, true>{}, r);
+                    });
+                } else {
+                    any_unit(N, r);
+                }
+            }
+            t = gridDim.x > 1 ? warp : t - top_tasks;
+        }
+        if (blockIdx.x != 0) continue;
+        for (int k = max(N - 1, F - 1); k >= F - 1;) {   // level F - 1: the short levels' task
+            const int tasks = k >= F ? (int)((a.pw[k - F] + 31) >> 5) : 1;
+            if (t >= tasks) {
+                t -= tasks;
+                --k;
+                continue;
+            }
+            if (k < F) {
+                short_levels();
+            } else {
+                const uint32_t r = (uint32_t)(t * 32 + lane);
+                if constexpr (D > 0) {
+                    with_level<F, row_max_top<DD>() - 1>(k, [&](auto kc) {
+                        unit(kc, std::integral_constant<bool, false>{}, r);
+                    });
+                } else {
+                    any_unit(k, r);
+                }
+            }
+            t += step;
+        }
+        if (tid == 0) out[0] = out0 + (T)l0 * (T)r0;   // level 0, in the rows' type
+    }
+}
+
+using RowFn = void (*)(RowArgs);
+
+template <typename T, typename TR, bool ACCUM>
+RowFn row_fn(int width)
+{
+    switch (width) {
+        case 2: return &product_rows_kernel<T, TR, ACCUM, 2, 3>;
+        case 3: return &product_rows_kernel<T, TR, ACCUM, 3, 2>;
+        case 4: return &product_rows_kernel<T, TR, ACCUM, 4, 1>;
+        case 5: return &product_rows_kernel<T, TR, ACCUM, 5, 1>;
+        case 6: return &product_rows_kernel<T, TR, ACCUM, 6, 1>;
+        case 7: return &product_rows_kernel<T, TR, ACCUM, 7, 1>;
+        case 8: return &product_rows_kernel<T, TR, ACCUM, 8, 1>;
+        default: return &product_rows_kernel<T, TR, ACCUM, 0, 1>;
+    }
+}
+
+}  // namespace
+
+bool product_rows_available(const Geometry& g, const ProductSpec& spec, const ProductRows& rows)
+{
+    const int N = spec.khi;
+    if (g.width < 2 || g.width > 16 || N < 1 || 2 * g.db[N] * 8 > kRowSmem) return false;
+    // the whole truncated product of whole rows
+    if (spec.klo != 1 || !spec.lhs0_from_mem || spec.lhs0_add != 0.0 || rows.addend) return false;
+    if (!spec.l0_write || !spec.l0_prod || spec.l0_const != 0.0 || spec.scale0 != 1.0 ||
+        spec.l0_base != (spec.accumulate ? 1 : 0))
+        return false;
+    for (int k = 1; k <= N; ++k)
+        if (spec.pmin[k] != 0 || spec.pmax[k] != k || spec.scale[k] != 1.0) return false;
+    return true;
+}
+
+int launch_product_rows(int dtype, const Geometry& g, const ProductSpec& spec,
+                        const ProductRows& rows, bool in_place, cudaStream_t stream)
+{
+    RowArgs a{};
+    a.width = g.width;
+    a.top = spec.khi;
+    for (int k = 0; k <= kMaxDepth + 1; ++k) a.db[k] = g.db[k];
+    for (int k = 0; k <= kMaxDepth; ++k) a.pw[k] = g.pw[k];
+    a.out = rows.out;
+    a.lhs = rows.lhs;
+    a.rhs = rows.rhs;
+    a.ld_out = rows.ld_out;
+    a.ld_lhs = rows.ld_lhs;
+    a.ld_rhs = rows.ld_rhs;
+    a.batch = rows.batch;
+    a.out_idx = rows.out_idx;
+    a.lhs_idx = rows.lhs_idx;
+    a.rhs_idx = rows.rhs_idx;
+    RowFn fn;
+    if (dtype == RPYB_F64)
+        fn = spec.accumulate ? row_fn<double, double, true>(g.width) : row_fn<double, double, false>(g.width);
+    else if (dtype == kMixedF64F32)
+        fn = spec.accumulate ? row_fn<double, float, true>(g.width) : row_fn<double, float, false>(g.width);
+    else
+        fn = spec.accumulate ? row_fn<float, float, true>(g.width) : row_fn<float, float, false>(g.width);
+    const int F = g.width == 2 ? 3 : g.width == 3 ? 2 : 1;
+    const size_t smem = (size_t)(2 * stage_room((int)g.db[a.top]) * 8);
+    // threads: one per top-level unit up to what gives an SM 1024 threads over
+    // the blocks its shared memory holds
+    const int64_t units = a.top >= F ? g.pw[a.top - F] : g.pw[a.top];
+    const int64_t per_sm = std::max<int64_t>(1, std::min<int64_t>(16, kRowSmem / (int64_t)(smem + 1024)));
+    int64_t threads = std::min<int64_t>({(units + 31) / 32 * 32,
+                                         std::max<int64_t>(64, 1024 / per_sm / 32 * 32), kRowThreads});
+    threads = std::max<int64_t>(threads, 32);
+    // fewer rows than SMs: blocks share a row's top level (not in place, where
+    // one block would write lower levels that another still has to stage)
+    int64_t slices = 1;
+    if (!in_place && rows.batch < 148)
+        slices = std::max<int64_t>(1, std::min<int64_t>({16, 296 / rows.batch, units / (2 * threads)}));
+    const dim3 grid((unsigned)slices, (unsigned)std::min<int64_t>(rows.batch, 65535), 1);
+    if (smem > 48 * 1024)
+        RPYB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    fn<<<grid, (unsigned)threads, smem, stream>>>(a);
+    RPYB_CUDA(cudaGetLastError());
+    return RPYB_OK;
+}
+
+}  // namespace rpyb

@@ -1,0 +1,109 @@
+// Units of a dense product with both factors' lower levels in shared memory:
+// shared by the series and the row-resident product kernels.
+#pragma once
+
+#include <type_traits>
+
+#include "common.cuh"
+
+namespace rpyb {
+
+template <int D, int E>
+struct Power {
+    static constexpr int value = D * Power<D, E - 1>::value;
+};
+template <int D>
+struct Power<D, 0> {
+    static constexpr int value = 1;
+};
+// first word of level K
+template <int D, int K>
+struct LevelStart {
+    static constexpr int value = LevelStart<D, K - 1>::value + Power<D, K - 1>::value;
+};
+template <int D>
+struct LevelStart<D, 0> {
+    static constexpr int value = 0;
+};
+
+// acc[u] += sum over p = K - 1 down to 1 of R_p (x) X_{K-p} at the words
+// u D^(K-F) + r of level K >= F (u over the first F letters, r the others), the
+// lower levels of R and X as float64 in shared memory.  Every split is
+// unrolled: word offsets are immediates, and a split costs one division by D,
+// two addresses and U + 1 shared loads.  Lanes of consecutive r read right
+// words as conflict-free runs and left words as broadcasts or short runs.
+template <int D, int F, int K, int U>
+__device__ __forceinline__ void split_unit(double (&acc)[U], const double* R, const double* X,
+                                            uint32_t r)
+{
+    // from the shortest right part up, peeling a letter a step
+    uint32_t q = r, m = 0;
+    auto split = [&](auto sc) {
+        constexpr int s = decltype(sc)::value;
+        const uint32_t q2 = q / (uint32_t)D;
+        m += (q - q2 * (uint32_t)D) * (uint32_t)Power<D, s - 1>::value;
+        q = q2;
+        constexpr int run = Power<D, K - s - F>::value;
+        const double x = X[LevelStart<D, s>::value + m];
+        const double* rp = R + LevelStart<D, K - s>::value + q;
+#pragma unroll
+        for (int u = 0; u < U; ++u) acc[u] = fma(rp[u * run], x, acc[u]);
+    };
+    auto walk = [&](auto self, auto sc) {
+        constexpr int s = decltype(sc)::value;
+        if constexpr (s <= K - F) {
+            split(sc);
+            self(self, std::integral_constant<int, s + 1>{});
+        }
+    };
+    walk(walk, std::integral_constant<int, 1>{});
+    // splits inside the owned first letters, p = 2 then 1
+    if constexpr (F >= 3 && K >= 3) {
+        constexpr int rest = Power<D, F - 2>::value, run = Power<D, K - F>::value;
+        const double* xp = X + LevelStart<D, K - 2>::value + r;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            acc[u] = fma(R[LevelStart<D, 2>::value + u / rest], xp[(u % rest) * run], acc[u]);
+    }
+    if constexpr (F >= 2 && K >= 2) {
+        constexpr int rest = Power<D, F - 1>::value, run = Power<D, K - F>::value;
+        const double* xp = X + LevelStart<D, K - 1>::value + r;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            acc[u] = fma(R[LevelStart<D, 1>::value + u / rest], xp[(u % rest) * run], acc[u]);
+    }
+}
+
+// The same for a runtime width (F = 1, up to 16 words a unit).
+__device__ __forceinline__ void split_unit_any(double (&acc)[16], const double* R, const double* X,
+                                                const int64_t* db, const int64_t* pw,
+                                                uint32_t d, int k, uint32_t r)
+{
+    uint32_t q = r, m = 0, ds = 1;
+    for (int s = 1; s < k; ++s) {
+        const uint32_t q2 = q / d;
+        m += (q - q2 * d) * ds;
+        q = q2;
+        ds *= d;
+        const int p = k - s;
+        const double x = X[db[s] + m];
+        const double* rp = R + db[p] + q;
+        const uint32_t run = (uint32_t)pw[p - 1];
+#pragma unroll
+        for (int u = 0; u < 16; ++u)
+            if (u < (int)d) acc[u] = fma(rp[u * run], x, acc[u]);
+    }
+}
+
+// Calls f(k as a compile-time constant) for a level F <= k <= KMAX.
+template <int F, int KMAX, typename Fn>
+__device__ __forceinline__ void with_level(int k, Fn&& f)
+{
+    if constexpr (KMAX >= F) {
+        if (k == KMAX) f(std::integral_constant<int, KMAX>{});
+        else with_level<F, KMAX - 1>(k, f);
+    }
+}
+
+
+}  // namespace rpyb

@@ -27,8 +27,9 @@
 // 1.25 requests an FMA.  Levels are compile-time constants inside a unit.
 #include "series.cuh"
 
+#include "row_units.cuh"
+
 #include <algorithm>
-#include <type_traits>
 
 namespace rpyb {
 namespace {
@@ -47,100 +48,6 @@ struct SeriesArgs {
     const void* mult;
     int64_t ld_out, ld_arg, ld_mult, batch;
 };
-
-template <int D, int E>
-struct Power {
-    static constexpr int value = D * Power<D, E - 1>::value;
-};
-template <int D>
-struct Power<D, 0> {
-    static constexpr int value = 1;
-};
-// first word of level K
-template <int D, int K>
-struct LevelStart {
-    static constexpr int value = LevelStart<D, K - 1>::value + Power<D, K - 1>::value;
-};
-template <int D>
-struct LevelStart<D, 0> {
-    static constexpr int value = 0;
-};
-
-// acc[u] += sum over 0 < p < K of R_p (x) x_{K-p} at the words u D^(K-F) + r of
-// level K >= F, every split unrolled: word offsets are immediates, and a split
-// costs one division by D, two addresses and U + 1 shared loads.
-template <int D, int F, int K, int U>
-__device__ __forceinline__ void series_unit(double (&acc)[U], const double* R, const double* X,
-                                            uint32_t r)
-{
-    // splits inside the owned first letters
-    if constexpr (F >= 2 && K >= 2) {
-        constexpr int rest = Power<D, F - 1>::value, run = Power<D, K - F>::value;
-        const double* xp = X + LevelStart<D, K - 1>::value + r;
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            acc[u] = fma(R[LevelStart<D, 1>::value + u / rest], xp[(u % rest) * run], acc[u]);
-    }
-    if constexpr (F >= 3 && K >= 3) {
-        constexpr int rest = Power<D, F - 2>::value, run = Power<D, K - F>::value;
-        const double* xp = X + LevelStart<D, K - 2>::value + r;
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            acc[u] = fma(R[LevelStart<D, 2>::value + u / rest], xp[(u % rest) * run], acc[u]);
-    }
-    // the others, from the shortest right part up, peeling a letter a step
-    uint32_t q = r, m = 0;
-    auto split = [&](auto sc) {
-        constexpr int s = decltype(sc)::value;
-        const uint32_t q2 = q / (uint32_t)D;
-        m += (q - q2 * (uint32_t)D) * (uint32_t)Power<D, s - 1>::value;
-        q = q2;
-        constexpr int run = Power<D, K - s - F>::value;
-        const double x = X[LevelStart<D, s>::value + m];
-        const double* rp = R + LevelStart<D, K - s>::value + q;
-#pragma unroll
-        for (int u = 0; u < U; ++u) acc[u] = fma(rp[u * run], x, acc[u]);
-    };
-    auto walk = [&](auto self, auto sc) {
-        constexpr int s = decltype(sc)::value;
-        if constexpr (s <= K - F) {
-            split(sc);
-            self(self, std::integral_constant<int, s + 1>{});
-        }
-    };
-    walk(walk, std::integral_constant<int, 1>{});
-}
-
-// The same for a runtime width (F = 1, up to 16 words a unit).
-__device__ __forceinline__ void series_unit_any(double (&acc)[16], const double* R, const double* X,
-                                                const SeriesArgs& a, int k, uint32_t r)
-{
-    const uint32_t d = (uint32_t)a.width;
-    uint32_t q = r, m = 0, ds = 1;
-    for (int s = 1; s < k; ++s) {
-        const uint32_t q2 = q / d;
-        m += (q - q2 * d) * ds;
-        q = q2;
-        ds *= d;
-        const int p = k - s;
-        const double x = X[a.db[s] + m];
-        const double* rp = R + a.db[p] + q;
-        const uint32_t run = (uint32_t)a.pw[p - 1];
-#pragma unroll
-        for (int u = 0; u < 16; ++u)
-            if (u < (int)d) acc[u] = fma(rp[u * run], x, acc[u]);
-    }
-}
-
-// Calls f(k as a compile-time constant) for a level F <= k <= KMAX.
-template <int F, int KMAX, typename Fn>
-__device__ __forceinline__ void with_level(int k, Fn&& f)
-{
-    if constexpr (KMAX >= F) {
-        if (k == KMAX) f(std::integral_constant<int, KMAX>{});
-        else with_level<F, KMAX - 1>(k, f);
-    }
-}
 
 // The deepest top level of width D whose lower levels fit (three copies).
 template <int D>
@@ -223,7 +130,7 @@ series_kernel(const SeriesArgs a)
                 const double* xp = X + begin + r;
 #pragma unroll
                 for (int u = 0; u < U; ++u) acc[u] = c * xp[u * run];
-                series_unit<DD, F, K, U>(acc, Rc, X, r);
+                split_unit<DD, F, K, U>(acc, Rc, X, r);
                 if constexpr (SCALE) {
 #pragma unroll
                     for (int u = 0; u < U; ++u) acc[u] *= scale;
@@ -255,7 +162,7 @@ series_kernel(const SeriesArgs a)
                 double acc[U];
 #pragma unroll
                 for (int u = 0; u < U; ++u) acc[u] = 0.0;
-                series_unit<DD, F, K, U>(acc, Rc, X, r);
+                split_unit<DD, F, K, U>(acc, Rc, X, r);
                 T* op = out + begin + r;
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
@@ -275,7 +182,7 @@ series_kernel(const SeriesArgs a)
                 for (int u = 0; u < 16; ++u)
                     if (u < d)
                         acc[u] = c * (k < N ? X[o + u * run] : xtop ? (double)__ldg(arg + o + u * run) : 0.0);
-                series_unit_any(acc, Rc, X, a, k, r);
+                split_unit_any(acc, Rc, X, a.db, a.pw, (uint32_t)d, k, r);
 #pragma unroll
                 for (int u = 0; u < 16; ++u) {
                     if (u >= d) break;

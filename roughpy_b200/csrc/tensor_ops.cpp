@@ -387,6 +387,20 @@ RPYB_API int rpyb_ft_inplace_mul(int dtype, int32_t width, int32_t depth, int64_
     rows.rhs = rhs;
     rows.ld_rhs = ld_rhs;
     rows.batch = batch;
+    // In place where one block has a whole row: three passes over the rows
+    // instead of five.  Rows of the two operands may be the same, but no row
+    // of one may reach into another row of the other.
+    const char* l0 = static_cast<const char*>(lhs);
+    const char* r0 = static_cast<const char*>(rhs);
+    const int64_t l_bytes = ((batch - 1) * ld_lhs + T) * (int64_t)es;
+    const int64_t r_bytes = ((batch - 1) * ld_rhs + T) * (int64_t)es;
+    const bool apart = r0 >= l0 + l_bytes || l0 >= r0 + r_bytes;
+    const bool same = l0 == r0 && (ld_lhs == ld_rhs || batch == 1);
+    if ((apart || same) && product_rows_enabled(dtype) && product_rows_available(g, sp, rows)) {
+        rows.out = lhs;
+        rows.ld_out = ld_lhs;
+        return launch_product_rows(dtype, g, sp, rows, true, s);
+    }
     if ((rc = launch_product(dtype, g, sp, rows, s))) return rc;
     const int64_t c0 = g.db[lmin], c1 = g.db[lmax + 1];
     RPYB_CUDA(cudaMemcpy2DAsync(static_cast<char*>(lhs) + c0 * es, (size_t)ld_lhs * es,
