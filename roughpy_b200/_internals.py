@@ -18,6 +18,7 @@ and degree bounds.
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import numpy as np
 import torch
@@ -213,6 +214,31 @@ def check_lie_basis_data(width, depth, data, degree_begin=None) -> bool:
 
 
 # -------------------------------------------------------------- array glue
+# A call on small CUDA tensors takes a few microseconds on the device, so what is
+# computed per call here is kept to look-ups: sizes and standard layouts by (width,
+# depth), bounds by value.
+_CODES = {torch.float64: _lib.F64, torch.float32: _lib.F32}
+
+
+@functools.lru_cache(maxsize=1024)
+def _size(width: int, depth: int) -> int:
+    return int(_lib.lib.rpyb_tensor_size(width, depth))
+
+
+@functools.lru_cache(maxsize=1024)
+def _standard_bytes(width: int, depth: int) -> bytes:
+    return _standard_degree_begin(width, depth).tobytes()
+
+
+@functools.lru_cache(maxsize=1024)
+def _bounds_array(vals):
+    return _lib.bounds(*vals)   # read by the library only
+
+
+def _bounds(*vals):
+    return _bounds_array(tuple([int(v) for v in vals]))
+
+
 def _dtype_code(dt) -> int:
     if dt in (np.float64, torch.float64):
         return _lib.F64
@@ -231,70 +257,78 @@ def _basis_wd(basis):
         db = np.asarray(db)
         if db.ndim != 1 or db.shape[0] < d + 2:
             raise ValueError("degree_begin must have at least depth + 2 elements")
-        if not np.array_equal(db[:d + 2], _standard_degree_begin(w, d)):
+        db = db[:d + 2]
+        if not (db.tobytes() == _standard_bytes(w, d) if db.dtype == np.intp
+                else np.array_equal(db, _standard_degree_begin(w, d))):
             raise NotImplementedError("only the standard dense degree layout is supported")
     return w, d
 
 
 class _Arg:
-    """One array argument: a CUDA tensor view of shape (batch, n) plus writeback."""
+    """One array argument: a contiguous CUDA tensor of batch rows of n words, plus writeback."""
+
+    __slots__ = ("name", "obj", "is_numpy", "t", "lead", "n", "writable", "dtype_code")
 
     def __init__(self, obj, name: str, need: int, writable: bool, device=None, fresh=False):
         self.name = name
         self.obj = obj
-        self.is_numpy = isinstance(obj, np.ndarray)
-        if self.is_numpy and fresh:
-            # wholly written by the call: nothing to copy to the device
-            if obj.dtype not in (np.float32, np.float64):
-                raise TypeError(f"{name}: unsupported dtype")
-            self.t = torch.empty(obj.shape, device=device or "cuda",
-                                 dtype=torch.float64 if obj.dtype == np.float64 else torch.float32)
-        elif self.is_numpy:
-            if obj.dtype not in (np.float32, np.float64):
-                raise TypeError(f"{name}: unsupported dtype")
-            host = np.ascontiguousarray(obj)
-            t = torch.from_numpy(host)
-            self.t = t.to(device or "cuda", non_blocking=False)
-        elif isinstance(obj, torch.Tensor):
-            if obj.dtype not in (torch.float32, torch.float64):
+        self.writable = writable
+        self.is_numpy = False
+        if isinstance(obj, torch.Tensor):
+            code = _CODES.get(obj.dtype)
+            if code is None:
                 raise TypeError(f"{name}: unsupported dtype")
             if not obj.is_cuda:
-                self.t = obj.contiguous().to(device or "cuda")
+                t = obj.contiguous().to(device or "cuda")
             else:
-                self.t = obj if obj.is_contiguous() else obj.contiguous()
+                t = obj if obj.is_contiguous() else obj.contiguous()
+        elif isinstance(obj, np.ndarray):
+            self.is_numpy = True
+            if obj.dtype not in (np.float32, np.float64):
+                raise TypeError(f"{name}: unsupported dtype")
+            if fresh:
+                # wholly written by the call: nothing to copy to the device
+                t = torch.empty(obj.shape, device=device or "cuda",
+                                dtype=torch.float64 if obj.dtype == np.float64 else torch.float32)
+            else:
+                t = torch.from_numpy(np.ascontiguousarray(obj)).to(device or "cuda",
+                                                                   non_blocking=False)
+            code = _CODES[t.dtype]
         else:
             raise TypeError(f"{name} must be a numpy array or a torch tensor")
-        if self.t.dim() < 1:
+        shape = t.shape
+        if len(shape) < 1:
             raise ValueError("invalid shape")
-        self.lead = tuple(self.t.shape[:-1])
-        self.n = int(self.t.shape[-1])
-        if self.n < need:
-            raise ValueError(f"{name}: last axis has {self.n} entries, needs {need}")
-        self.rows = self.t.reshape(-1, self.n)
-        self.writable = writable
+        n = shape[-1]
+        if n < need:
+            raise ValueError(f"{name}: last axis has {n} entries, needs {need}")
+        self.t = t
+        self.dtype_code = code
+        self.lead = shape[:-1]
+        self.n = n
 
     @property
-    def dtype_code(self):
-        return _dtype_code(self.t.dtype)
+    def rows(self) -> torch.Tensor:
+        return self.t.reshape(-1, self.n)
 
     @property
     def batch(self) -> int:
-        return int(self.rows.shape[0])
+        return self.t.numel() // self.n
 
     def ptr(self) -> int:
-        return self.rows.data_ptr()
+        return self.t.data_ptr()
 
     def finish(self):
-        if not self.writable:
+        if not self.writable or self.t is self.obj:
             return
         if self.is_numpy:
-            np.copyto(self.obj, self.rows.reshape(self.obj.shape).cpu().numpy())
-        elif isinstance(self.obj, torch.Tensor) and self.rows.data_ptr() != self.obj.data_ptr():
-            self.obj.copy_(self.rows.reshape(self.obj.shape))
+            np.copyto(self.obj, self.t.reshape(self.obj.shape).cpu().numpy())
+        elif self.t.data_ptr() != self.obj.data_ptr():
+            self.obj.copy_(self.t.reshape(self.obj.shape))
 
 
 def _stream_ptr(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(t.get_device())
 
 
 def _check_same(out: _Arg, *others: _Arg):
@@ -306,19 +340,19 @@ def _check_same(out: _Arg, *others: _Arg):
 
 
 def _workspace(nbytes: int, device) -> torch.Tensor:
-    return torch.empty(max(int(nbytes), 1), dtype=torch.uint8, device=device)
+    return torch.empty((max(int(nbytes), 1),), dtype=torch.uint8, device=device)
 
 
 # ------------------------------------------------------------- free tensors
 def dense_ft_fma(out, lhs, rhs, basis, out_depth=-1, lhs_depth=-1, rhs_depth=-1):
     """out += lhs (x) rhs (roughpy/compute/_src/dense_basic.cpp:85-151)."""
     w, d = _basis_wd(basis)
-    size = int(_lib.lib.rpyb_tensor_size(w, d))
+    size = _size(w, d)
     o = _Arg(out, "out", size, True)
     lh = _Arg(lhs, "lhs", size, False, o.t.device)
     rh = _Arg(rhs, "rhs", size, False, o.t.device)
     _check_same(o, lh, rh)
-    b = _lib.bounds(0, out_depth, 0, lhs_depth, 0, rhs_depth)
+    b = _bounds(0, out_depth, 0, lhs_depth, 0, rhs_depth)
     _lib.check(_lib.lib.rpyb_ft_fma(o.dtype_code, w, d, o.batch, o.ptr(), lh.ptr(), rh.ptr(),
                                     o.n, lh.n, rh.n, b, _stream_ptr(o.t)))
     o.finish()
@@ -327,11 +361,11 @@ def dense_ft_fma(out, lhs, rhs, basis, out_depth=-1, lhs_depth=-1, rhs_depth=-1)
 def dense_ft_inplace_mul(lhs, rhs, basis, out_depth=-1, rhs_depth=-1):
     """lhs <- lhs (x) rhs (roughpy/compute/_src/dense_basic.cpp:193-237)."""
     w, d = _basis_wd(basis)
-    size = int(_lib.lib.rpyb_tensor_size(w, d))
+    size = _size(w, d)
     lh = _Arg(lhs, "lhs", size, True)
     rh = _Arg(rhs, "rhs", size, False, lh.t.device)
     _check_same(lh, rh)
-    b = _lib.bounds(0, out_depth, 0, rhs_depth)
+    b = _bounds(0, out_depth, 0, rhs_depth)
     ws = _workspace(_lib.lib.rpyb_ft_inplace_mul_workspace_size(lh.dtype_code, w, d, lh.batch),
                     lh.t.device)
     _lib.check(_lib.lib.rpyb_ft_inplace_mul(lh.dtype_code, w, d, lh.batch, lh.ptr(), rh.ptr(),
@@ -343,7 +377,7 @@ def dense_ft_inplace_mul(lhs, rhs, basis, out_depth=-1, rhs_depth=-1):
 def dense_ft_antipode(out, arg, basis, out_depth=-1, arg_depth=-1):
     """out <- antipode(arg) (roughpy/compute/_src/dense_basic.cpp:295-334)."""
     w, d = _basis_wd(basis)
-    size = int(_lib.lib.rpyb_tensor_size(w, d))
+    size = _size(w, d)
     o = _Arg(out, "out", size, True)
     a = _Arg(arg, "arg", size, False, o.t.device)
     _check_same(o, a)
@@ -355,7 +389,7 @@ def dense_ft_antipode(out, arg, basis, out_depth=-1, arg_depth=-1):
 def dense_ft_exp(out, arg, basis, out_depth=-1, arg_depth=-1):
     """out <- exp(arg) (roughpy/compute/_src/dense_intermediate.cpp:62-96)."""
     w, d = _basis_wd(basis)
-    size = int(_lib.lib.rpyb_tensor_size(w, d))
+    size = _size(w, d)
     o = _Arg(out, "out", size, True)
     a = _Arg(arg, "arg", size, False, o.t.device)
     _check_same(o, a)
@@ -369,7 +403,7 @@ def dense_ft_fmexp(out, multiplier, exponent, basis, out_depth=-1, multiplier_de
                    exponent_depth=-1):
     """out <- multiplier * exp(exponent) (dense_intermediate.cpp:127-196)."""
     w, d = _basis_wd(basis)
-    size = int(_lib.lib.rpyb_tensor_size(w, d))
+    size = _size(w, d)
     o = _Arg(out, "out", size, True)
     m = _Arg(multiplier, "multiplier", size, False, o.t.device)
     x = _Arg(exponent, "exponent", size, False, o.t.device)
@@ -385,7 +419,7 @@ def dense_ft_fmexp(out, multiplier, exponent, basis, out_depth=-1, multiplier_de
 def dense_ft_log(out, arg, basis, out_depth=-1, arg_depth=-1):
     """out <- log(arg), float64 series (dense_intermediate.cpp:204-294)."""
     w, d = _basis_wd(basis)
-    size = int(_lib.lib.rpyb_tensor_size(w, d))
+    size = _size(w, d)
     o = _Arg(out, "out", size, True)
     a = _Arg(arg, "arg", size, False, o.t.device)
     _check_same(o, a)
@@ -400,12 +434,12 @@ def dense_ft_adjoint_left_mul(out, operator, argument, basis, out_depth=-1, lhs_
                               rhs_depth=-1):
     """out += L*_operator(argument) (roughpy/compute/_src/dense_basic.cpp:387-440)."""
     w, d = _basis_wd(basis)
-    size = int(_lib.lib.rpyb_tensor_size(w, d))
+    size = _size(w, d)
     o = _Arg(out, "out", size, True)
     op = _Arg(operator, "operator", size, False, o.t.device)
     ar = _Arg(argument, "argument", size, False, o.t.device)
     _check_same(o, op, ar)
-    b = _lib.bounds(out_depth, lhs_depth, rhs_depth)
+    b = _bounds(out_depth, lhs_depth, rhs_depth)
     _lib.check(_lib.lib.rpyb_ft_adjoint_left_mul(o.dtype_code, w, d, o.batch, o.ptr(), op.ptr(),
                                                  ar.ptr(), o.n, op.n, ar.n, b, _stream_ptr(o.t)))
     o.finish()
@@ -456,12 +490,12 @@ def dense_tensor_to_lie(out, arg, t2l_matrix, lie_basis, tensor_basis, scale_fac
 def ft_mul_into(out, lhs, rhs, basis, rhs_depth=-1):
     """out <- lhs (x) rhs."""
     w, d = _basis_wd(basis)
-    size = int(_lib.lib.rpyb_tensor_size(w, d))
+    size = _size(w, d)
     o = _Arg(out, "out", size, True, fresh=True)
     lh = _Arg(lhs, "lhs", size, False, o.t.device)
     rh = _Arg(rhs, "rhs", size, False, o.t.device)
     _check_same(o, lh, rh)
-    b = _lib.bounds(0, -1, 0, -1, 0, rhs_depth)
+    b = _bounds(0, -1, 0, -1, 0, rhs_depth)
     _lib.check(_lib.lib.rpyb_ft_mul(o.dtype_code, w, d, o.batch, o.ptr(), lh.ptr(), rh.ptr(),
                                     o.n, lh.n, rh.n, b, _stream_ptr(o.t)))
     o.finish()
@@ -470,7 +504,7 @@ def ft_mul_into(out, lhs, rhs, basis, rhs_depth=-1):
 def ft_log_into(out, arg, basis):
     """out <- log(arg), its scalar taken as zero."""
     w, d = _basis_wd(basis)
-    size = int(_lib.lib.rpyb_tensor_size(w, d))
+    size = _size(w, d)
     o = _Arg(out, "out", size, True, fresh=True)
     a = _Arg(arg, "arg", size, False, o.t.device)
     _check_same(o, a)
@@ -483,7 +517,7 @@ def ft_log_into(out, arg, basis):
 def ft_adjoint_left_mul_into(out, operator, argument, basis):
     """out <- L*_operator(argument)."""
     w, d = _basis_wd(basis)
-    size = int(_lib.lib.rpyb_tensor_size(w, d))
+    size = _size(w, d)
     o = _Arg(out, "out", size, True, fresh=True)
     op = _Arg(operator, "operator", size, False, o.t.device)
     ar = _Arg(argument, "argument", size, False, o.t.device)

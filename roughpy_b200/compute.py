@@ -70,7 +70,7 @@ def _empty_like(data, n=None):
     """An uninitialised result for a call that writes all of it."""
     shape = data.shape if n is None else (*data.shape[:-1], n)
     if isinstance(data, torch.Tensor):
-        return torch.empty(shape, dtype=data.dtype, device=data.device)
+        return data.new_empty(shape)
     return np.empty(shape, dtype=data.dtype)
 
 
