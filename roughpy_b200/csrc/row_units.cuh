@@ -1,5 +1,5 @@
 // Units of a dense product with both factors' lower levels in shared memory:
-// shared by the series and the row-resident product kernels.
+// shared by the series, row-resident product and chain kernels.
 #pragma once
 
 #include <type_traits>
@@ -105,5 +105,45 @@ __device__ __forceinline__ void with_level(int k, Fn&& f)
     }
 }
 
+// Room for n words staged by stage_words, in float64 words (16-byte multiple).
+__host__ __device__ constexpr int stage_room(int n) { return (n + 3) & ~1; }
+
+// n words of a row into shared memory as float64, at the returned place in
+// `room` (16-byte aligned, stage_room(n) words).  Float64: asynchronous copies
+// of 16 bytes, with a word before the first aligned piece and after the last
+// where the row starts or ends between two (8-byte copies throughout kept the
+// load/store queue full: mio_throttle 16.7 cycles an issue, (8,5) 173 -> 167
+// us).  Float32: words, eight of a thread's in flight (16-byte loads, whose
+// odd words wait for a latency of their own, were slower: (2,12) 43 -> 58 us).
+template <typename T>
+__device__ __forceinline__ double* stage_words(double* room, const T* src, int n, int tid, int B)
+{
+    if constexpr (sizeof(T) == 8) {
+        const int head = (int)((reinterpret_cast<uintptr_t>(src) >> 3) & 1);
+        double* dst = room + head;
+        const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst);
+        const int pieces = (n - head) / 2;
+        for (int i = tid; i < pieces; i += B)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + (head + 2 * i) * 8),
+                         "l"(src + head + 2 * i)
+                         : "memory");
+        const int odd = tid == 0 && head ? 0 : tid == 1 && head + 2 * pieces < n ? n - 1 : -1;
+        if (odd >= 0)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(to + odd * 8), "l"(src + odd)
+                         : "memory");
+        return dst;
+    } else {
+        constexpr int kLoads = 8;
+        for (int i0 = tid; i0 < n; i0 += kLoads * B) {
+            T v[kLoads];
+#pragma unroll
+            for (int j = 0; j < kLoads; ++j) v[j] = i0 + j * B < n ? src[i0 + j * B] : T(0);
+#pragma unroll
+            for (int j = 0; j < kLoads; ++j)
+                if (i0 + j * B < n) room[i0 + j * B] = (double)v[j];
+        }
+        return room;
+    }
+}
 
 }  // namespace rpyb

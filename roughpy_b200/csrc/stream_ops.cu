@@ -63,74 +63,8 @@ int upload(const std::vector<E>& h, const E** out)
     return RPYB_OK;
 }
 
-// The packed form of the t2l map for the chain kernel's projection: rows sorted by entry
-// count (most first, stably) in groups of 32, each group padded to its
-// longest row with zero entries and stored lane-interleaved (entry j of lane
-// l at 32 j + l from the group's offset); an entry is 8 * column | value id
-// << 19 (the byte offset of a float64 word of the row, so the kernel's
-// gather needs no scaling).  False when a column does not fit 16 bits or
-// the number of distinct values 13 bits.
-bool pack_csr(const std::vector<int64_t>& hp, const std::vector<int64_t>& hi,
-              const std::vector<double>& hv, int64_t n_rows, int64_t n_cols,
-              std::vector<uint32_t>& goff, std::vector<uint32_t>& ent,
-              std::vector<uint32_t>& perm, std::vector<double>& tab)
-{
-    if (n_cols > 0x10000) return false;
-    std::map<uint64_t, uint32_t> ids;   // keyed by the value's bits
-    tab.clear();
-    auto id_of = [&](double v, uint32_t* out) {
-        uint64_t bits;
-        std::memcpy(&bits, &v, sizeof bits);
-        auto it = ids.find(bits);
-        if (it == ids.end()) {
-            if (tab.size() > 0x1fff) return false;
-            it = ids.emplace(bits, (uint32_t)tab.size()).first;
-            tab.push_back(v);
-        }
-        *out = it->second;
-        return true;
-    };
-    uint32_t zero_id = 0;
-    if (!id_of(0.0, &zero_id)) return false;
-    std::vector<int64_t> order(n_rows);
-    for (int64_t r = 0; r < n_rows; ++r) order[r] = r;
-    std::stable_sort(order.begin(), order.end(), [&](int64_t x, int64_t y) {
-        return hp[x + 1] - hp[x] > hp[y + 1] - hp[y];
-    });
-    const int64_t groups = (n_rows + 31) / 32;
-    goff.assign(groups + 1, 0);
-    perm.assign(groups * 32, 0xffffffffu);
-    ent.clear();
-    for (int64_t g = 0; g < groups; ++g) {
-        int64_t len = 0;
-        for (int l = 0; l < 32 && g * 32 + l < n_rows; ++l) {
-            const int64_t r = order[g * 32 + l];
-            len = std::max<int64_t>(len, hp[r + 1] - hp[r]);
-            perm[g * 32 + l] = (uint32_t)r;
-        }
-        for (int64_t j = 0; j < len; ++j)
-            for (int l = 0; l < 32; ++l) {
-                uint32_t e = zero_id << 19;
-                if (g * 32 + l < n_rows) {
-                    const int64_t r = order[g * 32 + l];
-                    if (j < hp[r + 1] - hp[r]) {
-                        const int64_t k = hp[r] + j;
-                        uint32_t vid;
-                        if (hi[k] < 0 || hi[k] >= n_cols || !id_of(hv[k], &vid)) return false;
-                        e = ((uint32_t)hi[k] << 3) | (vid << 19);
-                    }
-                }
-                ent.push_back(e);
-            }
-        if (ent.size() >= ((size_t)1 << 32)) return false;
-        goff[g + 1] = (uint32_t)ent.size();
-    }
-    return true;
-}
-
 int upload_csr(const Geometry& g, int which, int64_t n_rows, const int64_t** ptr,
-               const int64_t** idx, const double** val, PackedMap* packed,
-               LieMapsDev* packed_into = nullptr)
+               const int64_t** idx, const double** val, PackedMap* packed)
 {
     const int64_t nnz = rpyb_lie_map_csr(g.width, g.depth, which, nullptr, nullptr, nullptr);
     if (nnz < 0) return (int)nnz;
@@ -145,21 +79,6 @@ int upload_csr(const Geometry& g, int which, int64_t n_rows, const int64_t** ptr
         const int rc = upload(block, &d_block);
         if (rc) return rc;
         packed->block = d_block;
-    }
-    if (packed_into) {
-        std::vector<uint32_t> goff, ent, perm;
-        std::vector<double> tab;
-        if (pack_csr(hp, hi, hv, n_rows, g.size(), goff, ent, perm, tab)) {
-            int rc;
-            if ((rc = upload(goff, &packed_into->t2l_goff)) ||
-                (rc = upload(ent, &packed_into->t2l_ent)) ||
-                (rc = upload(perm, &packed_into->t2l_perm)) ||
-                (rc = upload(tab, &packed_into->t2l_tab)))
-                return rc;
-            packed_into->t2l_slots = (int64_t)ent.size();
-            packed_into->t2l_groups = (int64_t)goff.size() - 1;
-            packed_into->t2l_ntab = (int64_t)tab.size();
-        }
     }
     int64_t* dp = nullptr;
     int64_t* di = nullptr;
@@ -176,6 +95,8 @@ int upload_csr(const Geometry& g, int which, int64_t n_rows, const int64_t** ptr
     return RPYB_OK;
 }
 
+
+
 // Pinned staging for host -> device uploads of index lists.  A copy from
 // pageable memory makes cudaMemcpyAsync wait for the stream, which would
 // serialise the host work of the next query chunk behind the device work of
@@ -186,6 +107,8 @@ struct PinnedStage {
     size_t cap = 0;
     cudaEvent_t ev = nullptr;
 };
+
+}  // namespace
 
 int upload_async(void* dst, const void* src, size_t bytes, cudaStream_t s)
 {
@@ -212,504 +135,6 @@ int upload_async(void* dst, const void* src, size_t bytes, cudaStream_t s)
     return RPYB_OK;
 }
 
-
-// ------------------------------------------------------------------------
-// Fused chain products: acc[q] <- src[r_0] * src[r_1] * ... (the unit for an
-// empty list), or its float64 log, one block per row q, so that the running
-// product never leaves the SM.  Its levels below the top are in shared
-// memory (float64, double-buffered); its top level is spread over the
-// threads' registers.  That split is exact: a top-level output word reads
-// the lower levels of the left operand, the factor's words and only its own
-// top-level word of the left operand (times the factor's scalar), so no
-// thread needs another thread's top-level words.  A product is split like
-// the blocked product kernel: a unit owns D first letters x V last letters
-// of one middle part at a level k >= 2; levels 0 and 1 are done by the first
-// threads.  Every thread owns TU top-level units (flat units tid, tid + B,
-// ...); the lower units follow in the same flat order from the level below
-// the top down, so the threads that take one more unit take a light one.
-// The first factor is copied, not multiplied by the unit.  Factors are read
-// from global memory (queries share them, so the popular ones stay in L2),
-// and the next one is prefetched into L2 while a product runs.
-struct ChainArgs {
-    int64_t T = 0;
-    int64_t db[kMaxDepth + 2] = {};
-    int64_t pw[kMaxDepth + 1] = {};
-    int64_t lo_begin[kMaxDepth + 2] = {};   // first lower unit of level k (2 <= k < depth)
-    int64_t utop = 0, ulow = 0;             // top-level and lower units
-    int depth = 0;
-    int64_t n = 0;
-    const int64_t* off = nullptr;      // [n + 1] into rows
-    const int64_t* rows = nullptr;     // source row of each factor
-    const void* src = nullptr;         // [*, T] factors (float or double)
-    double* acc = nullptr;             // [n, T] out
-    int log_out = 0;                   // write log(product) instead of the product
-    void* dst = nullptr;               // instead of acc: rows dst_rows[q] of this
-    const int64_t* dst_rows = nullptr; // [*, T] array of the factors' type
-    // log_out with lie != null: the block projects its log onto the Hall
-    // basis through the packed t2l map and writes lie[q * ld_lie + row]
-    // instead of the log tensor
-    double* lie = nullptr;
-    int64_t ld_lie = 0, lie_dim = 0, pgroups = 0;
-    const uint32_t* pgoff = nullptr;
-    const uint32_t* pent = nullptr;
-    const uint32_t* pperm = nullptr;
-    const double* ptab = nullptr;
-};
-
-constexpr int kChainThreads = 512;
-
-// out[D][V] (+)= sum over s = 1..k-1 of lhs level k-s (x) rhs level s at the
-// unit (rp, c0) of level k: the left factor's D words of first letters u at
-// middle part rp's prefix, the right factor's V words after it.  KC > 0 fixes
-// k = KC at compile time; the loop is then unrolled, which lets the loads of
-// all split points be issued together.
-template <int D, int V, typename TR, bool GLOBAL_RHS, int KC = 0>
-__device__ __forceinline__ void unit_splits(double (&acc)[D][V], const double* lhs, const TR* rhs,
-                                            const ChainArgs& a, int k, uint32_t rp, int c0)
-{
-    uint32_t qq = rp;
-    uint32_t m = 0;
-    if constexpr (KC > 0) k = KC;
-#pragma unroll
-    for (int s = 1; s <= (KC > 0 ? KC : k) - 1; ++s) {
-        const int p = k - s;
-        double lv[D];
-        double rv[V];
-        const double* lp = lhs + a.db[p] + qq;
-        const uint32_t dp1 = (uint32_t)a.pw[p - 1];
-#pragma unroll
-        for (int u = 0; u < D; ++u) lv[u] = lp[u * dp1];
-        const TR* rq = rhs + a.db[s] + (int64_t)m * D + c0;
-#pragma unroll
-        for (int j = 0; j < V; ++j) {
-            if constexpr (GLOBAL_RHS) rv[j] = (double)__ldg(rq + j);
-            else rv[j] = (double)rq[j];
-        }
-#pragma unroll
-        for (int u = 0; u < D; ++u)
-#pragma unroll
-            for (int j = 0; j < V; ++j) acc[u][j] = fma(lv[u], rv[j], acc[u][j]);
-        const uint32_t q2 = qq / (uint32_t)D;
-        m += (qq - q2 * (uint32_t)D) * (uint32_t)a.pw[s - 1];
-        qq = q2;
-    }
-}
-
-// the level and position of lower unit li (levels depth-1 down to 2)
-template <int D, int V>
-__device__ __forceinline__ void lower_unit(const ChainArgs& a, int64_t li, int& k, uint32_t& rp,
-                                           int& c0, int64_t& obase, int64_t& dk1)
-{
-    constexpr int NB = D / V;
-    k = a.depth - 1;
-    while (k > 2 && li >= a.lo_begin[k - 1]) --k;
-    const int64_t unit = li - a.lo_begin[k];
-    rp = (uint32_t)(unit / NB);
-    c0 = (int)(unit - (int64_t)rp * NB) * V;
-    dk1 = a.pw[k - 1];
-    obase = a.db[k] + (int64_t)rp * D + c0;
-}
-
-// NT > 0: the depth is NT (the top level's split loop is unrolled)
-#ifndef RPYB_CHAIN_MIN_BLOCKS
-#define RPYB_CHAIN_MIN_BLOCKS 1
-#endif
-template <typename TS, int D, int V, int TU, int NT>
-__global__ void __launch_bounds__(kChainThreads, RPYB_CHAIN_MIN_BLOCKS)
-chain_products_kernel(const ChainArgs a)
-{
-    constexpr int NB = D / V;
-    extern __shared__ __align__(16) unsigned char chain_smem[];
-    const int N = a.depth;
-    const int64_t TL = a.db[N];   // words below the top level
-    double* lo0 = reinterpret_cast<double*>(chain_smem);
-    double* lo1 = lo0 + TL;
-    const int tid = (int)threadIdx.x;
-    const int B = (int)blockDim.x;
-    const TS* src = static_cast<const TS*>(a.src);
-    const int64_t tdk1 = a.pw[N - 1];
-    // this thread's top-level units: output words tbase[t] + u * tdk1 + j
-    int64_t tbase[TU];
-    uint32_t trp[TU];
-    int tc0[TU];
-    bool town[TU];
-#pragma unroll
-    for (int t = 0; t < TU; ++t) {
-        const int64_t f = tid + (int64_t)t * B;
-        town[t] = f < a.utop;
-        trp[t] = town[t] ? (uint32_t)(f / NB) : 0u;
-        tc0[t] = town[t] ? (int)(f - (int64_t)trp[t] * NB) * V : 0;
-        tbase[t] = a.db[N] + (int64_t)trp[t] * D + tc0[t];
-    }
-    int64_t f_low = tid;   // this thread's first lower unit (flat index)
-    while (f_low < a.utop) f_low += B;
-
-    for (int64_t q = blockIdx.x; q < a.n; q += gridDim.x) {
-        const int64_t o0 = a.off[q], o1 = a.off[q + 1];
-        double* accq = a.acc ? a.acc + q * a.T : nullptr;
-        TS* dstq = a.dst ? static_cast<TS*>(a.dst) + a.dst_rows[q] * a.T : nullptr;
-        if (o0 == o1 && a.lie) {   // the log of the unit: zero coordinates
-            for (int64_t r = tid; r < a.lie_dim; r += B) a.lie[q * a.ld_lie + r] = 0.0;
-            continue;
-        }
-        if (o0 == o1) {   // the unit, or its log
-            for (int64_t i = tid; i < a.T; i += B) {
-                const double v = (i == 0 && !a.log_out) ? 1.0 : 0.0;
-                if (dstq) dstq[i] = (TS)v;
-                else accq[i] = v;
-            }
-            continue;
-        }
-        double* cur = lo0;
-        double* nxt = lo1;
-        __syncthreads();   // the previous row's reads of the buffers are done
-        const TS* first = src + a.rows[o0] * a.T;
-        for (int64_t i = tid; i < TL; i += B) cur[i] = (double)__ldg(first + i);
-        double top[TU][D][V];
-#pragma unroll
-        for (int t = 0; t < TU; ++t)
-#pragma unroll
-            for (int u = 0; u < D; ++u)
-#pragma unroll
-                for (int j = 0; j < V; ++j)
-                    top[t][u][j] = town[t] ? (double)__ldg(first + tbase[t] + u * tdk1 + j) : 0.0;
-        for (int64_t r = o0 + 1; r < o1; ++r) {
-            __syncthreads();
-            const TS* node = src + a.rows[r] * a.T;
-            if (r + 1 < o1) {
-                const char* nn = reinterpret_cast<const char*>(src + a.rows[r + 1] * a.T);
-                const int64_t bytes = a.T * (int64_t)sizeof(TS);
-                for (int64_t l = (int64_t)tid * 128; l < bytes; l += (int64_t)B * 128)
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(nn + l));
-            }
-            const double node0 = (double)__ldg(node);
-            const double c0v = cur[0];
-            if (tid == 0) nxt[0] = c0v * node0;
-            if (tid < D) nxt[1 + tid] = cur[1 + tid] * node0 + c0v * (double)__ldg(node + 1 + tid);
-            // top-level units, in registers
-#pragma unroll
-            for (int t = 0; t < TU; ++t) {
-                if (!town[t]) continue;
-#pragma unroll
-                for (int u = 0; u < D; ++u)
-#pragma unroll
-                    for (int j = 0; j < V; ++j) top[t][u][j] *= node0;
-                unit_splits<D, V, TS, true, NT>(top[t], cur, node, a, N, trp[t], tc0[t]);
-#pragma unroll
-                for (int u = 0; u < D; ++u)
-#pragma unroll
-                    for (int j = 0; j < V; ++j)
-                        top[t][u][j] =
-                            fma(c0v, (double)__ldg(node + tbase[t] + u * tdk1 + j), top[t][u][j]);
-            }
-            // lower units, in shared memory
-            for (int64_t f = f_low; f < a.utop + a.ulow; f += B) {
-                int k, c0;
-                uint32_t rp;
-                int64_t obase, dk1;
-                lower_unit<D, V>(a, f - a.utop, k, rp, c0, obase, dk1);
-                double acc[D][V];
-#pragma unroll
-                for (int u = 0; u < D; ++u)
-#pragma unroll
-                    for (int j = 0; j < V; ++j) acc[u][j] = cur[obase + u * dk1 + j] * node0;
-                unit_splits<D, V, TS, true>(acc, cur, node, a, k, rp, c0);
-#pragma unroll
-                for (int u = 0; u < D; ++u)
-#pragma unroll
-                    for (int j = 0; j < V; ++j)
-                        nxt[obase + u * dk1 + j] =
-                            fma(c0v, (double)__ldg(node + obase + u * dk1 + j), acc[u][j]);
-            }
-            __syncthreads();
-            double* t = cur;
-            cur = nxt;
-            nxt = t;
-        }
-        if (a.log_out) {
-            // log(X) of the product X by the Horner steps of the float64 log
-            // (free_tensor_log.hpp:23-38): with Y = X - X_0 and R = 0, for
-            // deg = N down to 1, R <- (R + c_deg) Y truncated to the levels
-            // N - deg + 1 and below, c_deg = (-1)^(deg+1) / deg.  Y's lower
-            // levels stay in `cur`, its top level in `top`; R's lower levels
-            // ping-pong between `nxt` and a third buffer.  R's top level is
-            // formed only in the last step, in place of Y's own top words.
-            double* rc = nxt;
-            double* rn = lo0 + 2 * TL;   // the third buffer
-            for (int s = 1; s <= N; ++s) {
-                const int deg = N - s + 1;
-                const double c = (deg % 2 == 0) ? -1.0 / (double)deg : 1.0 / (double)deg;
-                __syncthreads();   // R's previous step (and Y) complete
-                if (tid < D) rn[1 + tid] = c * cur[1 + tid];
-                if (s == N) {
-#pragma unroll
-                    for (int t = 0; t < TU; ++t) {
-                        if (!town[t]) continue;
-#pragma unroll
-                        for (int u = 0; u < D; ++u)
-#pragma unroll
-                            for (int j = 0; j < V; ++j) top[t][u][j] *= c;
-                        unit_splits<D, V, double, false, NT>(top[t], rc, cur, a, N, trp[t],
-                                                             tc0[t]);
-                    }
-                }
-                for (int64_t f = f_low; f < a.utop + a.ulow; f += B) {
-                    int k, c0;
-                    uint32_t rp;
-                    int64_t obase, dk1;
-                    lower_unit<D, V>(a, f - a.utop, k, rp, c0, obase, dk1);
-                    if (k > s) continue;
-                    double acc[D][V];
-#pragma unroll
-                    for (int u = 0; u < D; ++u)
-#pragma unroll
-                        for (int j = 0; j < V; ++j) acc[u][j] = c * cur[obase + u * dk1 + j];
-                    unit_splits<D, V, double, false>(acc, rc, cur, a, k, rp, c0);
-#pragma unroll
-                    for (int u = 0; u < D; ++u)
-#pragma unroll
-                        for (int j = 0; j < V; ++j) rn[obase + u * dk1 + j] = acc[u][j];
-                }
-                double* t = rc;
-                rc = rn;
-                rn = t;
-            }
-            __syncthreads();
-            if (tid == 0) rc[0] = 0.0;
-            __syncthreads();
-            cur = rc;
-        }
-        if (a.lie) {
-            // the whole log into shared memory (after the three log
-            // buffers), then one warp per group of 32 Lie rows; an entry is
-            // 8 * column | value id << 19 (see pack_csr)
-            double* xs = lo0 + 3 * TL;
-            for (int64_t i = tid; i < TL; i += B) xs[i] = cur[i];
-#pragma unroll
-            for (int t = 0; t < TU; ++t)
-                if (town[t])
-#pragma unroll
-                    for (int u = 0; u < D; ++u)
-#pragma unroll
-                        for (int j = 0; j < V; ++j) xs[tbase[t] + u * tdk1 + j] = top[t][u][j];
-            __syncthreads();
-            const unsigned char* xb = reinterpret_cast<const unsigned char*>(xs);
-            const int lane = tid & 31, nw = B >> 5;
-            double* yq = a.lie + q * a.ld_lie;
-            for (int64_t gi = tid >> 5; gi < a.pgroups; gi += nw) {
-                double accp = 0.0;
-                const uint32_t e1 = __ldg(a.pgoff + gi + 1);
-#pragma unroll 4
-                for (uint32_t k = __ldg(a.pgoff + gi) + lane; k < e1; k += 32) {
-                    const uint32_t w = __ldg(a.pent + k);
-                    accp = fma(__ldg(a.ptab + (w >> 19)),
-                               *reinterpret_cast<const double*>(xb + (w & 0x7ffffu)), accp);
-                }
-                const uint32_t row = __ldg(a.pperm + gi * 32 + lane);
-                if (row != 0xffffffffu) yq[row] = accp;
-            }
-            continue;
-        }
-        if (dstq) {
-            // straight into the factors' array, rounded once to its type
-            for (int64_t i = tid; i < TL; i += B) dstq[i] = (TS)cur[i];
-#pragma unroll
-            for (int t = 0; t < TU; ++t)
-                if (town[t])
-#pragma unroll
-                    for (int u = 0; u < D; ++u)
-#pragma unroll
-                        for (int j = 0; j < V; ++j) dstq[tbase[t] + u * tdk1 + j] = (TS)top[t][u][j];
-        } else {
-            for (int64_t i = tid; i < TL; i += B) accq[i] = cur[i];
-#pragma unroll
-            for (int t = 0; t < TU; ++t)
-                if (town[t])
-#pragma unroll
-                    for (int u = 0; u < D; ++u)
-#pragma unroll
-                        for (int j = 0; j < V; ++j) accq[tbase[t] + u * tdk1 + j] = top[t][u][j];
-        }
-    }
-}
-
-// width -> last-letter block of the chain kernel (0: not available)
-int chain_v(int width)
-{
-    switch (width) {
-        case 2: return 2;
-        case 3: return 3;
-        case 4: return 4;
-        case 5: return 1;
-        case 6: return 3;
-        case 8: return 2;
-        default: return 0;
-    }
-}
-
-// top-level units a thread holds in registers (0: the shape is not
-// covered); two only where two units' words fit the registers unspilled
-int chain_tu(const Geometry& g)
-{
-    const int V = chain_v(g.width);
-    if (V == 0 || g.depth < 2) return 0;
-    const int64_t utop = g.pw[g.depth - 2] * (g.width / V);
-    const int64_t tu = (utop + kChainThreads - 1) / kChainThreads;
-    if (tu == 1) return 1;
-    if (tu == 2 && g.width <= 3) return 2;
-    return 0;
-}
-
-using ChainFn = void (*)(ChainArgs);
-
-template <typename TS, int NT>
-ChainFn chain_fn_nt(int width, int tu)
-{
-    if (tu == 2) {
-        switch (width) {
-            case 2: return &chain_products_kernel<TS, 2, 2, 2, NT>;
-            case 3: return &chain_products_kernel<TS, 3, 3, 2, NT>;
-            default: return nullptr;
-        }
-    }
-    switch (width) {
-        case 2: return &chain_products_kernel<TS, 2, 2, 1, NT>;
-        case 3: return &chain_products_kernel<TS, 3, 3, 1, NT>;
-        case 4: return &chain_products_kernel<TS, 4, 4, 1, NT>;
-        case 5: return &chain_products_kernel<TS, 5, 1, 1, NT>;
-        case 6: return &chain_products_kernel<TS, 6, 3, 1, NT>;
-        case 8: return &chain_products_kernel<TS, 8, 2, 1, NT>;
-        default: return nullptr;
-    }
-}
-
-// depths 5 and 6 get a kernel with the top level's split loop unrolled
-template <typename TS>
-ChainFn chain_fn(int width, int depth, int tu)
-{
-    if (depth == 5) return chain_fn_nt<TS, 5>(width, tu);
-    if (depth == 6) return chain_fn_nt<TS, 6>(width, tu);
-    return chain_fn_nt<TS, 0>(width, tu);
-}
-
-constexpr int64_t kChainSmemLimit = 200 * 1024;
-
-}  // namespace
-
-bool chain_products_available(const Geometry& g)
-{
-    return chain_tu(g) > 0 && 3 * g.db[g.depth] * 8 <= kChainSmemLimit;
-}
-
-static int chain_launch(int src_mode, const Geometry& g, int64_t n, double* acc, const void* src,
-                        const std::vector<int64_t>& off, const std::vector<int64_t>& src_rows,
-                        bool log_out, void* dst, const std::vector<int64_t>* dst_rows,
-                        cudaStream_t s, const LieMapsDev* maps = nullptr, double* lie = nullptr,
-                        int64_t ld_lie = 0);
-
-int chain_products(int src_mode, const Geometry& g, int64_t n, double* acc, const void* src,
-                   const std::vector<int64_t>& off, const std::vector<int64_t>& src_rows,
-                   bool log_out, cudaStream_t s)
-{
-    return chain_launch(src_mode, g, n, acc, src, off, src_rows, log_out, nullptr, nullptr, s);
-}
-
-int chain_products_into(int src_mode, const Geometry& g, int64_t n, void* nodes,
-                        const std::vector<int64_t>& off, const std::vector<int64_t>& src_rows,
-                        const std::vector<int64_t>& dst_rows, cudaStream_t s)
-{
-    return chain_launch(src_mode, g, n, nullptr, nodes, off, src_rows, false, nodes, &dst_rows, s);
-}
-
-bool chain_lie_available(const Geometry& g, const LieMapsDev& maps)
-{
-    return chain_products_available(g) && maps.t2l_ent &&
-           (size_t)(3 * g.db[g.depth] + g.size()) * 8 <= (size_t)kChainSmemLimit;
-}
-
-int chain_products_lie(int src_mode, const Geometry& g, int64_t n, const void* src,
-                       const std::vector<int64_t>& off, const std::vector<int64_t>& src_rows,
-                       const LieMapsDev& maps, double* lie, int64_t ld_lie, cudaStream_t s)
-{
-    if (!chain_lie_available(g, maps)) return fail(RPYB_E_UNSUPPORTED, "no fused projection for this shape");
-    return chain_launch(src_mode, g, n, nullptr, src, off, src_rows, true, nullptr, nullptr, s,
-                        &maps, lie, ld_lie);
-}
-
-static int chain_launch(int src_mode, const Geometry& g, int64_t n, double* acc, const void* src,
-                        const std::vector<int64_t>& off, const std::vector<int64_t>& src_rows,
-                        bool log_out, void* dst, const std::vector<int64_t>* dst_rows,
-                        cudaStream_t s, const LieMapsDev* maps, double* lie, int64_t ld_lie)
-{
-    if (n == 0) return RPYB_OK;
-    if (!chain_products_available(g)) return fail(RPYB_E_UNSUPPORTED, "no chain kernel for this shape");
-    if (off[n] == 0 && lie) {
-        RPYB_CUDA(cudaMemset2DAsync(lie, (size_t)ld_lie * 8, 0, (size_t)maps->lie_dim * 8,
-                                    (size_t)n, s));
-        return RPYB_OK;
-    }
-    if (off[n] == 0 && !dst) {
-        if (log_out) {
-            RPYB_CUDA(cudaMemsetAsync(acc, 0, (size_t)(n * g.size() * 8), s));
-            return RPYB_OK;
-        }
-        return unit_rows(RPYB_F64, acc, g.size(), g.size(), nullptr, n, s);
-    }
-    const int V = chain_v(g.width), NB = g.width / V, tu = chain_tu(g);
-    ChainArgs a;
-    a.T = g.size();
-    for (int k = 0; k <= kMaxDepth + 1; ++k) a.db[k] = g.db[k];
-    for (int k = 0; k <= kMaxDepth; ++k) a.pw[k] = g.pw[k];
-    a.utop = g.pw[g.depth - 2] * NB;
-    // lower levels depth-1 down to 2, in that order
-    int64_t u = 0;
-    for (int k = g.depth - 1; k >= 2; --k) {
-        a.lo_begin[k] = u;
-        u += g.pw[k - 2] * NB;
-    }
-    a.lo_begin[1] = u;
-    a.ulow = u;
-    a.depth = g.depth;
-    a.n = n;
-    // offsets and rows in one upload
-    std::vector<int64_t> packed(off.begin(), off.begin() + n + 1);
-    packed.insert(packed.end(), src_rows.begin(), src_rows.begin() + off[n]);
-    if (dst) packed.insert(packed.end(), dst_rows->begin(), dst_rows->begin() + n);
-    Scratch sc(nullptr, 0, s);
-    void* mem = nullptr;
-    int rc;
-    if ((rc = sc.get(packed.size() * 8, &mem))) return rc;
-    int64_t* d = static_cast<int64_t*>(mem);
-    if ((rc = upload_async(d, packed.data(), packed.size() * 8, s))) return rc;
-    a.off = d;
-    a.rows = d + n + 1;
-    a.src = src;
-    a.acc = acc;
-    a.log_out = log_out ? 1 : 0;
-    a.dst = dst;
-    a.dst_rows = dst ? d + n + 1 + off[n] : nullptr;
-    if (lie) {
-        a.lie = lie;
-        a.ld_lie = ld_lie;
-        a.lie_dim = maps->lie_dim;
-        a.pgroups = maps->t2l_groups;
-        a.pgoff = maps->t2l_goff;
-        a.pent = maps->t2l_ent;
-        a.pperm = maps->t2l_perm;
-        a.ptab = maps->t2l_tab;
-    }
-    const size_t smem =
-        (size_t)((log_out ? 3 : 2) * g.db[g.depth] * 8) + (lie ? (size_t)g.size() * 8 : 0);
-    const unsigned grid = (unsigned)std::min<int64_t>(n, 1 << 20);
-    ChainFn fn = src_mode == RPYB_F64 ? chain_fn<double>(g.width, g.depth, tu)
-                                      : chain_fn<float>(g.width, g.depth, tu);
-    if (smem > 48 * 1024)
-        RPYB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    fn<<<grid, kChainThreads, smem, s>>>(a);
-    RPYB_CUDA(cudaGetLastError());
-    return RPYB_OK;
-}
-
 int lie_maps_device(const Geometry& g, const LieMapsDev** out)
 {
     static std::mutex mu;
@@ -733,7 +158,7 @@ int lie_maps_device(const Geometry& g, const LieMapsDev** out)
     e.lie_dim = lie_dim;
     int rc;
     if ((rc = upload_csr(g, 0, g.size(), &e.l2t_ptr, &e.l2t_idx, &e.l2t_val, &e.l2t)) ||
-        (rc = upload_csr(g, 1, lie_dim, &e.t2l_ptr, &e.t2l_idx, &e.t2l_val, &e.t2l, &e)))
+        (rc = upload_csr(g, 1, lie_dim, &e.t2l_ptr, &e.t2l_idx, &e.t2l_val, &e.t2l)))
         return rc;
     entries[n_entries] = e;
     *out = &entries[n_entries++];

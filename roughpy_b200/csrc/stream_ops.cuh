@@ -23,18 +23,6 @@ struct LieMapsDev {
     const int64_t* t2l_ptr = nullptr;   // lie_dim rows x tensor_size
     const int64_t* t2l_idx = nullptr;
     const double* t2l_val = nullptr;
-    // t2l packed for the projection inside the chain kernel (null when a column
-    // does not fit 16 bits or the number of distinct values 13 bits).  Rows sorted by
-    // entry count, in groups of 32 (one per warp lane), each group padded to
-    // its longest row; entry j of lane l of group g is t2l_ent[t2l_goff[g] +
-    // 32 j + l] = 8 * column | (value id << 19), the distinct values (and a zero
-    // for the padding) in t2l_tab; t2l_perm[32 g + l] is the lane's row, or
-    // 0xffffffff past the last row.
-    const uint32_t* t2l_goff = nullptr;   // groups + 1
-    const uint32_t* t2l_ent = nullptr;
-    const uint32_t* t2l_perm = nullptr;   // 32 * groups
-    const double* t2l_tab = nullptr;
-    int64_t t2l_slots = 0, t2l_groups = 0, t2l_ntab = 0;
     PackedMap l2t, t2l;   // for launch_packed_map (block null: not packable)
 };
 int lie_maps_device(const Geometry& g, const LieMapsDev** out);
@@ -47,6 +35,10 @@ int lie_project(int dtype, const Geometry& g, const LieMapsDev& maps, int64_t m,
 // x[b] <- l2t(lie[b]) for m rows (assigning, as above)
 int lie_embed(int dtype, const Geometry& g, const LieMapsDev& maps, int64_t m, void* x,
               int64_t ld_x, const void* lie, int64_t ld_lie, cudaStream_t s);
+
+// Copies host bytes to the device on s through pinned staging: the host buffer
+// may be reused when the call returns.
+int upload_async(void* dst, const void* src, size_t bytes, cudaStream_t s);
 
 // rows idx[i] (or i) of `out` (stride ld) <- the unit tensor
 int unit_rows(int mode, void* out, int64_t ld, int64_t cols, const int64_t* idx, int64_t n,
@@ -62,12 +54,10 @@ int ordered_products(int acc_mode, int src_mode, const Geometry& g, int64_t n, v
                      const std::vector<int64_t>& src_rows, cudaStream_t s);
 
 // acc[q] <- src[r_0] * src[r_1] * ... (float64; the unit for an empty list),
-// or its float64 log when log_out is set (the log's Horner steps run in the
-// same block on the product still on the SM), fused: one block per row keeps
-// the running product on the SM across its whole list of factors (levels
-// below the top in shared memory, the top level in registers).  Available
-// for widths 2..6 and 8 when the top level fits the block's registers and
-// three copies of its lower levels 200 KB of shared memory.
+// or its float64 log when log_out is set, fused: one block per row keeps the
+// running product in shared memory across its whole list of factors
+// (chain.cu).  Available for widths 2..8 from depth 2 while a row and three
+// copies of its lower levels fit.
 bool chain_products_available(const Geometry& g);
 int chain_products(int src_mode, const Geometry& g, int64_t n, double* acc, const void* src,
                    const std::vector<int64_t>& off, const std::vector<int64_t>& src_rows,
@@ -81,7 +71,7 @@ int chain_products_into(int src_mode, const Geometry& g, int64_t n, void* nodes,
                         const std::vector<int64_t>& dst_rows, cudaStream_t s);
 // log(product) projected onto the Hall basis inside the chain kernel (the
 // log never leaves the SM): Lie coordinates to lie[i * ld_lie + r].  Needs
-// the packed t2l map and room for the whole log in shared memory.
+// the packed t2l map.
 bool chain_lie_available(const Geometry& g, const LieMapsDev& maps);
 int chain_products_lie(int src_mode, const Geometry& g, int64_t n, const void* src,
                        const std::vector<int64_t>& off, const std::vector<int64_t>& src_rows,
