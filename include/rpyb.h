@@ -395,9 +395,9 @@ RPYB_API int rpyb_sparse_map(int dtype, int64_t n_rows, int64_t n_cols, int64_t 
                              int64_t ld_y, int64_t ld_x, double scale, void* stream);
 
 /*
- * Packs a CSR matrix (host arrays) for rpyb_sparse_map_packed: returns the
- * block's size in bytes, writes the block when `block` is not null (of at
- * least that many bytes), and its three counts to layout.  Entries whose
+ * Packs a CSR matrix (host arrays) for rpyb_sparse_map_packed: writes the block
+ * and its three counts (layout) and returns the block's size in bytes.  With a
+ * null block, returns room enough for it.  Entries whose
  * column lies outside [0, n_cols) are left out.  RPYB_E_UNSUPPORTED when the
  * matrix has over 2^20 columns or over 4096 distinct values.  The caller
  * copies the block to the device.

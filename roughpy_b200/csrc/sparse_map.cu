@@ -14,6 +14,7 @@
 // 94 us (HBM time of x and y: 57 and 28 us).
 #include <algorithm>
 #include <cstring>
+#include <new>
 #include <numeric>
 #include <unordered_map>
 
@@ -180,74 +181,127 @@ int launch_map_rows(const MapArgs& a, T* y, const T* x, cudaStream_t s)
 
 }  // namespace
 
+// Where the rows of a map go: its groups' rows and longest counts, heaviest
+// group first.
+struct PackLayout {
+    std::vector<uint32_t> count;     // entries kept, per row
+    std::vector<int64_t> order;      // rows, 32 to a group
+    std::vector<uint32_t> longest;   // per group of `order`
+    std::vector<int64_t> by_len;     // groups, longest first
+    int64_t entries = 0, slots = 0;
+};
+
+static bool pack_layout(int64_t n_rows, int64_t n_cols, const int64_t* ptr, const int64_t* idx,
+                        PackLayout& l)
+{
+    if (n_cols > (int64_t(1) << kColBits) || n_rows >= 0x7fffffff) return false;
+    l.count.assign(n_rows, 0);
+    for (int64_t r = 0; r < n_rows; ++r) {
+        uint32_t c = 0;
+        for (int64_t k = ptr[r]; k < ptr[r + 1]; ++k) c += (uint64_t)idx[k] < (uint64_t)n_cols;
+        l.count[r] = c;
+        l.entries += c;
+    }
+    l.order.resize(n_rows);
+    std::iota(l.order.begin(), l.order.end(), int64_t(0));
+    for (int64_t r0 = 0; l.entries >= kSortEntries * n_rows && r0 < n_rows; r0 += kSortWindow)
+        std::stable_sort(l.order.begin() + r0, l.order.begin() + std::min(r0 + kSortWindow, n_rows),
+                         [&](int64_t p, int64_t q) { return l.count[p] > l.count[q]; });
+    const int64_t groups = (n_rows + 31) / 32;
+    l.longest.assign(groups, 0);
+    for (int64_t g = 0; g < groups; ++g)
+        for (int64_t i = g * 32; i < std::min(g * 32 + 32, n_rows); ++i)
+            l.longest[g] = std::max(l.longest[g], l.count[l.order[i]]);
+    l.by_len.resize(groups);
+    std::iota(l.by_len.begin(), l.by_len.end(), int64_t(0));
+    std::stable_sort(l.by_len.begin(), l.by_len.end(),
+                     [&](int64_t p, int64_t q) { return l.longest[p] > l.longest[q]; });
+    for (int64_t g = 0; g < groups; ++g) l.slots += 32 * (int64_t)l.longest[g];
+    return l.slots < (int64_t(1) << 32);
+}
+
+// Value ids by the values' bits, through a direct-mapped cache: the maps have a
+// dozen values in no predictable order.
+class ValueTable {
+public:
+    std::vector<double> tab;
+    // false when there are too many
+    bool id(double v, uint32_t* out)
+    {
+        uint64_t bits;
+        std::memcpy(&bits, &v, sizeof bits);
+        Slot& s = cache_[(bits * 0x9E3779B97F4A7C15ull) >> 56];
+        if (s.id == kNone || s.bits != bits) {
+            auto it = ids_.find(bits);
+            if (it == ids_.end()) {
+                if ((int64_t)tab.size() == kMaxTab) return false;
+                it = ids_.emplace(bits, (uint32_t)tab.size()).first;
+                tab.push_back(v);
+            }
+            s = Slot{bits, it->second};
+        }
+        *out = s.id;
+        return true;
+    }
+
+private:
+    static constexpr uint32_t kNone = 0xffffffffu;
+    struct Slot {
+        uint64_t bits = 0;
+        uint32_t id = kNone;
+    };
+    Slot cache_[256];
+    std::unordered_map<uint64_t, uint32_t> ids_;
+};
+
 bool pack_map(int64_t n_rows, int64_t n_cols, const int64_t* ptr, const int64_t* idx,
               const double* val, PackedMap& m, std::vector<unsigned char>& block)
 {
     m = PackedMap{};
     m.n_rows = n_rows;
     m.n_cols = n_cols;
-    if (n_cols > (int64_t(1) << kColBits) || n_rows >= 0x7fffffff) return false;
-    // entries kept, per row
-    std::vector<uint32_t> count(n_rows, 0);
-    std::unordered_map<uint64_t, uint32_t> ids;   // keyed by the value's bits
-    std::vector<double> tab;
-    for (int64_t r = 0; r < n_rows; ++r) {
-        for (int64_t k = ptr[r]; k < ptr[r + 1]; ++k) {
-            if (idx[k] < 0 || idx[k] >= n_cols) continue;
-            ++count[r];
-            uint64_t bits;
-            std::memcpy(&bits, val + k, sizeof bits);
-            if (ids.emplace(bits, (uint32_t)tab.size()).second) {
-                if ((int64_t)tab.size() == kMaxTab) return false;
-                tab.push_back(val[k]);
-            }
-        }
-    }
-    const int64_t entries = std::accumulate(count.begin(), count.end(), int64_t(0));
-    std::vector<int64_t> order(n_rows);
-    std::iota(order.begin(), order.end(), int64_t(0));
-    for (int64_t r0 = 0; entries >= kSortEntries * n_rows && r0 < n_rows; r0 += kSortWindow)
-        std::stable_sort(order.begin() + r0, order.begin() + std::min(r0 + kSortWindow, n_rows),
-                         [&](int64_t p, int64_t q) { return count[p] > count[q]; });
-    const int64_t groups = (n_rows + 31) / 32;
-    std::vector<uint32_t> longest(groups, 0);
-    for (int64_t g = 0; g < groups; ++g)
-        for (int64_t i = g * 32; i < std::min(g * 32 + 32, n_rows); ++i)
-            longest[g] = std::max(longest[g], count[order[i]]);
-    std::vector<int64_t> by_len(groups);
-    std::iota(by_len.begin(), by_len.end(), int64_t(0));
-    std::stable_sort(by_len.begin(), by_len.end(),
-                     [&](int64_t p, int64_t q) { return longest[p] > longest[q]; });
-    int64_t slots = 0;
-    for (int64_t g = 0; g < groups; ++g) slots += 32 * (int64_t)longest[g];
-    if (slots >= (int64_t(1) << 32)) return false;
-    m.groups = groups;
-    m.slots = slots;
-    m.ntab = (int64_t)tab.size();
-    block.assign(packed_map_bytes(m), 0);
-    double* btab = reinterpret_cast<double*>(block.data());
-    std::copy(tab.begin(), tab.end(), btab);
-    uint32_t* goff = reinterpret_cast<uint32_t*>(btab + m.ntab);
-    uint32_t* perm = goff + groups + 1;
-    uint32_t* len = perm + 32 * groups;
-    uint32_t* ent = len + 32 * groups;
-    std::fill(perm, perm + 32 * groups, 0xffffffffu);
-    for (int64_t i = 0; i < groups; ++i) {
-        const int64_t g = by_len[i];
-        goff[i + 1] = goff[i] + 32 * longest[g];
-        for (int l = 0; l < 32 && g * 32 + l < n_rows; ++l) {
-            const int64_t r = order[g * 32 + l];
-            perm[i * 32 + l] = (uint32_t)r;
-            len[i * 32 + l] = count[r];
-            uint32_t j = 0;
+    PackLayout l;
+    if (!pack_layout(n_rows, n_cols, ptr, idx, l)) return false;
+    // the entries first: the number of distinct values decides where they go
+    std::vector<uint32_t> ent(l.slots, 0);
+    ValueTable values;
+    m.groups = (int64_t)l.longest.size();
+    m.slots = l.slots;
+    uint32_t e0 = 0;
+    for (int64_t i = 0; i < m.groups; ++i) {
+        const int64_t g = l.by_len[i];
+        for (int lane = 0; lane < 32 && g * 32 + lane < n_rows; ++lane) {
+            const int64_t r = l.order[g * 32 + lane];
+            uint32_t* e = ent.data() + e0 + lane;
             for (int64_t k = ptr[r]; k < ptr[r + 1]; ++k) {
-                if (idx[k] < 0 || idx[k] >= n_cols) continue;
-                uint64_t bits;
-                std::memcpy(&bits, val + k, sizeof bits);
-                ent[goff[i] + 32 * j++ + l] = (uint32_t)idx[k] | (ids[bits] << kColBits);
+                if ((uint64_t)idx[k] >= (uint64_t)n_cols) continue;
+                uint32_t vid;
+                if (!values.id(val[k], &vid)) return false;
+                *e = (uint32_t)idx[k] | (vid << kColBits);
+                e += 32;
             }
         }
+        e0 += 32 * l.longest[g];
     }
+    m.ntab = (int64_t)values.tab.size();
+    block.resize(packed_map_bytes(m));
+    double* btab = reinterpret_cast<double*>(block.data());
+    std::copy(values.tab.begin(), values.tab.end(), btab);
+    uint32_t* goff = reinterpret_cast<uint32_t*>(btab + m.ntab);
+    uint32_t* perm = goff + m.groups + 1;
+    uint32_t* len = perm + 32 * m.groups;
+    goff[0] = 0;
+    for (int64_t i = 0; i < m.groups; ++i) {
+        const int64_t g = l.by_len[i];
+        goff[i + 1] = goff[i] + 32 * l.longest[g];
+        for (int lane = 0; lane < 32; ++lane) {
+            const bool has = g * 32 + lane < n_rows;
+            const int64_t r = has ? l.order[g * 32 + lane] : 0;
+            perm[i * 32 + lane] = has ? (uint32_t)r : 0xffffffffu;
+            len[i * 32 + lane] = has ? l.count[r] : 0u;
+        }
+    }
+    std::memcpy(len + 32 * m.groups, ent.data(), ent.size() * sizeof(uint32_t));
     return true;
 }
 
@@ -291,21 +345,29 @@ RPYB_API int64_t rpyb_sparse_pack(int64_t n_rows, int64_t n_cols, const int64_t*
     if (indptr[n_rows] > indptr[0] && (!indices || !values))
         return fail(RPYB_E_INVALID, "null pointer");
     PackedMap m;
-    std::vector<unsigned char> packed;
     try {
+        if (!block) {
+            // room for the block whatever its number of distinct values
+            PackLayout l;
+            if (!pack_layout(n_rows, n_cols, indptr, indices, l))
+                return fail(RPYB_E_UNSUPPORTED, "map too large to pack");
+            m.groups = (int64_t)l.longest.size();
+            m.slots = l.slots;
+            m.ntab = std::min(l.entries, kMaxTab);
+            return (int64_t)packed_map_bytes(m);
+        }
+        std::vector<unsigned char> packed;
         if (!pack_map(n_rows, n_cols, indptr, indices, values, m, packed))
-            return fail(RPYB_E_UNSUPPORTED, "map too wide or with too many distinct values to pack");
+            return fail(RPYB_E_UNSUPPORTED, "map too large or with too many distinct values to pack");
+        if (block_bytes < (int64_t)packed.size()) return fail(RPYB_E_INVALID, "block too small");
+        std::memcpy(block, packed.data(), packed.size());
+        layout[0] = m.groups;
+        layout[1] = m.slots;
+        layout[2] = m.ntab;
+        return (int64_t)packed.size();
     } catch (const std::bad_alloc&) {
         return fail(RPYB_E_NOMEM, "out of host memory");
     }
-    layout[0] = m.groups;
-    layout[1] = m.slots;
-    layout[2] = m.ntab;
-    if (block) {
-        if (block_bytes < (int64_t)packed.size()) return fail(RPYB_E_INVALID, "block too small");
-        std::memcpy(block, packed.data(), packed.size());
-    }
-    return (int64_t)packed.size();
 }
 
 RPYB_API int rpyb_sparse_map_packed(int dtype, int64_t n_rows, int64_t n_cols, int64_t batch,

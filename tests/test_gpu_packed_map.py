@@ -63,7 +63,9 @@ def test_pack_refuses_what_does_not_fit():
     layout = (ctypes.c_int64 * 3)()
     many = I.SparseMatrix([0, 5000], np.arange(5000), np.arange(5000) + 0.5, (1, 5000))
     wide = I.SparseMatrix([0, 1], [0], [1.0], (1, (1 << 20) + 1))
+    room = np.empty(1 << 20, dtype=np.uint8)
     for m in (many, wide):
         assert m.device_packed("cuda") is None
         assert _lib.lib.rpyb_sparse_pack(*m.shape, m.indptr.ctypes.data, m.indices.ctypes.data,
-                                         m.data.ctypes.data, None, 0, layout) == _lib.E_UNSUPPORTED
+                                         m.data.ctypes.data, room.ctypes.data, room.size,
+                                         layout) == _lib.E_UNSUPPORTED
