@@ -40,8 +40,9 @@ struct ChainArgs {
     int64_t pw[kMaxDepth + 1] = {};
     int depth = 0;
     int64_t n = 0;
-    const int64_t* off = nullptr;      // [n + 1] into rows
-    const int64_t* rows = nullptr;     // source row of each factor
+    const int64_t* off = nullptr;      // [n + 1] into rows, or (stride > 0) the
+    const int64_t* rows = nullptr;     // source rows of q's off[q] factors at q * stride
+    int64_t stride = 0;
     const void* src = nullptr;         // [*, T] factors (float or double)
     double* acc = nullptr;             // [n, T] out
     int log_out = 0;                   // write log(product) instead of the product
@@ -152,7 +153,8 @@ chain_products_kernel(const ChainArgs a)
     };
 
     for (int64_t q = blockIdx.x; q < a.n; q += gridDim.x) {
-        const int64_t o0 = a.off[q], o1 = a.off[q + 1];
+        const int64_t o0 = a.stride ? q * a.stride : a.off[q];
+        const int64_t o1 = a.stride ? o0 + a.off[q] : a.off[q + 1];
         double* accq = a.acc ? a.acc + q * a.T : nullptr;
         TS* dstq = a.dst ? static_cast<TS*>(a.dst) + a.dst_rows[q] * a.T : nullptr;
         if (o0 == o1 && a.lie) {   // the log of the unit: zero coordinates
@@ -362,6 +364,67 @@ int chain_products_lie(int src_mode, const Geometry& g, int64_t n, const void* s
                         &maps, lie, ld_lie);
 }
 
+static ChainArgs chain_args(const Geometry& g, int64_t n)
+{
+    ChainArgs a;
+    a.T = g.size();
+    for (int k = 0; k <= kMaxDepth + 1; ++k) a.db[k] = g.db[k];
+    for (int k = 0; k <= kMaxDepth; ++k) a.pw[k] = g.pw[k];
+    a.depth = g.depth;
+    a.n = n;
+    return a;
+}
+
+static void set_projection(ChainArgs& a, const LieMapsDev& maps, double* lie, int64_t ld_lie)
+{
+    const PackedMap& m = maps.t2l;
+    a.lie = lie;
+    a.ld_lie = ld_lie;
+    a.lie_dim = maps.lie_dim;
+    a.groups = (int)m.groups;
+    a.tab = static_cast<const double*>(m.block);
+    a.goff = reinterpret_cast<const uint32_t*>(a.tab + m.ntab);
+    a.perm = a.goff + m.groups + 1;
+    a.len = a.perm + 32 * m.groups;
+    a.ent = a.len + 32 * m.groups;
+}
+
+static int run_chain(int src_mode, const Geometry& g, const ChainArgs& a, cudaStream_t s)
+{
+    const size_t smem = (size_t)chain_words(g.size(), g.db[g.depth]) * 8;
+    // threads: one per top-level unit up to what gives an SM 1024 threads over
+    // the blocks its shared memory holds
+    const int F = g.width == 2 ? 3 : g.width == 3 ? 2 : 1;
+    const int64_t units = g.depth >= F ? g.pw[g.depth - F] : g.pw[g.depth];
+    const int64_t per_sm = std::max<int64_t>(1, std::min<int64_t>(16, kChainSmem / (int64_t)(smem + 1024)));
+    int64_t threads = std::min<int64_t>({(units + 31) / 32 * 32,
+                                         std::max<int64_t>(64, 1024 / per_sm / 32 * 32), kChainThreads});
+    threads = std::max<int64_t>(threads, 32);
+    const unsigned grid = (unsigned)std::min<int64_t>(a.n, 1 << 20);
+    ChainFn fn = src_mode == RPYB_F64 ? chain_fn<double>(g.width) : chain_fn<float>(g.width);
+    if (smem > 48 * 1024)
+        RPYB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    fn<<<grid, (unsigned)threads, smem, s>>>(a);
+    RPYB_CUDA(cudaGetLastError());
+    return RPYB_OK;
+}
+
+int chain_products_lie_strided(int src_mode, const Geometry& g, int64_t n, const void* src,
+                               const int64_t* counts, const int64_t* rows, int64_t stride,
+                               const LieMapsDev& maps, double* lie, int64_t ld_lie, cudaStream_t s)
+{
+    if (n == 0) return RPYB_OK;
+    if (!chain_lie_available(g, maps)) return fail(RPYB_E_UNSUPPORTED, "no fused projection for this shape");
+    ChainArgs a = chain_args(g, n);
+    a.off = counts;
+    a.rows = rows;
+    a.stride = stride;
+    a.src = src;
+    a.log_out = 1;
+    set_projection(a, maps, lie, ld_lie);
+    return run_chain(src_mode, g, a, s);
+}
+
 static int chain_launch(int src_mode, const Geometry& g, int64_t n, double* acc, const void* src,
                         const std::vector<int64_t>& off, const std::vector<int64_t>& src_rows,
                         bool log_out, void* dst, const std::vector<int64_t>* dst_rows,
@@ -381,12 +444,7 @@ static int chain_launch(int src_mode, const Geometry& g, int64_t n, double* acc,
         }
         return unit_rows(RPYB_F64, acc, g.size(), g.size(), nullptr, n, s);
     }
-    ChainArgs a;
-    a.T = g.size();
-    for (int k = 0; k <= kMaxDepth + 1; ++k) a.db[k] = g.db[k];
-    for (int k = 0; k <= kMaxDepth; ++k) a.pw[k] = g.pw[k];
-    a.depth = g.depth;
-    a.n = n;
+    ChainArgs a = chain_args(g, n);
     // offsets and rows in one upload
     std::vector<int64_t> packed(off.begin(), off.begin() + n + 1);
     packed.insert(packed.end(), src_rows.begin(), src_rows.begin() + off[n]);
@@ -404,34 +462,8 @@ static int chain_launch(int src_mode, const Geometry& g, int64_t n, double* acc,
     a.log_out = log_out ? 1 : 0;
     a.dst = dst;
     a.dst_rows = dst ? d + n + 1 + off[n] : nullptr;
-    if (lie) {
-        a.lie = lie;
-        a.ld_lie = ld_lie;
-        a.lie_dim = maps->lie_dim;
-        const PackedMap& m = maps->t2l;
-        a.groups = (int)m.groups;
-        a.tab = static_cast<const double*>(m.block);
-        a.goff = reinterpret_cast<const uint32_t*>(a.tab + m.ntab);
-        a.perm = a.goff + m.groups + 1;
-        a.len = a.perm + 32 * m.groups;
-        a.ent = a.len + 32 * m.groups;
-    }
-    const size_t smem = (size_t)chain_words(g.size(), g.db[g.depth]) * 8;
-    // threads: one per top-level unit up to what gives an SM 1024 threads over
-    // the blocks its shared memory holds
-    const int F = g.width == 2 ? 3 : g.width == 3 ? 2 : 1;
-    const int64_t units = g.depth >= F ? g.pw[g.depth - F] : g.pw[g.depth];
-    const int64_t per_sm = std::max<int64_t>(1, std::min<int64_t>(16, kChainSmem / (int64_t)(smem + 1024)));
-    int64_t threads = std::min<int64_t>({(units + 31) / 32 * 32,
-                                         std::max<int64_t>(64, 1024 / per_sm / 32 * 32), kChainThreads});
-    threads = std::max<int64_t>(threads, 32);
-    const unsigned grid = (unsigned)std::min<int64_t>(n, 1 << 20);
-    ChainFn fn = src_mode == RPYB_F64 ? chain_fn<double>(g.width) : chain_fn<float>(g.width);
-    if (smem > 48 * 1024)
-        RPYB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    fn<<<grid, (unsigned)threads, smem, s>>>(a);
-    RPYB_CUDA(cudaGetLastError());
-    return RPYB_OK;
+    if (lie) set_projection(a, *maps, lie, ld_lie);
+    return run_chain(src_mode, g, a, s);
 }
 
 }  // namespace rpyb

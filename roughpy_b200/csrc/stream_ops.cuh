@@ -77,6 +77,12 @@ int chain_products_lie(int src_mode, const Geometry& g, int64_t n, const void* s
                        const std::vector<int64_t>& off, const std::vector<int64_t>& src_rows,
                        const LieMapsDev& maps, double* lie, int64_t ld_lie, cudaStream_t s);
 
+// The same with the lists on the device already: query i has counts[i] factors,
+// rows i * stride and on of `rows`.
+int chain_products_lie_strided(int src_mode, const Geometry& g, int64_t n, const void* src,
+                               const int64_t* counts, const int64_t* rows, int64_t stride,
+                               const LieMapsDev& maps, double* lie, int64_t ld_lie, cudaStream_t s);
+
 // Bytes of scratch finish_queries needs for up to `n` rows.
 size_t finish_scratch_bytes(const Geometry& g, int64_t lie_dim, int64_t n);
 

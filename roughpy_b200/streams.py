@@ -197,7 +197,7 @@ class _StreamQueries:
     """Query front end shared by the stream classes (the reference's
     Stream::log_signature / signature / signature_derivative and its Python
     argument rules, roughpy/src/streams/signature_arguments.cpp:56-160).
-    Subclasses provide ``_query(infs, sups, resolution, logsig, sig)``."""
+    Subclasses provide ``_query(infs, sups, resolution, logsig, sig, out)``."""
 
     def _interval_args(self, interval_or_inf, sup, resolution=None):
         """(inf, sup, resolution): an interval, an inf/sup pair, nothing (the
@@ -235,23 +235,22 @@ class _StreamQueries:
         resolution = _resolution_arg(resolution)
         infs = np.asarray(infs, dtype=np.float64).reshape(-1)
         sups = np.asarray(sups, dtype=np.float64).reshape(-1)
-        outs = [self._query(infs[i:i + chunk], sups[i:i + chunk], resolution)[0]
-                for i in range(0, infs.shape[0], chunk)]
-        if not outs:
-            return torch.zeros((0, self.lie_basis.size()), dtype=torch.float64, device=self.device)
-        return torch.cat(outs)
+        return self._batch(infs, sups, resolution, chunk, self.lie_basis.size(), False)
 
     def signature_batch(self, infs, sups, resolution=None, chunk=16384):
         """Signatures exp(l2t(log_signature)) (float64) of many clopen intervals."""
         resolution = _resolution_arg(resolution)
         infs = np.asarray(infs, dtype=np.float64).reshape(-1)
         sups = np.asarray(sups, dtype=np.float64).reshape(-1)
-        outs = [self._query(infs[i:i + chunk], sups[i:i + chunk], resolution, False, True)[1]
-                for i in range(0, infs.shape[0], chunk)]
-        if not outs:
-            return torch.zeros((0, self.tensor_basis.size()), dtype=torch.float64,
-                               device=self.device)
-        return torch.cat(outs)
+        return self._batch(infs, sups, resolution, chunk, self.tensor_basis.size(), True)
+
+    def _batch(self, infs, sups, resolution, chunk, cols, sig):
+        """All rows in one array, `chunk` queries a call (each writes its rows in place)."""
+        out = torch.empty((infs.shape[0], cols), dtype=torch.float64, device=self.device)
+        for i in range(0, infs.shape[0], chunk):
+            self._query(infs[i:i + chunk], sups[i:i + chunk], resolution, not sig, sig,
+                        out[i:i + chunk])
+        return out
 
     def _log_signature_batch(self, infs, sups, resolution=None):
         return self._query(infs, sups, resolution)[0]
@@ -518,8 +517,9 @@ class LieIncrementStream(_StreamQueries):
         return st
 
     # ------------------------------------------------------------- queries
-    def _query(self, infs, sups, resolution, logsig=True, sig=False):
-        """One rpyb_dyadic_query over clopen intervals; float64 device outputs."""
+    def _query(self, infs, sups, resolution, logsig=True, sig=False, out=None):
+        """One rpyb_dyadic_query over clopen intervals; float64 device outputs (`out` where
+        given and one of them is asked for)."""
         tr = self._build_tree()
         infs = np.ascontiguousarray(infs, dtype=np.float64).reshape(-1)
         if (self.auto_range_table and not tr.range_table and infs.shape[0] >= 1024
@@ -528,8 +528,11 @@ class LieIncrementStream(_StreamQueries):
         sups = np.ascontiguousarray(sups, dtype=np.float64).reshape(-1)
         n = infs.shape[0]
         L, T = self.lie_basis.size(), self.tensor_basis.size()
-        lie = torch.empty((n, L), dtype=torch.float64, device=self.device) if logsig else None
-        sg = torch.empty((n, T), dtype=torch.float64, device=self.device) if sig else None
+        if out is not None:
+            lie, sg = (out, None) if logsig else (None, out)
+        else:
+            lie = torch.empty((n, L), dtype=torch.float64, device=self.device) if logsig else None
+            sg = torch.empty((n, T), dtype=torch.float64, device=self.device) if sig else None
         if n == 0:
             return lie, sg
         res = _lib.QUERY_RESOLUTION_AUTO if resolution is None else int(resolution)
@@ -659,13 +662,16 @@ class PiecewiseAbelianStream(_StreamQueries):
         return cls(infs, sups, lies, width, depth, 0 if resolution is None else resolution,
                    support, device)
 
-    def _query(self, infs, sups, resolution, logsig=True, sig=False):
+    def _query(self, infs, sups, resolution, logsig=True, sig=False, out=None):
         infs = np.ascontiguousarray(infs, dtype=np.float64).reshape(-1)
         sups = np.ascontiguousarray(sups, dtype=np.float64).reshape(-1)
         n = infs.shape[0]
         L, T = self.lie_basis.size(), self.tensor_basis.size()
-        lie = torch.empty((n, L), dtype=torch.float64, device=self.device) if logsig else None
-        sg = torch.empty((n, T), dtype=torch.float64, device=self.device) if sig else None
+        if out is not None:
+            lie, sg = (out, None) if logsig else (None, out)
+        else:
+            lie = torch.empty((n, L), dtype=torch.float64, device=self.device) if logsig else None
+            sg = torch.empty((n, T), dtype=torch.float64, device=self.device) if sig else None
         if n == 0:
             return lie, sg
         res = _lib.QUERY_RESOLUTION_AUTO if resolution is None else int(resolution)
