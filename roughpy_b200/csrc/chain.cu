@@ -38,6 +38,7 @@ struct ChainArgs {
     int64_t T = 0;
     int64_t db[kMaxDepth + 2] = {};
     int64_t pw[kMaxDepth + 1] = {};
+    double coeff[kMaxDepth + 1] = {};       // (-1)^(deg+1) / deg
     int depth = 0;
     int64_t n = 0;
     const int64_t* off = nullptr;      // [n + 1] into rows, or (stride > 0) the
@@ -253,7 +254,7 @@ chain_products_kernel(const ChainArgs a)
             double* rn = x_room[1];
             for (int s = 1; s <= N; ++s) {
                 const int deg = N - s + 1;
-                const double c = (deg % 2 == 0) ? -1.0 / (double)deg : 1.0 / (double)deg;
+                const double c = a.coeff[deg];
                 auto unit = [&](auto kc, uint32_t ru) {
                     constexpr int K = decltype(kc)::value;
                     constexpr int run = Power<D, K - F>::value, begin = LevelStart<D, K>::value;
@@ -370,6 +371,7 @@ static ChainArgs chain_args(const Geometry& g, int64_t n)
     a.T = g.size();
     for (int k = 0; k <= kMaxDepth + 1; ++k) a.db[k] = g.db[k];
     for (int k = 0; k <= kMaxDepth; ++k) a.pw[k] = g.pw[k];
+    for (int deg = 1; deg <= g.depth; ++deg) a.coeff[deg] = (deg % 2 == 0 ? -1.0 : 1.0) / deg;
     a.depth = g.depth;
     a.n = n;
     return a;

@@ -70,10 +70,16 @@ struct SigArgs {
     void* out;
     int64_t ld_out;
     const int64_t* order;
+    const int64_t* ends;   // (first row, end row) in processing order, or null: a
+                           // lookup that does not wait for order's
     int64_t n_streams;
     int64_t items_per_stream;
     int64_t total_items;
-    int* queue;   // device work counter (zeroed before launch)
+    // Items come from a device counter (zeroed before the launch), unless the
+    // grid has a warp for each (`single`): then a warp takes the item of its own
+    // number and the counter is neither zeroed nor read.
+    int* queue;
+    bool single;
     int fold;     // fold interval of the classic compensated mode (steps)
     int fold_chunks;  // split kernel: chunks of kChunk steps between folds
     // output rows: row s of `out` unless dst_row is given, in which case
@@ -251,7 +257,8 @@ signature_kernel(const SigArgs a)
 
     while (true) {
         int item = 0;
-        if (lane == 0) item = atomicAdd(a.queue, 1);
+        if (lane == 0)
+            item = a.single ? (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) : atomicAdd(a.queue, 1);
         item = __shfl_sync(0xffffffffu, item, 0);
         if (item >= a.total_items) break;
 
@@ -274,8 +281,8 @@ signature_kernel(const SigArgs a)
             }
         }
 
-        const int64_t start = a.offsets[s];
-        const int64_t len = a.offsets[s + 1] - start;
+        const int64_t start = a.ends ? a.ends[2 * slot] : a.offsets[s];
+        const int64_t len = (a.ends ? a.ends[2 * slot + 1] : a.offsets[s + 1]) - start;
         const T* __restrict__ xs = static_cast<const T*>(a.inc) + start * D;
 
         // ---- state
@@ -308,6 +315,73 @@ signature_kernel(const SigArgs a)
             __syncwarp();
             if (t0 + kChunk + lane < len) load_row<T, D>(nx, xs + (t0 + kChunk + lane) * D);
             const int nsteps = (int)min((int64_t)kChunk, len - t0);
+            if constexpr (F64) {
+                // Software pipeline, two steps an iteration on alternating
+                // registers: the next step's chains, seven dependent FP64
+                // operations, run beside this step's products.  Measured on B200
+                // against one step after the other: (4,5) 256 x 128 16.4 -> 14.4 us,
+                // (8,5) 1000 x 16..2000 3.58 -> 3.44 ms, (5,4) 20 x 500 45 -> 37 us.
+                // chains and path update of a step, from the path words before it:
+                auto chains = [&](int jj, T (&xv)[D], T (&xg)[G], T& ax, T& am) {
+                    const T* row = xbuf + jj * D;
+                    load_row_smem<T, D>(xv, row);
+                    load_slice<T, G>(xg, row + sub * G);
+                    T xc[P > 0 ? P : 1];
+#pragma unroll
+                    for (int i = 0; i < P; ++i) xc[i] = row[c[i]];
+                    ax = T(0.5);
+                    am = T(1);
+                    if constexpr (P > 0) {
+                        T acc = ph[0] + xc[0] * (T(1) / T(N));
+                        am = ph[0] + xc[0] * (T(1) / T(N - 1));
+#pragma unroll
+                        for (int i = 2; i <= P; ++i) {
+                            acc = fma_t(acc, xc[i - 1] * (T(1) / T(N - i + 1)), ph[i - 1]);
+                            am = fma_t(am, xc[i - 1] * (T(1) / T(N - i)), ph[i - 1]);
+                        }
+                        ax = acc * T(0.5);
+                    }
+#pragma unroll
+                    for (int kk = P; kk >= 1; --kk) {
+                        if (kk == 1) {
+                            ph[0] += xc[0];
+                        } else {
+                            T acc = ph[0] + xc[0] * (T(1) / T(kk));
+#pragma unroll
+                            for (int i = 2; i <= kk - 1; ++i)
+                                acc = fma_t(acc, xc[i - 1] * (T(1) / T(kk - i + 1)), ph[i - 1]);
+                            ph[kk - 1] += acc * xc[kk - 1];
+                        }
+                    }
+                };
+                auto products = [&](const T (&xv)[D], const T (&xg)[G], T ax, T am) {
+#pragma unroll
+                    for (int g = 0; g < G; ++g) {
+                        const T w = fma_t(ax, xg[g], mh[g]);
+#pragma unroll
+                        for (int b = 0; b < D; ++b) th[g][b] = fma_t(w, xv[b], th[g][b]);
+                    }
+#pragma unroll
+                    for (int g = 0; g < G; ++g) mh[g] = fma_t(am, xg[g], mh[g]);
+                };
+                T x[D], xa[G], ax, am, x1[D], xa1[G], ax1, am1;
+                chains(0, x, xa, ax, am);
+                int j = 0;
+#pragma unroll 1
+                for (; j + 2 < nsteps; j += 2) {
+                    chains(j + 1, x1, xa1, ax1, am1);
+                    products(x, xa, ax, am);
+                    chains(j + 2, x, xa, ax, am);
+                    products(x1, xa1, ax1, am1);
+                }
+                if (j + 1 < nsteps) {
+                    chains(j + 1, x1, xa1, ax1, am1);
+                    products(x, xa, ax, am);
+                    products(x1, xa1, ax1, am1);
+                } else {
+                    products(x, xa, ax, am);
+                }
+            } else {
             for (int j = 0; j < nsteps; ++j) {
             const T* row = xbuf + j * D;
             T x[D];
@@ -318,11 +392,11 @@ signature_kernel(const SigArgs a)
 #pragma unroll
             for (int i = 0; i < P; ++i) xc[i] = row[c[i]];
 
-            // pre-step values of the path words (float: hi + delta, hi being
-            // kept as the rounded value of hi + lo)
+            // pre-step values of the path words: hi + delta, hi being kept as the
+            // rounded value of hi + lo
             T vp[P > 0 ? P : 1];
 #pragma unroll
-            for (int i = 0; i < P; ++i) vp[i] = F64 ? ph[i] : (ph[i] + pd[i]);
+            for (int i = 0; i < P; ++i) vp[i] = ph[i] + pd[i];
 
             // ---- level N (top): chain through the path, then the mid words
             {
@@ -336,9 +410,9 @@ signature_kernel(const SigArgs a)
                 const T accx = acc * (T(1) / T(2));
 #pragma unroll
                 for (int g = 0; g < G; ++g) {
-                    // am = S_{N-1} + acc * x/2; in float mode the delta joins the
-                    // product before the (large) hi word
-                    const T am = F64 ? fma_t(accx, xa[g], mh[g]) : (mh[g] + fma_t(accx, xa[g], md[g]));
+                    // am = S_{N-1} + acc * x/2; the delta joins the product before the
+                    // (large) hi word
+                    const T am = mh[g] + fma_t(accx, xa[g], md[g]);
                     if constexpr (PACK) {
                         // packed f32x2 FMAs: two top words per instruction
                         const float2 am2 = make_float2(am, am);
@@ -351,10 +425,7 @@ signature_kernel(const SigArgs a)
                         }
                     } else {
 #pragma unroll
-                        for (int b = 0; b < D; ++b) {
-                            if constexpr (F64) th[g][b] = fma_t(am, x[b], th[g][b]);
-                            else td[g][b] = fma_t(am, x[b], td[g][b]);
-                        }
+                        for (int b = 0; b < D; ++b) td[g][b] = fma_t(am, x[b], td[g][b]);
                     }
                 }
             }
@@ -368,10 +439,7 @@ signature_kernel(const SigArgs a)
                         acc = fma_t(acc, xc[i - 1] * (T(1) / T(N - i)), vp[i - 1]);
                 }
 #pragma unroll
-                for (int g = 0; g < G; ++g) {
-                    if constexpr (F64) mh[g] = fma_t(acc, xa[g], mh[g]);
-                    else md[g] = fma_t(acc, xa[g], md[g]);
-                }
+                for (int g = 0; g < G; ++g) md[g] = fma_t(acc, xa[g], md[g]);
             }
             // ---- path levels k = P .. 1
 #pragma unroll
@@ -386,12 +454,10 @@ signature_kernel(const SigArgs a)
                         acc = fma_t(acc, xc[i - 1] * (T(1) / T(k - i + 1)), vp[i - 1]);
                     upd = acc * xc[k - 1];
                 }
-                if constexpr (F64) ph[k - 1] += upd;
-                else pd[k - 1] += upd;
+                pd[k - 1] += upd;
             }
 
-            if constexpr (!F64) {
-                if (++since_fold >= a.fold) {
+            if (++since_fold >= a.fold) {
                     since_fold = 0;
                     // Fold the deltas into (hi, lo) with an exact two-sum, then
                     // renormalise (hi, lo) so that hi is the rounded value: the
@@ -484,6 +550,7 @@ signature_kernel(const SigArgs a)
                 }
             }
         }
+        if (a.single) break;
     }
 }
 
@@ -603,7 +670,8 @@ signature_kernel_split(const SigArgs a)
 
     while (true) {
         int item = 0;
-        if (lane == 0) item = atomicAdd(a.queue, 1);
+        if (lane == 0)
+            item = a.single ? (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) : atomicAdd(a.queue, 1);
         item = __shfl_sync(0xffffffffu, item, 0);
         if (item >= a.total_items) break;
 
@@ -626,8 +694,8 @@ signature_kernel_split(const SigArgs a)
             }
         }
 
-        const int64_t start = a.offsets[s];
-        const int64_t len = a.offsets[s + 1] - start;
+        const int64_t start = a.ends ? a.ends[2 * slot] : a.offsets[s];
+        const int64_t len = (a.ends ? a.ends[2 * slot + 1] : a.offsets[s + 1]) - start;
         const float* __restrict__ xs = static_cast<const float*>(a.inc) + start * D;
 
         double ph[PP];
@@ -900,6 +968,7 @@ signature_kernel_split(const SigArgs a)
                 for (int b = 0; b < D; ++b) o[a.db[N] + mw * D + b] = tv[b];
             }
         }
+        if (a.single) break;
     }
     if constexpr (TM) {
         tmem_fence_before();
@@ -1296,8 +1365,8 @@ namespace {
 // only reset the queue and launch.
 int launch_signature_variant(const SigVariant& v, const Geometry& g, int64_t n_items,
                              const int64_t* offsets, const void* inc, void* out, int64_t ld_out,
-                             const int64_t* order, const int64_t* dst_row, void* alt,
-                             int64_t ld_alt, int* queue, int wpb_forced, cudaStream_t s)
+                             const int64_t* order, const int64_t* ends, const int64_t* dst_row,
+                             void* alt, int64_t ld_alt, int* queue, int wpb_forced, cudaStream_t s)
 {
     SigArgs a{};
     a.offsets = offsets;
@@ -1305,6 +1374,7 @@ int launch_signature_variant(const SigVariant& v, const Geometry& g, int64_t n_i
     a.out = out;
     a.ld_out = ld_out;
     a.order = order;
+    a.ends = ends;
     a.n_streams = n_items;
     a.items_per_stream = (v.lanes + 31) / 32;
     a.total_items = a.items_per_stream * n_items;
@@ -1374,11 +1444,17 @@ int launch_signature_variant(const SigVariant& v, const Geometry& g, int64_t n_i
         if (forced_bps) per_sm = v.tmem ? std::min(forced_bps, 512 / tmem_cols_for(wpb)) : forced_bps;
     }
     if (per_sm < 1) per_sm = 1;
+    if (wpb_forced == 0 && signature_warps_per_block() == 0 && !v.tmem) {
+        // fewer items than one block an SM holds: smaller blocks, so that every SM
+        // has some (512 warps at (4,5): 64 blocks of eight 25 us, 256 of two 18 us)
+        while (wpb > 1 && a.total_items <= (int64_t)device_sm_count() * (wpb - 1)) --wpb;
+    }
     const size_t smem = smem_warp * wpb;
     int64_t blocks = (int64_t)per_sm * device_sm_count();
     blocks = std::min<int64_t>(blocks, (a.total_items + wpb - 1) / wpb);
     if (blocks < 1) blocks = 1;
-    RPYB_CUDA(cudaMemsetAsync(queue, 0, sizeof(int), s));
+    a.single = a.total_items <= blocks * wpb;
+    if (!a.single) RPYB_CUDA(cudaMemsetAsync(queue, 0, sizeof(int), s));
     v.fn<<<(unsigned)blocks, wpb * 32, smem, s>>>(a);
     RPYB_CUDA(cudaGetLastError());
     return RPYB_OK;
@@ -1404,8 +1480,8 @@ int64_t signature_lanes_per_stream(int mode, int width, int depth, int g)
 
 int signature_launch(int mode, int width, int depth, int g_lane, int wpb, int64_t n_items,
                      const int64_t* offsets, const void* inc, void* out, int64_t ld_out,
-                     const int64_t* order, const int64_t* dst_row, void* alt, int64_t ld_alt,
-                     int* queue, cudaStream_t s)
+                     const int64_t* order, const int64_t* ends, const int64_t* dst_row, void* alt,
+                     int64_t ld_alt, int* queue, cudaStream_t s)
 {
     int rc;
     Geometry g;
@@ -1418,8 +1494,8 @@ int signature_launch(int mode, int width, int depth, int g_lane, int wpb, int64_
     const bool vec = (mode == RPYB_F32) ? (width % 4 == 0) : (width % 2 == 0);
     if (vec && (reinterpret_cast<uintptr_t>(inc) & 15) != 0)
         return fail(RPYB_E_INVALID, "increments must be 16-byte aligned");
-    return launch_signature_variant(v, g, n_items, offsets, inc, out, ld_out, order, dst_row, alt,
-                                    ld_alt, queue, wpb, s);
+    return launch_signature_variant(v, g, n_items, offsets, inc, out, ld_out, order, ends, dst_row,
+                                    alt, ld_alt, queue, wpb, s);
 }
 
 int signature_error_report(int width, int depth, int64_t n_streams, const int64_t* offsets,
@@ -1505,7 +1581,7 @@ RPYB_API int rpyb_signature(int mode, int32_t width, int32_t depth, int64_t n_st
         if (vec && (reinterpret_cast<uintptr_t>(increments) & 15) != 0)
             return fail(RPYB_E_INVALID, "increments must be 16-byte aligned");
         return launch_signature_variant(v, g, n_streams, offsets, increments, out, ld_out, order,
-                                        nullptr, nullptr, 0, static_cast<int*>(ws), 0, s);
+                                        nullptr, nullptr, nullptr, 0, static_cast<int*>(ws), 0, s);
     }
     // generic path
     const int sms = device_sm_count();

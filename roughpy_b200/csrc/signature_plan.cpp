@@ -230,6 +230,7 @@ struct rpyb_sig_plan {
     const int64_t* d_stream_offsets = nullptr;
     const int64_t* d_item_offsets = nullptr;
     const int64_t* d_order = nullptr;
+    const int64_t* d_ends = nullptr;        // the items' (first, end) rows in that order
     const int64_t* d_stream_order = nullptr; // longest-first order of whole streams
     const int64_t* d_dst = nullptr;         // nullptr when no stream is split
     int64_t n_items = 0;
@@ -341,6 +342,12 @@ int build_layout(rpyb_sig_plan* p, int64_t seg)
     const size_t at_soff = put(p->offsets);
     const size_t at_ioff = put(item_off);
     const size_t at_order = put(order);
+    std::vector<int64_t> item_ends;
+    for (const int64_t i : order) {
+        item_ends.push_back(item_off[i]);
+        item_ends.push_back(item_off[i + 1]);
+    }
+    const size_t at_ends = put(item_ends);
     const size_t at_sorder = put(stream_order);
     size_t at_dst = 0, at_fs = 0, at_fd = 0;
     if (any_split) {
@@ -362,6 +369,7 @@ int build_layout(rpyb_sig_plan* p, int64_t seg)
     p->d_stream_offsets = base + at_soff;
     p->d_item_offsets = base + at_ioff;
     p->d_order = base + at_order;
+    p->d_ends = base + at_ends;
     p->d_stream_order = base + at_sorder;
     p->n_items = n_items;
     p->d_dst = any_split ? base + at_dst : nullptr;
@@ -387,7 +395,7 @@ int run_plan(rpyb_sig_plan* p, const void* inc, void* out, int64_t ld_out, cudaS
                               out, ld_out, p->d_stream_order, p->queue.p, p->queue_bytes, s);
     }
     if ((rc = signature_launch(p->mode, p->width, p->depth, p->sched.g, p->sched.wpb, p->n_items,
-                               p->d_item_offsets, inc, out, ld_out, p->d_order, p->d_dst,
+                               p->d_item_offsets, inc, out, ld_out, p->d_order, p->d_ends, p->d_dst,
                                p->rows.p, T, static_cast<int*>(p->queue.p), s)))
         return rc;
     for (const auto& lv : p->levels) {
