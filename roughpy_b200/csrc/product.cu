@@ -958,6 +958,26 @@ static bool blocked_accumulates_faster(int dtype, const Geometry& g, const Produ
     return staged > (dtype == RPYB_F32 ? 128 : 72) * 1024;
 }
 
+// Where the slab kernel beats the kernels below.  Measured on B200, slabs /
+// others: widths 5 and 7, which have no two-letter blocks, (5,7) x 500 float64
+// 299 / 333 us accumulating and 229 / 319 assigning, (7,6) float32 x 600 308 /
+// 528 us; width 8 float32, (8,6) x 1024 1000 / 1149 and 910 / 1074 us; width 4
+// assigning float64, (4,8) x 500 219 / 239 us.  Not: (8,6) float64 904 / 835 us
+// accumulating, (4,8) float32 407 / 351 us, accumulating float64 266 / 252 us.
+// A row is only `width` blocks, so few rows leave SMs idle: (8,6) float32 x 10
+// 37 / 18 us.
+static bool slabs_faster(int dtype, const Geometry& g, const ProductSpec& spec, int64_t batch)
+{
+    if (batch < 64) return false;
+    switch (g.width) {
+        case 4: return dtype == RPYB_F64 && !spec.accumulate;
+        case 5:
+        case 7: return true;
+        case 8: return dtype == RPYB_F32;
+        default: return false;
+    }
+}
+
 int launch_product(int dtype, const Geometry& g, const ProductSpec& spec,
                    const ProductRows& rows, cudaStream_t stream)
 {
@@ -965,6 +985,9 @@ int launch_product(int dtype, const Geometry& g, const ProductSpec& spec,
     if (product_rows_enabled(dtype) && product_rows_available(g, spec, rows) &&
         !blocked_accumulates_faster(dtype, g, spec))
         return launch_product_rows(dtype, g, spec, rows, false, stream);
+    if (product_rows_enabled(dtype) && product_slabs_available(g, spec, rows) &&
+        slabs_faster(dtype, g, spec, rows.batch))
+        return launch_product_slabs(dtype, g, spec, rows, false, stream);
     // float64 rows of width 2 up to level kW2MinTop or higher: the
     // lane-letter kernel
     if (dtype == RPYB_F64 && blocked_enabled() && g.width == 2 && w2_kernel_enabled() &&

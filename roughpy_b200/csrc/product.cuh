@@ -56,6 +56,11 @@ bool product_rows_available(const Geometry& g, const ProductSpec& spec, const Pr
 int launch_product_rows(int dtype, const Geometry& g, const ProductSpec& spec,
                         const ProductRows& rows, bool in_place, cudaStream_t stream);
 
+// The same one level deeper, the top level in slabs of one second letter.
+bool product_slabs_available(const Geometry& g, const ProductSpec& spec, const ProductRows& rows);
+int launch_product_slabs(int dtype, const Geometry& g, const ProductSpec& spec,
+                         const ProductRows& rows, bool in_place, cudaStream_t stream);
+
 // Elementwise helpers used by the Horner drivers.
 int launch_convert_rows(int dst_dtype, void* dst, int64_t ld_dst, int src_dtype,
                         const void* src, int64_t ld_src, int64_t cols, int64_t batch,

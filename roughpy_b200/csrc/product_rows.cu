@@ -232,6 +232,106 @@ product_rows_kernel(const RowArgs a)
     }
 }
 
+// The top level of rows whose lower levels do not fit but whose next lower
+// level's do (width 8 depth 6, 4 and 8, 5 and 7, ...), in slabs: a block takes
+// the words (u, a, rho) of one second letter a, all first letters u and the
+// N - 2 letters rho.  With 2 <= p < N their left words are L_p[u, a, ..], a
+// d-th of each level, and their right words the levels R_1 .. R_{N-2}, so both
+// are staged as float64 as before; L_p's part is as many words as level p - 1,
+// and in that place split_unit sees a product of depth N - 1.  Left over are
+// p = 1, whose right words R_{N-1}[a, rho] are one run, and the streamed ends.
+// Levels below N are a row-resident product of their own.   Measured on B200, (8,6)
+// float32 x 1024 accumulating 1149 -> 1000 us (4.9 TB/s); in place (8,6) float32
+// x 500 1.23 -> 0.47 ms.  What bounds it is the latency of the streamed words at
+// 27 warps an SM: 45 % DRAM, 43 % shared-memory pipe, 41 % issue.
+template <typename T, typename TR, bool ACCUM, int D>
+__global__ void __launch_bounds__(kRowThreads, 1)
+product_slab_kernel(const RowArgs a)
+{
+    constexpr int U = D;
+    extern __shared__ __align__(16) unsigned char row_smem[];
+    __shared__ double first[D];   // L_1
+    const int N = a.top;
+    const int TL = (int)a.db[N - 1];   // words below level N - 1
+    double* const l_room = reinterpret_cast<double*>(row_smem);
+    double* const r_room = l_room + stage_room(TL);
+    const int tid = (int)threadIdx.x, B = (int)blockDim.x;
+    const int lane = tid & 31, warp = tid >> 5, nwarps = B >> 5;
+    const uint32_t letter = blockIdx.x;
+    const uint32_t rho_n = (uint32_t)a.pw[N - 2], run = (uint32_t)a.pw[N - 1];
+
+    for (int64_t b = blockIdx.y; b < a.batch; b += gridDim.y) {
+        T* out = static_cast<T*>(a.out) + (a.out_idx ? a.out_idx[b] : b) * a.ld_out;
+        const T* lhs = static_cast<const T*>(a.lhs) + (a.lhs_idx ? a.lhs_idx[b] : b) * a.ld_lhs;
+        const TR* rhs = static_cast<const TR*>(a.rhs) + (a.rhs_idx ? a.rhs_idx[b] : b) * a.ld_rhs;
+        __syncthreads();   // the previous row is done with the buffers
+        const double* R = stage_words(r_room, rhs, TL, tid, B);
+        for (int j = 1; j <= N - 2; ++j) {
+            // level j's place: L_{j+1}[u, letter, ..]
+            const uint32_t n = (uint32_t)a.pw[j], part = (uint32_t)a.pw[j - 1];
+            const T* src = lhs + a.db[j + 1] + (int64_t)letter * part;
+            double* dst = l_room + a.db[j];
+            constexpr int kLoads = 8;
+            for (uint32_t i0 = tid; i0 < n; i0 += kLoads * B) {
+                T v[kLoads];
+#pragma unroll
+                for (int k = 0; k < kLoads; ++k) {
+                    const uint32_t i = i0 + k * B, u = i / part;
+                    v[k] = i < n ? src[(int64_t)u * n + (i - u * part)] : T(0);
+                }
+#pragma unroll
+                for (int k = 0; k < kLoads; ++k)
+                    if (i0 + k * B < n) dst[i0 + k * B] = (double)v[k];
+            }
+        }
+        if (tid < D) first[tid] = (double)lhs[1 + tid];
+        const int tasks = (int)((rho_n + 31) >> 5);
+        const int64_t begin = a.db[N] + (int64_t)letter * rho_n;
+        auto prefetch_task = [&](int t) {
+            if (t >= tasks) return;
+            const int64_t left = rho_n - t * 32;
+            prefetch_runs(lhs + begin + t * 32, run, D, left, lane);
+            prefetch_runs(rhs + begin + t * 32, run, D, left, lane);
+            prefetch_runs(rhs + a.db[N - 1] + (int64_t)letter * rho_n + t * 32, run, 1, left, lane);
+            if (ACCUM) prefetch_runs(static_cast<const T*>(out) + begin + t * 32, run, D, left, lane);
+        };
+        prefetch_task(warp);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        const double l0 = (double)lhs[0], r0 = R[0];
+        with_level<1, row_max_top<D>()>(N - 1, [&](auto kc) {
+            constexpr int K = decltype(kc)::value;   // depth of what split_unit sees
+            constexpr int RHO = Power<D, K - 1>::value, RUN = Power<D, K>::value;
+            for (int t = warp; t < tasks; t += nwarps) {
+                prefetch_task(t + nwarps);
+                const uint32_t rho = (uint32_t)(t * 32 + lane);
+                if (RHO % 32 != 0 && rho >= (uint32_t)RHO) continue;
+                T* op = out + begin + rho;
+                const T* lp = lhs + begin + rho;
+                const TR* rp = rhs + begin + rho;
+                T av[U], lv[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    if (ACCUM) av[u] = op[(int64_t)u * RUN];
+                    lv[u] = lp[(int64_t)u * RUN];
+                }
+                double acc[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) acc[u] = fma((double)lv[u], r0, ACCUM ? (double)av[u] : 0.0);
+                TR rv[U];   // in flight during the splits
+#pragma unroll
+                for (int u = 0; u < U; ++u) rv[u] = rp[(int64_t)u * RUN];
+                const double x1 = (double)rhs[LevelStart<D, K>::value + (int64_t)letter * RHO + rho];
+                split_unit<D, 1, K, U>(acc, l_room, R, rho);
+#pragma unroll
+                for (int u = 0; u < U; ++u) acc[u] = fma(first[u], x1, acc[u]);
+#pragma unroll
+                for (int u = 0; u < U; ++u) op[(int64_t)u * RUN] = (T)fma(l0, (double)rv[u], acc[u]);
+            }
+        });
+    }
+}
+
 using RowFn = void (*)(RowArgs);
 
 template <typename T, typename TR, bool ACCUM>
@@ -249,28 +349,24 @@ RowFn row_fn(int width)
     }
 }
 
-}  // namespace
-
-bool product_rows_available(const Geometry& g, const ProductSpec& spec, const ProductRows& rows)
+template <typename T, typename TR, bool ACCUM>
+RowFn slab_fn(int width)
 {
-    const int N = spec.khi;
-    if (g.width < 2 || g.width > 16 || N < 1 || 2 * g.db[N] * 8 > kRowSmem) return false;
-    // the whole truncated product of whole rows
-    if (spec.klo != 1 || !spec.lhs0_from_mem || spec.lhs0_add != 0.0 || rows.addend) return false;
-    if (!spec.l0_write || !spec.l0_prod || spec.l0_const != 0.0 || spec.scale0 != 1.0 ||
-        spec.l0_base != (spec.accumulate ? 1 : 0))
-        return false;
-    for (int k = 1; k <= N; ++k)
-        if (spec.pmin[k] != 0 || spec.pmax[k] != k || spec.scale[k] != 1.0) return false;
-    return true;
+    switch (width) {
+        case 4: return &product_slab_kernel<T, TR, ACCUM, 4>;
+        case 5: return &product_slab_kernel<T, TR, ACCUM, 5>;
+        case 6: return &product_slab_kernel<T, TR, ACCUM, 6>;
+        case 7: return &product_slab_kernel<T, TR, ACCUM, 7>;
+        case 8: return &product_slab_kernel<T, TR, ACCUM, 8>;
+        default: return nullptr;
+    }
 }
 
-int launch_product_rows(int dtype, const Geometry& g, const ProductSpec& spec,
-                        const ProductRows& rows, bool in_place, cudaStream_t stream)
+RowArgs row_args(const Geometry& g, int top, const ProductRows& rows)
 {
     RowArgs a{};
     a.width = g.width;
-    a.top = spec.khi;
+    a.top = top;
     for (int k = 0; k <= kMaxDepth + 1; ++k) a.db[k] = g.db[k];
     for (int k = 0; k <= kMaxDepth; ++k) a.pw[k] = g.pw[k];
     a.out = rows.out;
@@ -283,6 +379,44 @@ int launch_product_rows(int dtype, const Geometry& g, const ProductSpec& spec,
     a.out_idx = rows.out_idx;
     a.lhs_idx = rows.lhs_idx;
     a.rhs_idx = rows.rhs_idx;
+    return a;
+}
+
+// threads a block: one per unit up to what gives an SM 1024 threads over the
+// blocks its shared memory holds
+int64_t row_threads(int64_t units, size_t smem)
+{
+    const int64_t per_sm = std::max<int64_t>(1, std::min<int64_t>(16, kRowSmem / (int64_t)(smem + 1024)));
+    const int64_t t = std::min<int64_t>({(units + 31) / 32 * 32,
+                                         std::max<int64_t>(64, 1024 / per_sm / 32 * 32), kRowThreads});
+    return std::max<int64_t>(t, 32);
+}
+
+// whether the spec is the whole truncated product of whole rows
+bool whole_product(const ProductSpec& spec, const ProductRows& rows)
+{
+    if (spec.klo != 1 || !spec.lhs0_from_mem || spec.lhs0_add != 0.0 || rows.addend) return false;
+    if (!spec.l0_write || !spec.l0_prod || spec.l0_const != 0.0 || spec.scale0 != 1.0 ||
+        spec.l0_base != (spec.accumulate ? 1 : 0))
+        return false;
+    for (int k = 1; k <= spec.khi; ++k)
+        if (spec.pmin[k] != 0 || spec.pmax[k] != k || spec.scale[k] != 1.0) return false;
+    return true;
+}
+
+}  // namespace
+
+bool product_rows_available(const Geometry& g, const ProductSpec& spec, const ProductRows& rows)
+{
+    const int N = spec.khi;
+    if (g.width < 2 || g.width > 16 || N < 1 || 2 * g.db[N] * 8 > kRowSmem) return false;
+    return whole_product(spec, rows);
+}
+
+int launch_product_rows(int dtype, const Geometry& g, const ProductSpec& spec,
+                        const ProductRows& rows, bool in_place, cudaStream_t stream)
+{
+    RowArgs a = row_args(g, spec.khi, rows);
     RowFn fn;
     if (dtype == RPYB_F64)
         fn = spec.accumulate ? row_fn<double, double, true>(g.width) : row_fn<double, double, false>(g.width);
@@ -292,13 +426,8 @@ int launch_product_rows(int dtype, const Geometry& g, const ProductSpec& spec,
         fn = spec.accumulate ? row_fn<float, float, true>(g.width) : row_fn<float, float, false>(g.width);
     const int F = g.width == 2 ? 3 : g.width == 3 ? 2 : 1;
     const size_t smem = (size_t)(2 * stage_room((int)g.db[a.top]) * 8);
-    // threads: one per top-level unit up to what gives an SM 1024 threads over
-    // the blocks its shared memory holds
     const int64_t units = a.top >= F ? g.pw[a.top - F] : g.pw[a.top];
-    const int64_t per_sm = std::max<int64_t>(1, std::min<int64_t>(16, kRowSmem / (int64_t)(smem + 1024)));
-    int64_t threads = std::min<int64_t>({(units + 31) / 32 * 32,
-                                         std::max<int64_t>(64, 1024 / per_sm / 32 * 32), kRowThreads});
-    threads = std::max<int64_t>(threads, 32);
+    const int64_t threads = row_threads(units, smem);
     // fewer rows than SMs: blocks share a row's top level (not in place, where
     // one block would write lower levels that another still has to stage)
     int64_t slices = 1;
@@ -310,6 +439,37 @@ int launch_product_rows(int dtype, const Geometry& g, const ProductSpec& spec,
     fn<<<grid, (unsigned)threads, smem, stream>>>(a);
     RPYB_CUDA(cudaGetLastError());
     return RPYB_OK;
+}
+
+bool product_slabs_available(const Geometry& g, const ProductSpec& spec, const ProductRows& rows)
+{
+    const int N = spec.khi;
+    return g.width >= 4 && g.width <= 8 && N >= 3 && 2 * g.db[N] * 8 > kRowSmem &&
+           2 * g.db[N - 1] * 8 <= kRowSmem && whole_product(spec, rows);
+}
+
+int launch_product_slabs(int dtype, const Geometry& g, const ProductSpec& spec,
+                         const ProductRows& rows, bool in_place, cudaStream_t stream)
+{
+    const RowArgs a = row_args(g, spec.khi, rows);
+    RowFn fn;
+    if (dtype == RPYB_F64)
+        fn = spec.accumulate ? slab_fn<double, double, true>(g.width) : slab_fn<double, double, false>(g.width);
+    else if (dtype == kMixedF64F32)
+        fn = spec.accumulate ? slab_fn<double, float, true>(g.width) : slab_fn<double, float, false>(g.width);
+    else
+        fn = spec.accumulate ? slab_fn<float, float, true>(g.width) : slab_fn<float, float, false>(g.width);
+    const size_t smem = (size_t)(2 * stage_room((int)g.db[a.top - 1]) * 8);
+    const int64_t threads = row_threads(g.pw[a.top - 2], smem);
+    if (smem > 48 * 1024)
+        RPYB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const dim3 grid((unsigned)g.width, (unsigned)std::min<int64_t>(rows.batch, 65535), 1);
+    // the top level first: in place, the lower levels it reads are still the old ones
+    fn<<<grid, (unsigned)threads, smem, stream>>>(a);
+    RPYB_CUDA(cudaGetLastError());
+    ProductSpec low = spec;
+    low.khi = spec.khi - 1;
+    return launch_product_rows(dtype, g, low, rows, in_place, stream);
 }
 
 }  // namespace rpyb

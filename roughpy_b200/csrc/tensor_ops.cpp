@@ -388,7 +388,7 @@ RPYB_API int rpyb_ft_inplace_mul(int dtype, int32_t width, int32_t depth, int64_
     rows.ld_rhs = ld_rhs;
     rows.batch = batch;
     // In place where one block has a whole row: three passes over the rows
-    // instead of five.  Rows of the two operands may be the same, but no row
+    // instead of five (a row in slabs is a few blocks: not for a few rows).  Rows of the two operands may be the same, but no row
     // of one may reach into another row of the other.
     const char* l0 = static_cast<const char*>(lhs);
     const char* r0 = static_cast<const char*>(rhs);
@@ -396,10 +396,13 @@ RPYB_API int rpyb_ft_inplace_mul(int dtype, int32_t width, int32_t depth, int64_
     const int64_t r_bytes = ((batch - 1) * ld_rhs + T) * (int64_t)es;
     const bool apart = r0 >= l0 + l_bytes || l0 >= r0 + r_bytes;
     const bool same = l0 == r0 && (ld_lhs == ld_rhs || batch == 1);
-    if ((apart || same) && product_rows_enabled(dtype) && product_rows_available(g, sp, rows)) {
+    const bool whole = product_rows_available(g, sp, rows);
+    if ((apart || same) && product_rows_enabled(dtype) &&
+        (whole || (batch >= 64 && product_slabs_available(g, sp, rows)))) {
         rows.out = lhs;
         rows.ld_out = ld_lhs;
-        return launch_product_rows(dtype, g, sp, rows, true, s);
+        return whole ? launch_product_rows(dtype, g, sp, rows, true, s)
+                     : launch_product_slabs(dtype, g, sp, rows, true, s);
     }
     if ((rc = launch_product(dtype, g, sp, rows, s))) return rc;
     const int64_t c0 = g.db[lmin], c1 = g.db[lmax + 1];

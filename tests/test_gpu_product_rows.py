@@ -17,7 +17,8 @@ pytestmark = pytest.mark.gpu
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SHAPES = [(2, 1, 3), (2, 2, 4), (2, 3, 2), (2, 7, 150), (2, 13, 1), (3, 1, 2), (3, 2, 5), (3, 6, 3),
           (3, 9, 1), (4, 1, 3), (4, 5, 149), (4, 7, 2), (5, 2, 3), (5, 6, 1), (6, 3, 4), (6, 6, 2),
-          (7, 5, 1), (7, 2, 9), (8, 5, 2), (8, 3, 150), (9, 4, 2), (10, 5, 1), (16, 2, 3)]
+          (7, 5, 1), (7, 2, 9), (8, 5, 2), (8, 3, 150), (9, 4, 2), (10, 5, 1), (16, 2, 3),
+          (4, 8, 64), (5, 7, 64), (5, 7, 2), (7, 6, 65), (8, 6, 64)]   # 64 rows on: slabs
 
 
 def compute_all():
