@@ -2,6 +2,7 @@
 // multiplication, and batched sparse (CSR) linear maps for Lie <-> tensor.
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -22,27 +23,90 @@ __device__ __forceinline__ int level_of(const LevelTab& t, int64_t i)
     return k;
 }
 
-// out[rev(w)] = (-1)^k arg[w] per level; computed from the output side so
-// that stores are coalesced (free_tensor_antipode.hpp:56-99).
-template <typename T>
-__global__ void antipode_kernel(T* out, const T* arg, int64_t ld_out, int64_t ld_arg,
-                                int64_t batch, const LevelTab t)
+// Antipode: out[w] = (-1)^k arg[rev(w)] per level (free_tensor_antipode.hpp:56-99).
+// Reversing a word turns its last letters into its first, so a warp's
+// consecutive words of out lie d^(k-1) apart in arg.  Levels of at least 2 L
+// letters go through square tiles in shared memory: for one middle part, the
+// d^L runs of d^L words (P, rev m, Q) of arg are read as runs and the runs
+// (p, m, q) of out written as runs.  Lower levels, a few hundred words, are
+// gathered from L1 one by one, with divisions by a compile-time width.  Before,
+// every word was gathered so, with 64-bit divisions by a runtime width.
+// Measured on B200, before -> after: (8,5) float32 x 1000 419 -> 76 us (3.9
+// TB/s), (4,6) float64 x 3000 222 -> 73 us, (2,14) float32 x 500 393 -> 60 us,
+// (2,5) float32 x 100000 90 -> 39 us (index arithmetic).
+
+// the first `words` words of every row, one a thread (32-bit indices: the grid's
+// stride past the last word fits)
+template <typename T, int D, typename Index>
+__global__ void antipode_words_kernel(T* out, const T* arg, int64_t ld_out, int64_t ld_arg,
+                                      int64_t batch, Index words, const LevelTab t)
 {
-    const int64_t size = t.db[t.depth + 1];
-    const int64_t total = size * batch;
-    for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < total;
-         g += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t b = g / size;
-        const int64_t i = g - b * size;
+    const Index total = (Index)batch * words;
+    for (Index g = blockIdx.x * (Index)blockDim.x + threadIdx.x; g < total;
+         g += (Index)gridDim.x * blockDim.x) {
+        const Index b = g / words;
+        const uint32_t i = (uint32_t)(g - b * words);
         const int k = level_of(t, i);
-        int64_t j = i - t.db[k];
-        int64_t rev = 0;
+        const uint32_t d = D > 0 ? (uint32_t)D : (uint32_t)t.width;
+        uint32_t j = i - (uint32_t)t.db[k], rev = 0;
         for (int q = 0; q < k; ++q) {
-            rev = rev * t.width + (j % t.width);
-            j /= t.width;
+            const uint32_t next = j / d;
+            rev = rev * d + (j - next * d);
+            j = next;
         }
-        const T v = __ldg(arg + b * ld_arg + t.db[k] + rev);
-        out[b * ld_out + i] = (k & 1) ? -v : v;
+        const T v = __ldg(arg + (int64_t)b * ld_arg + t.db[k] + rev);
+        out[(int64_t)b * ld_out + i] = (k & 1) ? -v : v;
+    }
+}
+
+template <int D, int L>
+struct Letters {
+    static constexpr int count = D * Letters<D, L - 1>::count;
+    // the L digits of v in reverse
+    static __device__ __forceinline__ int reverse(int v)
+    {
+        return (v % D) * Letters<D, L - 1>::count + Letters<D, L - 1>::reverse(v / D);
+    }
+};
+template <int D>
+struct Letters<D, 0> {
+    static constexpr int count = 1;
+    static __device__ __forceinline__ int reverse(int) { return 0; }
+};
+
+constexpr int kAntipodeThreads = 256;
+
+// levels 2 L and above: one tile a block
+template <typename T, int D, int L>
+__global__ void __launch_bounds__(kAntipodeThreads)
+antipode_tiles_kernel(T* out, const T* arg, int64_t ld_out, int64_t ld_arg, int64_t batch,
+                      uint32_t row_tiles, const LevelTab t)
+{
+    constexpr int S = Letters<D, L>::count;
+    __shared__ T tile[S][S + 1];
+    const int64_t total = batch * row_tiles;
+    for (int64_t g = blockIdx.x; g < total; g += gridDim.x) {
+        const int64_t b = g / row_tiles;
+        uint32_t m = (uint32_t)(g - b * row_tiles);
+        int k = 2 * L;
+        while (m >= (uint32_t)t.pw[k - 2 * L]) m -= (uint32_t)t.pw[k++ - 2 * L];
+        uint32_t rev = 0, j = m;
+        for (int q = 0; q < k - 2 * L; ++q) {
+            rev = rev * D + j % D;
+            j /= D;
+        }
+        const uint32_t stride = (uint32_t)t.pw[k - L];   // between the runs of a tile
+        const T* src = arg + b * ld_arg + t.db[k] + rev * (uint32_t)S;
+        T* dst = out + b * ld_out + t.db[k] + m * (uint32_t)S;
+        for (int e = threadIdx.x; e < S * S; e += kAntipodeThreads)
+            tile[e / S][e % S] = __ldg(src + (uint32_t)(e / S) * stride + e % S);
+        __syncthreads();
+        for (int e = threadIdx.x; e < S * S; e += kAntipodeThreads) {
+            const int p = e / S, q = e % S;
+            const T v = tile[Letters<D, L>::reverse(q)][Letters<D, L>::reverse(p)];
+            dst[(uint32_t)p * stride + q] = (k & 1) ? -v : v;
+        }
+        __syncthreads();
     }
 }
 
@@ -275,14 +339,44 @@ RPYB_API int rpyb_ft_antipode(int dtype, int32_t width, int32_t depth, int64_t b
         return fail(RPYB_E_INVALID, "row stride smaller than the tensor size");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const LevelTab t = make_tab(g);
-    const int threads = 256;
-    const unsigned blocks = grid_for(g.size() * batch, threads);
-    if (dtype == RPYB_F64)
-        antipode_kernel<double><<<blocks, threads, 0, s>>>(
-            static_cast<double*>(out), static_cast<const double*>(arg), ld_out, ld_arg, batch, t);
-    else
-        antipode_kernel<float><<<blocks, threads, 0, s>>>(
-            static_cast<float*>(out), static_cast<const float*>(arg), ld_out, ld_arg, batch, t);
+    auto go = [&](auto kind, auto width, auto letters) {
+        using V = decltype(kind);
+        constexpr int D = decltype(width)::value, L = decltype(letters)::value;
+        V* o = static_cast<V*>(out);
+        const V* x = static_cast<const V*>(arg);
+        int64_t words = g.size();
+        if constexpr (L > 0) {
+            if (depth >= 2 * L) {
+                words = g.db[2 * L];
+                const int64_t tiles = g.db[depth - 2 * L + 1];   // sum of d^(k - 2 L)
+                const unsigned blocks = (unsigned)std::min<int64_t>(batch * tiles, 148 * 4096);
+                antipode_tiles_kernel<V, D, L><<<blocks, kAntipodeThreads, 0, s>>>(
+                    o, x, ld_out, ld_arg, batch, (uint32_t)tiles, t);
+            }
+        }
+        const unsigned blocks = grid_for(words * batch, 256);
+        if (words * batch < (int64_t(1) << 31))
+            antipode_words_kernel<V, D, uint32_t><<<blocks, 256, 0, s>>>(o, x, ld_out, ld_arg, batch,
+                                                                         (uint32_t)words, t);
+        else
+            antipode_words_kernel<V, D, int64_t><<<blocks, 256, 0, s>>>(o, x, ld_out, ld_arg, batch,
+                                                                        words, t);
+    };
+    // L letters make runs of 25 to 64 words
+    auto by_width = [&](auto kind) {
+        switch (width) {
+            case 2: go(kind, std::integral_constant<int, 2>{}, std::integral_constant<int, 5>{}); break;
+            case 3: go(kind, std::integral_constant<int, 3>{}, std::integral_constant<int, 3>{}); break;
+            case 4: go(kind, std::integral_constant<int, 4>{}, std::integral_constant<int, 3>{}); break;
+            case 5: go(kind, std::integral_constant<int, 5>{}, std::integral_constant<int, 2>{}); break;
+            case 6: go(kind, std::integral_constant<int, 6>{}, std::integral_constant<int, 2>{}); break;
+            case 7: go(kind, std::integral_constant<int, 7>{}, std::integral_constant<int, 2>{}); break;
+            case 8: go(kind, std::integral_constant<int, 8>{}, std::integral_constant<int, 2>{}); break;
+            default: go(kind, std::integral_constant<int, 0>{}, std::integral_constant<int, 0>{}); break;
+        }
+    };
+    if (dtype == RPYB_F64) by_width(double{});
+    else by_width(float{});
     RPYB_CUDA(cudaGetLastError());
     return RPYB_OK;
 }
