@@ -23,12 +23,15 @@
 // in shared memory next to the constant top level of G.  S_t is recovered from
 // S_{t+1} by the inverse step S_t = S_{t+1} (x) exp(-x_t) and re-anchored to
 // a forward checkpoint every K steps.  The lanes' subtree terms need no
-// communication.  Up to four extra "fold" warps per block trail the lanes by
-// a step: they fold the adjoints of the shared ancestors (levels 1..N-3)
-// level by level and sum the step's gradient (lane partials come pre-reduced
-// by a warp reduce-scatter).  Lanes and fold warps hand buffers over through
-// named barriers (bar.arrive / bar.sync), so the lanes wait for the folding
-// only when they run NB steps ahead.
+// communication.  Extra "fold" warps trail the lanes: they fold the adjoints
+// of the shared ancestors (levels 1..N-3) level by level and sum the step's
+// gradient (lane partials come pre-reduced by a warp reduce-scatter).  They
+// mostly work in two stages, one to three warps (or four) on level N-3 and one
+// warp, a step behind, on the levels above it.  Lanes and stages hand buffers
+// over through named barriers (bar.arrive / bar.sync), so the lanes wait for
+// the folding only when they run NB steps ahead.  What is left is arithmetic:
+// (5,6) float32 x 512 streams of 1024 steps takes 9.97 ms (10.46 with all the
+// levels of a step folded in turn), its 512 blocks being 3.46 waves.
 //
 // Block kernel (every other shape): one block per stream walks all words of
 // the tensor in global memory:
@@ -286,8 +289,31 @@ struct LaneLayout {
     static constexpr int PP = P > 0 ? P : 1;
     static constexpr int64_t W = ipow_c(D, P > 0 ? P : 0);   // lanes per stream
     static constexpr int64_t NT = (W + 31) / 32 * 32;    // lane threads
-    static constexpr int64_t NF = (1024 - NT) / 32 >= 4 ? 4 : (1024 - NT) / 32;  // fold warps
-    static constexpr int64_t NTB = NT + 32 * NF;
+    // Fold warps.  In two stages, NF of them take the ancestors' last level
+    // (P - 1), which the lanes feed, and one more the levels above it and the
+    // step's gradient, a step behind.  In one stage four take every level in
+    // turn.  Folding all levels of a step in turn was what the lanes waited for:
+    // two stages take float32 (5,6) x 512 streams of 1024 steps from 10.46 to
+    // 9.99 ms, (4,6) x 512 of 200 from 1.17 to 1.04 ms.  Not so for float64 lanes
+    // of more than 16 warps, which wait for the float64 pipe: (5,6) x 512 of 200
+    // is 2.31 ms in one stage and 2.51 in two, (3,8) x 148 1.01 and 1.05.
+    // NF follows the words of level P - 1: one warp for up to 32, since fewer
+    // warps a block leave room for more blocks (an SM holds twice as many at
+    // (4,4), 0.35 -> 0.20 ms x 512 of 300); else three, which with the last make
+    // the four schedulers' shares even, or four where one is missing to that.
+    // Nor where the last level is more than two rounds of its warps: (2,11) x
+    // 148 of 100, 0.62 and 0.68 ms.
+    static constexpr int64_t fold_words = P >= 2 ? ipow_c(D, P - 1) : 1;
+    static constexpr int64_t NF2 =
+        fold_words <= 32 ? 1 : (fold_words > 96 && NT / 32 % 4 == 3 ? 4 : 3);
+    // With no shared ancestors (depth 3 and less) one warp sums the gradient, in
+    // one stage ((3,3) x 2000 of 100: 0.23 ms with four, 0.25 with two stages).
+    static constexpr bool TWO =
+        P >= 2 && !(sizeof(T) == 8 && NT > 512) && fold_words <= 64 * NF2;
+    static constexpr int64_t NF = TWO ? NF2 : (P < 2 ? 1 : 4);
+    static constexpr int64_t NTB = NT + 32 * NF + (TWO ? 32 : 0);
+    static_assert(NTB <= 1024, "threads of a block");
+    static constexpr int MINB = NT == 128 ? 2 : 1;       // blocks an SM the registers are held to
     static constexpr int64_t NWARP = NT / 32;
     static constexpr int64_t TOPW = ipow_c(D, N);
     static constexpr bool GT_SMEM = TOPW * (int64_t)sizeof(T) <= 160 * 1024;
@@ -306,16 +332,23 @@ struct LaneLayout {
         return s;
     }
     static constexpr int64_t n_anc = anc_off(P > 1 ? P : 1);
-    static constexpr int64_t n_mbuf = mbuf_off(P > 1 ? P : 1);
+    // M vectors of levels 1..P-1, and a second buffer of level P-1's, which the
+    // fold warps hand over to the last warp
+    static constexpr int64_t n_hand = TWO && P >= 2 ? (int64_t)(N - P + 2) * ipow_c(D, P - 1) : 0;
+    static constexpr int64_t n_mbuf = mbuf_off(P > 1 ? P : 1) + n_hand;
+    __host__ __device__ static constexpr int64_t hand_off(int slot)
+    {
+        return slot == 0 ? mbuf_off(P > 1 ? P - 1 : 1) : mbuf_off(P > 1 ? P : 1);
+    }
     static constexpr int64_t n_mlev = P >= 2 ? 3 * W : 0;
     // shared memory: per hand-off buffer b < NB the lane warps' gradient
     // partials, the fold warps' partials, the lanes' M vectors and the states
     // of shared prefixes; then fold-private ancestor data, the staged
     // increments, the top-level adjoints and the lanes' child adjoints G[pi m]
     // (kept here rather than in registers, which the fold warps cap)
-    __host__ __device__ static constexpr int64_t per_buf()
+    __host__ __device__ static constexpr int64_t ring(int nb)
     {
-        return NWARP * 8 * 8 + NF * 8 * 8 + align16(n_mlev * 8) + align16(n_anc * 8);
+        return nb * align16(n_mlev * 8) + (TWO ? 2 : 1) * nb * (NWARP * 8 * 8 + NF * 8 * 8 + align16(n_anc * 8));
     }
     __host__ __device__ static constexpr int64_t fixed()
     {
@@ -323,12 +356,13 @@ struct LaneLayout {
                align16((int64_t)CH * D * (int64_t)sizeof(T)) +
                (GT_SMEM ? align16(TOPW * (int64_t)sizeof(T)) : 0);
     }
-    static constexpr int NB = (4 * per_buf() + fixed() <= 200 * 1024) ? 4 : 2;   // hand-off buffers
-    static constexpr int64_t o_gxw = 0;                                   // f64 [NB][NWARP][8]
-    static constexpr int64_t o_anct = o_gxw + NB * NWARP * 8 * 8;         // f64 [NB][NF][8]
-    static constexpr int64_t o_mlev = o_anct + NB * NF * 8 * 8;           // f64 [NB][3][W]
-    static constexpr int64_t o_sanc = o_mlev + NB * align16(n_mlev * 8);  // f64 [NB][n_anc]
-    static constexpr int64_t o_mbuf = o_sanc + NB * align16(n_anc * 8);
+    static constexpr int NB = (ring(4) + fixed() <= 200 * 1024) ? 4 : 2;   // hand-off buffers
+    static constexpr int NS = (TWO ? 2 : 1) * NB;
+    static constexpr int64_t o_gxw = 0;                                   // f64 [NS][NWARP][8]
+    static constexpr int64_t o_anct = o_gxw + NS * NWARP * 8 * 8;         // f64 [NS][NF][8]
+    static constexpr int64_t o_mlev = o_anct + NS * NF * 8 * 8;           // f64 [NB][3][W]
+    static constexpr int64_t o_sanc = o_mlev + NB * align16(n_mlev * 8);  // f64 [NS][n_anc]
+    static constexpr int64_t o_mbuf = o_sanc + NS * align16(n_anc * 8);
     static constexpr int64_t o_ganc = o_mbuf + align16(n_mbuf * 8);
     static constexpr int64_t o_xd = o_ganc + align16(n_anc * 8);          // f64 [CH][D]
     static constexpr int64_t o_xt = o_xd + align16((int64_t)CH * D * 8);  // T [CH][D]
@@ -337,11 +371,20 @@ struct LaneLayout {
     static constexpr int64_t bytes = o_gms + align16(D * W * 8);
     static constexpr int64_t mlev_stride = align16(n_mlev * 8) / 8;
     static constexpr int64_t sanc_stride = align16(n_anc * 8) / 8;
-    // named barriers (0 is __syncthreads): lanes filled buffer b, fold warps
-    // released buffer b, and among the fold warps
+    // named barriers (0 is __syncthreads), with the threads that take part:
+    // lanes filled buffer b (lanes arrive, fold warps wait); fold warps are done
+    // with buffer b (they arrive, lanes wait); fold warps filled hand-over slot h
+    // (they arrive, the last warp waits); the last warp is done with slot h (it
+    // arrives, fold warps wait).  What the last warp reads besides its slot has
+    // NS = 2 NB buffers and needs no barrier of its own: fold warps done with step
+    // i - NB have waited for the last warp's step i - NB - 2, and NB >= 2.
     __host__ __device__ static constexpr int bar_full(int b) { return 1 + b; }
     __host__ __device__ static constexpr int bar_empty(int b) { return 1 + NB + b; }
-    static constexpr int bar_fold = 1 + 2 * NB;
+    __host__ __device__ static constexpr int bar_mid(int h) { return 1 + 2 * NB + h; }
+    __host__ __device__ static constexpr int bar_free(int h) { return 3 + 2 * NB + h; }
+    static constexpr int bar_fold = 1 + 2 * NB;          // one stage: among the fold warps
+    static constexpr int n_full = (int)(NT + 32 * NF), n_mid = (int)(32 * NF + 32);
+    static_assert(4 + 2 * NB < 16, "sixteen named barriers");
     __host__ __device__ static constexpr int64_t db(int k) { return (ipow_c(D, k) - 1) / (D - 1); }
 };
 
@@ -418,78 +461,99 @@ struct WarpScatter {
         for (int st = 0; st < LQ; ++st) l = 2 * l + ((lane >> (4 - st)) & 1);
         return l;
     }
+    // a lane that holds letter l's total
+    static __device__ __forceinline__ int lane_of(int l)
+    {
+        int lane = 0;
+#pragma unroll
+        for (int st = 0; st < LQ; ++st) lane |= ((l >> (LQ - 1 - st)) & 1) << (4 - st);
+        return lane;
+    }
     static __device__ __forceinline__ bool writer(int lane) { return (lane & ((16 >> (LQ - 1)) - 1)) == 0; }
 };
 
-// Fold warps, ancestor level K (1 <= K <= P-1): node u (strided over the
-// fold threads) folds its children's M vectors into its own, updates its
-// adjoint and adds its gradient term sum_q F_q(parent(u)) M_q(u) to letter
-// u mod D.
-template <typename T, int D, int N, int K>
-__device__ __forceinline__ void fold_levels(int fl, const double* __restrict__ xr,
-                                            const double* mlev, double* mbuf, double* ganc,
-                                            const double* sanc, double (&gacc)[D])
+// Ancestor level K (1 <= K <= P-1) by NFT threads: node u (strided over them)
+// folds its children's M vectors (child) into its own (own, for the level
+// above), updates its adjoint and adds its gradient term
+// sum_q F_q(parent(u)) M_q(u) to letter u mod D.
+template <typename T, int D, int N, int K, int NFT>
+__device__ __forceinline__ void fold_level(int fl, const double* __restrict__ xr,
+                                           const double* child, double* own, double* ganc,
+                                           const double* sanc, double (&gacc)[D])
+{
+    using LY = LaneLayout<T, D, N>;
+    constexpr int NQ = N - K + 1;
+    constexpr int NU = (int)ipow_c(D, K);
+    constexpr int64_t CS = ipow_c(D, K + 1);
+#pragma unroll
+    for (int u0 = 0; u0 < NU; u0 += NFT) {
+        const int u = u0 + fl;
+        if (u >= NU) break;
+        double Mq[NQ];
+        Mq[0] = ganc[LY::anc_off(K) + u];
+#pragma unroll
+        for (int q = 1; q < NQ; ++q) {
+            double acc = 0.0;
+#pragma unroll
+            for (int cc = 0; cc < D; ++cc)
+                acc = fma(xr[cc], child[(q - 1) * CS + (int64_t)u * D + cc], acc);
+            Mq[q] = acc;
+        }
+        if constexpr (K > 1) {
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) own[q * NU + u] = Mq[q];
+        }
+        double g = Mq[0];
+#pragma unroll
+        for (int q = 1; q < NQ; ++q) g = fma(Mq[q], inv_fact(q), g);
+        ganc[LY::anc_off(K) + u] = g;
+        // parent(u) = u / D at level K-1; the states of its prefixes are in sanc
+        const int par = u / D;
+        double contrib = 0.0;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            double h = 1.0;
+#pragma unroll
+            for (int i = 1; i <= K - 1; ++i) {
+                const int pref = par / (int)ipow_c(D, K - 1 - i);
+                h = fma(h, xr[pref % D] * (1.0 / (double)(q + K + 1 - i)),
+                        sanc[LY::anc_off(i) + pref]);
+            }
+            contrib = fma(h * inv_fact(q + 1), Mq[q], contrib);
+        }
+        const int l = u % D;
+#pragma unroll
+        for (int b = 0; b < D; ++b) gacc[b] += (b == l) ? contrib : 0.0;
+    }
+}
+
+// Levels K down to 1 by NFT threads, each level's M vectors feeding the next:
+// one warp, or the fold warps of one stage.
+template <typename T, int D, int N, int K, int NFT>
+__device__ __forceinline__ void fold_up(int fl, const double* __restrict__ xr,
+                                        const double* child, double* mbuf, double* ganc,
+                                        const double* sanc, double (&gacc)[D])
 {
     if constexpr (K >= 1) {
         using LY = LaneLayout<T, D, N>;
-        constexpr int P = LY::P;
-        constexpr int NQ = N - K + 1;
-        constexpr int NU = (int)ipow_c(D, K);
-        constexpr int64_t CS = ipow_c(D, K + 1);
-        constexpr int NFT = (int)LY::NF * 32;
-        const double* child = (K + 1 == P) ? mlev : (mbuf + LY::mbuf_off(K + 1));
-#pragma unroll
-        for (int u0 = 0; u0 < NU; u0 += NFT) {
-            const int u = u0 + fl;
-            if (u >= NU) break;
-            double Mq[NQ];
-            Mq[0] = ganc[LY::anc_off(K) + u];
-#pragma unroll
-            for (int q = 1; q < NQ; ++q) {
-                double acc = 0.0;
-#pragma unroll
-                for (int cc = 0; cc < D; ++cc)
-                    acc = fma(xr[cc], child[(q - 1) * CS + (int64_t)u * D + cc], acc);
-                Mq[q] = acc;
-            }
-            if constexpr (K > 1) {
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) mbuf[LY::mbuf_off(K) + q * NU + u] = Mq[q];
-            }
-            double g = Mq[0];
-#pragma unroll
-            for (int q = 1; q < NQ; ++q) g = fma(Mq[q], inv_fact(q), g);
-            ganc[LY::anc_off(K) + u] = g;
-            // parent(u) = u / D at level K-1; the states of its prefixes are in sanc
-            const int par = u / D;
-            double contrib = 0.0;
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) {
-                double h = 1.0;
-#pragma unroll
-                for (int i = 1; i <= K - 1; ++i) {
-                    const int pref = par / (int)ipow_c(D, K - 1 - i);
-                    h = fma(h, xr[pref % D] * (1.0 / (double)(q + K + 1 - i)),
-                            sanc[LY::anc_off(i) + pref]);
-                }
-                contrib = fma(h * inv_fact(q + 1), Mq[q], contrib);
-            }
-            const int l = u % D;
-#pragma unroll
-            for (int b = 0; b < D; ++b) gacc[b] += (b == l) ? contrib : 0.0;
-        }
-        bar_sync_n(LY::bar_fold, NFT);
-        fold_levels<T, D, N, K - 1>(fl, xr, mlev, mbuf, ganc, sanc, gacc);
+        double* own = mbuf + LY::mbuf_off(K);
+        fold_level<T, D, N, K, NFT>(fl, xr, child, own, ganc, sanc, gacc);
+        if constexpr (NFT == 32)
+            __syncwarp();
+        else
+            bar_sync_n(LY::bar_fold, NFT);
+        fold_up<T, D, N, K - 1, NFT>(fl, xr, own, mbuf, ganc, sanc, gacc);
     }
 }
 
 template <typename T, int D, int N>
-__global__ void __launch_bounds__(LaneLayout<T, D, N>::NTB, 1)
+__global__ void __launch_bounds__(LaneLayout<T, D, N>::NTB, LaneLayout<T, D, N>::MINB)
 signature_backward_lanes(const BwdArgs a)
 {
     using LY = LaneLayout<T, D, N>;
     constexpr int P = LY::P, PP = LY::PP, CH = LY::CH, NB = LY::NB;
     constexpr int W = (int)LY::W, NT = (int)LY::NT, NTB = (int)LY::NTB, NWARP = (int)LY::NWARP;
+    constexpr int NF = (int)LY::NF;
     constexpr bool GT_SMEM = LY::GT_SMEM;
 
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -618,7 +682,7 @@ signature_backward_lanes(const BwdArgs a)
                 for (int i = 0; i < n; ++i) {
                     const int j = n - 1 - i;
                     const int64_t t = t0 + j;
-                    const int bb = i % NB;
+                    const int bb = i % NB, sb = i & (LY::NS - 1);
                     const double* row = xd + j * D;
                     const T* rowt = xt + j * D;
                     double x[D], xc[PP];
@@ -639,11 +703,11 @@ signature_backward_lanes(const BwdArgs a)
                         --rc;
                     }
                     // buffer bb is free once the fold warps are done with step i - NB
-                    if (i >= NB) bar_sync_n(LY::bar_empty(bb), NTB);
+                    if (i >= NB) bar_sync_n(LY::bar_empty(bb), LY::n_full);
 
                     // states of shared prefixes (levels 1..P-2) for the fold warps
                     if constexpr (P >= 3) {
-                        double* sa = sanc + bb * LY::sanc_stride;
+                        double* sa = sanc + sb * LY::sanc_stride;
 #pragma unroll
                         for (int q = 1; q <= P - 2; ++q)
                             if (own & (1u << q)) sa[LY::anc_off(q) + pi / (int)ipow_c(D, P - q)] = sp[q - 1];
@@ -712,27 +776,27 @@ signature_backward_lanes(const BwdArgs a)
                     {
                         const T r = WS::run(gx, lane);
                         const int l = WS::letter(lane);
-                        if (WS::writer(lane) && l < D) gxw[(bb * NWARP + warp) * 8 + l] = (double)r;
+                        if (WS::writer(lane) && l < D) gxw[(sb * NWARP + warp) * 8 + l] = (double)r;
                     }
-                    bar_arrive_n(LY::bar_full(bb), NTB);
+                    bar_arrive_n(LY::bar_full(bb), LY::n_full);
                 }
                 // take the fold warps' last releases so every barrier is balanced
-                for (int i = (n > NB ? n - NB : 0); i < n; ++i) bar_sync_n(LY::bar_empty(i % NB), NTB);
-            } else {
+                for (int i = (n > NB ? n - NB : 0); i < n; ++i)
+                    bar_sync_n(LY::bar_empty(i % NB), LY::n_full);
+            } else if constexpr (!LY::TWO) {
                 using WS = WarpScatter<D, double>;
-                constexpr int NF = (int)LY::NF;
                 const int fl = tid - NT;          // 0 .. 32 NF - 1
                 const int fw = fl >> 5;
                 for (int i = 0; i < n; ++i) {
                     const int j = n - 1 - i;
                     const int64_t t = t0 + j;
                     const int bb = i % NB;
-                    bar_sync_n(LY::bar_full(bb), NTB);
+                    bar_sync_n(LY::bar_full(bb), LY::n_full);
                     double gacc[D];
 #pragma unroll
                     for (int b = 0; b < D; ++b) gacc[b] = 0.0;
-                    fold_levels<T, D, N, P - 1>(fl, xd + j * D, mlev + bb * LY::mlev_stride, mbuf,
-                                                ganc, sanc + bb * LY::sanc_stride, gacc);
+                    fold_up<T, D, N, P - 1, 32 * NF>(fl, xd + j * D, mlev + bb * LY::mlev_stride, mbuf,
+                                                     ganc, sanc + bb * LY::sanc_stride, gacc);
                     const double r = WS::run(gacc, lane);
                     const int l = WS::letter(lane);
                     if (WS::writer(lane) && l < D) anct[(bb * NF + fw) * 8 + l] = r;
@@ -745,7 +809,70 @@ signature_backward_lanes(const BwdArgs a)
                         for (int w2 = 0; w2 < NWARP; ++w2) v += gxw[(bb * NWARP + w2) * 8 + fl];
                         gout[t * D + fl] = (T)v;
                     }
-                    bar_arrive_n(LY::bar_empty(bb), NTB);
+                    bar_arrive_n(LY::bar_empty(bb), LY::n_full);
+                }
+            } else if (tid < NT + 32 * NF) {
+                // the last ancestor level, from the lanes' M vectors
+                using WS = WarpScatter<D, double>;
+                const int fl = tid - NT;          // 0 .. 32 NF - 1
+                const int fw = fl >> 5;
+                for (int i = 0; i < n; ++i) {
+                    const int j = n - 1 - i;
+                    const int bb = i % NB, sb = i & (LY::NS - 1), h = i & 1;
+                    bar_sync_n(LY::bar_full(bb), LY::n_full);
+                    // slot h is free once the last warp is done with step i - 2
+                    if (i >= 2) bar_sync_n(LY::bar_free(h), LY::n_mid);
+                    double gacc[D];
+#pragma unroll
+                    for (int b = 0; b < D; ++b) gacc[b] = 0.0;
+                    if constexpr (P >= 2)
+                        fold_level<T, D, N, P - 1, 32 * NF>(
+                            fl, xd + j * D, mlev + bb * LY::mlev_stride, mbuf + LY::hand_off(h), ganc,
+                            sanc + sb * LY::sanc_stride, gacc);
+                    const double r = WS::run(gacc, lane);
+                    const int l = WS::letter(lane);
+                    if (WS::writer(lane) && l < D) anct[(sb * NF + fw) * 8 + l] = r;
+                    bar_arrive_n(LY::bar_mid(h), LY::n_mid);
+                    bar_arrive_n(LY::bar_empty(bb), LY::n_full);
+                }
+                // take the last warp's last releases
+                for (int i = (n > 2 ? n - 2 : 0); i < n; ++i) bar_sync_n(LY::bar_free(i & 1), LY::n_mid);
+            } else {
+                // the levels above, and the step's gradient
+                using WS = WarpScatter<D, double>;
+                for (int i = 0; i < n; ++i) {
+                    const int j = n - 1 - i;
+                    const int64_t t = t0 + j;
+                    const int sb = i & (LY::NS - 1), h = i & 1;
+                    bar_sync_n(LY::bar_mid(h), LY::n_mid);
+                    double gacc[D];
+#pragma unroll
+                    for (int b = 0; b < D; ++b) gacc[b] = 0.0;
+                    if constexpr (P >= 3)
+                        fold_up<T, D, N, P - 2, 32>(lane, xd + j * D, mbuf + LY::hand_off(h), mbuf, ganc,
+                                                sanc + sb * LY::sanc_stride, gacc);
+                    // the fold warps' and the lanes' partials join lane by lane: lane
+                    // 8 part + letter takes every fourth of them
+                    const int letter = lane & 7, part = lane >> 3;
+                    double v = 0.0;
+                    if (letter < D) {
+#pragma unroll
+                        for (int w2 = part; w2 < NF; w2 += 4) v += anct[(sb * NF + w2) * 8 + letter];
+#pragma unroll
+                        for (int w2 = 0; w2 < (NWARP + 3) / 4; ++w2)
+                            if (4 * w2 + part < NWARP) v += gxw[(sb * NWARP + 4 * w2 + part) * 8 + letter];
+                    }
+                    if constexpr (P >= 3) {
+                        // this warp's own terms, scattered to the same lanes
+                        const double r = WS::run(gacc, lane);
+                        const int from = letter < D ? WS::lane_of(letter) : 0;
+                        const double mine = __shfl_sync(0xffffffffu, r, from);
+                        if (part == 0 && letter < D) v += mine;
+                    }
+                    v += __shfl_xor_sync(0xffffffffu, v, 8);
+                    v += __shfl_xor_sync(0xffffffffu, v, 16);
+                    if (lane < D) gout[t * D + lane] = (T)v;
+                    bar_arrive_n(LY::bar_free(h), LY::n_mid);
                 }
             }
         }
@@ -766,6 +893,7 @@ struct LaneEntry {
     void (*fn)(BwdArgs) = nullptr;
     int64_t smem = 0;
     int threads = 0;
+    int least_threads = 0;
     int64_t lanes = 0;
     int ckw = 0;
 };
@@ -779,6 +907,7 @@ bool lane_fill(LaneEntry& e)
             e.fn = &signature_backward_lanes<T, D, N>;
             e.smem = LY::bytes;
             e.threads = (int)LY::NTB;
+            e.least_threads = (int)LY::NT + 160;
             e.lanes = LY::W;
             e.ckw = LY::PP + D;
             return true;
@@ -831,18 +960,37 @@ int64_t lane_slot_bytes(const LaneEntry& e, int64_t max_segments)
     return (max_segments * e.ckw * e.lanes * 8 + 255) / 256 * 256;
 }
 
-// blocks in flight for the lane kernel (one workspace slot each)
-int64_t lane_slots(const LaneEntry& e, int64_t n_streams)
+// Blocks in flight for the lane kernel (one workspace slot each): as many as
+// fit, or, with `least`, as many as fit of blocks of least_threads, which is
+// the count that a caller's workspace has to hold.
+int64_t lane_slots(const LaneEntry& e, int64_t n_streams, bool least)
 {
     int dev = 0, sms = 148, occ = 1;
     if (cudaGetDevice(&dev) == cudaSuccess) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (cudaFuncSetAttribute(e.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)e.smem) == cudaSuccess)
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, e.fn, e.threads, (size_t)e.smem);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                &occ, e.fn, least ? e.least_threads : e.threads, (size_t)e.smem);
         cudaGetLastError();
     }
     return std::min<int64_t>(std::max<int64_t>(1, n_streams), (int64_t)sms * std::max(occ, 1));
+}
+
+// The slots beyond the least are taken while the checkpoints of all of them
+// stay within this (they are 24 MB for 512 streams of 1024 steps at width 8,
+// depth 4; streams of a million steps would take 23 GB).
+constexpr int64_t kLaneScratch = (int64_t)256 << 20;
+
+int64_t lane_workspace(const LaneEntry& e, int64_t n_streams, int64_t segments, bool least)
+{
+    const int64_t slot = lane_slot_bytes(e, segments);
+    const int64_t few = lane_slots(e, n_streams, true);
+    if (!least) {
+        const int64_t all = lane_slots(e, n_streams, false);
+        if (all > few && all * slot <= kLaneScratch) return 256 + all * slot;
+    }
+    return 256 + few * slot;
 }
 
 template <typename T>
@@ -943,7 +1091,7 @@ RPYB_API int64_t rpyb_signature_backward_workspace_size(int mode, int32_t width,
     const int64_t segs = std::max<int64_t>(1, (max_len + checkpoint_every - 1) / checkpoint_every);
     LaneEntry e;
     if (lane_entry(mode, width, depth, e))
-        return 256 + lane_slots(e, n_streams) * lane_slot_bytes(e, segs);
+        return lane_workspace(e, n_streams, segs, false);
     const int64_t slots = std::min<int64_t>(backward_slots(), std::max<int64_t>(1, n_streams));
     return 256 + slots * slot_bytes_for(mode, g, checkpoint_every, segs);
 }
@@ -985,11 +1133,26 @@ RPYB_API int rpyb_signature_backward(int mode, int32_t width, int32_t depth, int
                                         " increments, more than max_len = " +
                                         std::to_string(max_len));
     }
-    const int64_t need = rpyb_signature_backward_workspace_size(mode, width, depth, n_streams,
-                                                                max_len, checkpoint_every);
+    int64_t need = rpyb_signature_backward_workspace_size(mode, width, depth, n_streams, max_len,
+                                                          checkpoint_every);
+    LaneEntry e;
+    const bool lanes = lane_entry(mode, width, depth, e);
+    int64_t least = need;
+    if (lanes) {
+        // a smaller workspace runs fewer blocks, down to the least count
+        least = lane_workspace(e, n_streams,
+                               std::max<int64_t>(1, (max_len + checkpoint_every - 1) / checkpoint_every),
+                               true);
+        if (workspace) need = std::max<int64_t>(least, std::min<int64_t>(need, (int64_t)workspace_bytes));
+    }
     Scratch scratch(workspace, workspace_bytes, s);
     void* ws = nullptr;
-    if ((rc = scratch.get((size_t)need, &ws))) return rc;
+    if ((rc = scratch.get((size_t)need, &ws))) {
+        if (need == least || workspace) return rc;
+        cudaGetLastError();
+        need = least;
+        if ((rc = scratch.get((size_t)need, &ws))) return rc;
+    }
 
     BwdArgs a{};
     a.width = width;
@@ -1008,10 +1171,10 @@ RPYB_API int rpyb_signature_backward(int mode, int32_t width, int32_t depth, int
     a.queue = static_cast<int*>(ws);
     a.scratch = static_cast<char*>(ws) + 256;
     RPYB_CUDA(cudaMemsetAsync(ws, 0, sizeof(int), s));
-    LaneEntry e;
-    if (lane_entry(mode, width, depth, e)) {
+    if (lanes) {
         a.slot_bytes = lane_slot_bytes(e, a.max_segments);
-        const int64_t slots = lane_slots(e, n_streams);
+        const int64_t slots = std::min<int64_t>(lane_slots(e, n_streams, false),
+                                                (need - 256) / std::max<int64_t>(a.slot_bytes, 1));
         e.fn<<<(unsigned)slots, e.threads, (size_t)e.smem, s>>>(a);
         RPYB_CUDA(cudaGetLastError());
         return RPYB_OK;
