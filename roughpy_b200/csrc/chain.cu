@@ -18,10 +18,10 @@
 // The layout before kept the top level in registers (18 words a thread, one
 // block of 512 an SM) and read every operand of a split through L1 in strided
 // words: 1.39 ms for 8192 queries of at most four (6,5) factors, log and
-// projection, on a 2^14-event float64 tree, against 0.57 ms here, where
-// shared-memory wavefronts (68 % busy) bound it, the projection's gathers among
-// them.  100000 such queries, with the host's dissection: 18.6 -> 14.0 ms (the
-// host then being the longer side); 20000 at (5,5), which did not fit the
+// projection, on a 2^14-event float64 tree, against 1.06 ms here, where
+// shared-memory wavefronts (73 % busy) and issue (54 %) bound it, the
+// projection's gathers among them.  100000 such queries: 18.5 -> 14.0 ms with
+// the host's dissection, 13.0 with the device's; 20000 at (5,5), which did not fit the
 // registers, 4.9 -> 2.0 ms.
 #include <algorithm>
 

@@ -17,8 +17,8 @@
 //     at the pair of blocks -1, 0 (no dyadic interval spans the origin).
 //
 // A query [a, b) is trimmed to the support (streams/src/stream.cpp:37-71),
-// dissected into maximal dyadic pieces on the host
-// (intervals/src/dyadic_interval.cpp:191-224), each piece is mapped to a tree
+// dissected into maximal dyadic pieces on the host, or on the device for
+// batches of 256 and more (intervals/src/dyadic_interval.cpp:191-224), each piece is mapped to a tree
 // node, and every query's node signatures are multiplied in order on the
 // device in float64 (float32 nodes enter through the mixed-precision
 // product).  log, then the tensor->Lie map, give the log-signature
@@ -902,8 +902,9 @@ RPYB_API int rpyb_dyadic_query(const rpyb_dyadic_tree* t, int64_t n_queries,
     const int R = t->resolution;
 
     // Many queries whose shape has the fused kernel are dissected on the device:
-    // on the host it took 0.14 us a query, 14 ms of the 14 ms for 100000 (6,5)
-    // queries; few are as fast here, without the extra launch.
+    // on the host it takes 0.09 to 0.14 us a query, which was most of the time of
+    // 100000 queries at (3,4) (9.35 -> 0.75 ms) and the last millisecond of it at
+    // (6,5) (14.0 -> 13.0 ms); few are as fast here, without the extra launch.
     int max_tol = 0;
     if (n_queries >= 256 && chain_lie_available(g, *t->maps) &&
         device_dissection(t, n_queries, inf_host, sup_host, resolution, &max_tol))

@@ -14,7 +14,10 @@
 // levels stay hot in L2, blockIdx.y walks rows.  Float64 rows of width 2
 // take their levels >= 8 from a kernel whose 32 lanes own the last five
 // letters of a word instead (product_kernel_w2: every load one coalesced
-// request or one broadcast).
+// request or one broadcast).  Rows whose lower levels fit shared memory as
+// float64 go to the row-resident kernels of product_rows.cu, unless a level is
+// bounded (max_degree) or one of the RPYB_* choices of a kernel here is made;
+// width 2 then reaches the lane-letter kernel for depths above 13 only.
 //
 // Arithmetic.  float64: the terms are added in the reference order (lhs
 // degree from high to low, free_tensor_fma.hpp:31-46) with FMA.  float32: by

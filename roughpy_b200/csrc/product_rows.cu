@@ -242,7 +242,7 @@ product_rows_kernel(const RowArgs a)
 // p = 1, whose right words R_{N-1}[a, rho] are one run, and the streamed ends.
 // Levels below N are a row-resident product of their own.   Measured on B200, (8,6)
 // float32 x 1024 accumulating 1149 -> 1000 us (4.9 TB/s); in place (8,6) float32
-// x 500 1.23 -> 0.47 ms.  What bounds it is the latency of the streamed words at
+// x 500 1.16 -> 0.47 ms.  What bounds it is the latency of the streamed words at
 // 27 warps an SM: 45 % DRAM, 43 % shared-memory pipe, 41 % issue.
 template <typename T, typename TR, bool ACCUM, int D>
 __global__ void __launch_bounds__(kRowThreads, 1)

@@ -25,10 +25,10 @@ on the GPU by the native runtime behind the C ABI (``rpyb_dyadic_build``): leaf
 signatures come from the batched signature kernel (level-1 increments) or from
 exp of the embedded Lie increments (general increments), and every coarser node
 is the product of its children (one batched product launch per level).  A query
-batch (``rpyb_dyadic_query``) is trimmed and dissected on the host, then each
-query is the ordered product of at most ~2 x resolution cached node signatures
-(batched across queries, one launch per piece position), followed by a float64
-log and the Lie projection.  Since ``log``/``exp`` are mutually inverse on
+batch (``rpyb_dyadic_query``) is trimmed and dissected, on the device where it
+is large and on the host otherwise, then each query is the ordered product of at
+most ~2 x resolution cached node signatures, followed by a float64 log and the
+Lie projection (one launch where the shape fits shared memory).  Since ``log``/``exp`` are mutually inverse on
 group-like elements and CBH is associative, this equals the reference's CBH
 recursion up to rounding.  This module keeps the reference's construction
 rules (event de-duplication, the resolution heuristic, the default support).
