@@ -423,7 +423,8 @@ static int adjoint_left_mul(int dtype, int32_t width, int32_t depth, int64_t bat
     const int64_t T = g.db[out_max + 1];
     const bool warp = T <= 1024;
     const bool stage = !warp && staged <= 108 * 1024 && batch >= 64;
-    const int threads = warp ? 32 : (T >= 16384 && batch <= 64) ? 1024 : 256;
+    // columns of a tile: the threads of the kernel that is launched below
+    const int threads = warp ? 32 : !stage && T >= 16384 && batch <= 64 ? 1024 : 256;
     int32_t tiles = 0;
     for (int k = 0; k <= out_max; ++k) {
         a.tile0[k] = tiles;
