@@ -162,11 +162,12 @@ __device__ __forceinline__ void adjoint_tile(const AdjointArgs& a, T* __restrict
     }
     const int i = c0 + (t - slice * cols);
     const T* ar = arg + a.db[k] + i;
-    const int E = (int)a.E[k];
+    // unsigned: e passes E, which may be close to 2^31, by up to 8 slices
+    const unsigned E = (unsigned)a.E[k];
     double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
     if (slice < slices) {
-        int e = slice;
-        for (; e + 7 * slices < E; e += 8 * slices) {
+        unsigned e = (unsigned)slice;
+        for (; e + 7u * slices < E; e += 8u * slices) {
             double o[8], x[8];
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
@@ -178,7 +179,7 @@ __device__ __forceinline__ void adjoint_tile(const AdjointArgs& a, T* __restrict
             s2 = fma(o[2], x[2], fma(o[6], x[6], s2));
             s3 = fma(o[3], x[3], fma(o[7], x[7], s3));
         }
-        for (; e < E; e += slices) s0 = fma((double)op[e], (double)ar[(int64_t)e * n], s0);
+        for (; e < E; e += (unsigned)slices) s0 = fma((double)op[e], (double)ar[(int64_t)e * n], s0);
     }
     double sum = (s0 + s1) + (s2 + s3);
     // the slices, halved until one is left
