@@ -231,6 +231,7 @@ adjoint_warp_kernel(T* out, const T* op, const T* arg, const AdjointArgs a)
 // per group of tiles of few terms (a block of one multiply-add a thread costs
 // more to start than to run)
 constexpr int kAdjointGroup = 8;
+constexpr int64_t kAdjointSmem = 108 * 1024;   // staged words of a block
 template <typename T, int THREADS, bool STAGED>
 __global__ void __launch_bounds__(THREADS)
 adjoint_block_kernel(T* out, const T* op, const T* arg, const AdjointArgs a)
@@ -423,7 +424,7 @@ static int adjoint_left_mul(int dtype, int32_t width, int32_t depth, int64_t bat
     // rows would leave the chip idle, so there the tiles are spread over it.
     const int64_t T = g.db[out_max + 1];
     const bool warp = T <= 1024;
-    const bool stage = !warp && staged <= 108 * 1024 && batch >= 64;
+    const bool stage = !warp && staged <= kAdjointSmem && batch >= 64;
     // columns of a tile: the threads of the kernel that is launched below
     const int threads = warp ? 32 : !stage && T >= 16384 && batch <= 64 ? 1024 : 256;
     int32_t tiles = 0;
@@ -450,8 +451,7 @@ static int adjoint_left_mul(int dtype, int32_t width, int32_t depth, int64_t bat
             adjoint_warp_kernel<V><<<nb, 256, 0, s>>>(o, p, x, a);
         } else if (stage) {
             auto fn = adjoint_block_kernel<V, 256, true>;
-            RPYB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)staged));
+            if (int rc = allow_shared_memory(fn, staged, kAdjointSmem)) return rc;
             fn<<<nb, 256, staged, s>>>(o, p, x, a);
         } else if (threads == 256) {
             adjoint_block_kernel<V, 256, false><<<nb, 256, 0, s>>>(o, p, x, a);

@@ -404,8 +404,7 @@ static int run_chain(int src_mode, const Geometry& g, const ChainArgs& a, cudaSt
     threads = std::max<int64_t>(threads, 32);
     const unsigned grid = (unsigned)std::min<int64_t>(a.n, 1 << 20);
     ChainFn fn = src_mode == RPYB_F64 ? chain_fn<double>(g.width) : chain_fn<float>(g.width);
-    if (smem > 48 * 1024)
-        RPYB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int rc = allow_shared_memory(fn, smem, kChainSmem)) return rc;
     fn<<<grid, (unsigned)threads, smem, s>>>(a);
     RPYB_CUDA(cudaGetLastError());
     return RPYB_OK;

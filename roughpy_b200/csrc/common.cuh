@@ -62,6 +62,18 @@ private:
     void* owned_ = nullptr;
 };
 
+// Leave for `fn` to take `bytes` of dynamic shared memory.  The limit is a
+// property of the function, which calls of other shapes on other host threads
+// share: every call sets it to the same `most`, so that none lowers it between
+// another's setting and launch.  (48 KB, static part included, need no leave.)
+template <typename Fn>
+int allow_shared_memory(Fn fn, size_t bytes, int64_t most)
+{
+    if (bytes > 40 * 1024)
+        RPYB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    return RPYB_OK;
+}
+
 // ----------------------------------------------- compensated arithmetic --
 // Error-free transformations (Knuth two-sum, FMA two-product).  The
 // explicit _rn intrinsics stop the compiler from contracting a product into

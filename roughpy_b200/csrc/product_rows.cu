@@ -31,6 +31,7 @@ namespace {
 
 // dynamic shared memory a block may take (227 KB less the static part)
 constexpr int64_t kRowSmem = 226 * 1024;
+constexpr int64_t kRowSmemMost = kRowSmem + 64;   // with stage_room's padding
 constexpr int kRowThreads = 1024;   // most threads a block
 
 struct RowArgs {
@@ -434,8 +435,7 @@ int launch_product_rows(int dtype, const Geometry& g, const ProductSpec& spec,
     if (!in_place && rows.batch < 148)
         slices = std::max<int64_t>(1, std::min<int64_t>({16, 296 / rows.batch, units / (2 * threads)}));
     const dim3 grid((unsigned)slices, (unsigned)std::min<int64_t>(rows.batch, 65535), 1);
-    if (smem > 48 * 1024)
-        RPYB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int rc = allow_shared_memory(fn, smem, kRowSmemMost)) return rc;
     fn<<<grid, (unsigned)threads, smem, stream>>>(a);
     RPYB_CUDA(cudaGetLastError());
     return RPYB_OK;
@@ -461,8 +461,7 @@ int launch_product_slabs(int dtype, const Geometry& g, const ProductSpec& spec,
         fn = spec.accumulate ? slab_fn<float, float, true>(g.width) : slab_fn<float, float, false>(g.width);
     const size_t smem = (size_t)(2 * stage_room((int)g.db[a.top - 1]) * 8);
     const int64_t threads = row_threads(g.pw[a.top - 2], smem);
-    if (smem > 48 * 1024)
-        RPYB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int rc = allow_shared_memory(fn, smem, kRowSmemMost)) return rc;
     const dim3 grid((unsigned)g.width, (unsigned)std::min<int64_t>(rows.batch, 65535), 1);
     // the top level first: in place, the lower levels it reads are still the old ones
     fn<<<grid, (unsigned)threads, smem, stream>>>(a);

@@ -337,8 +337,7 @@ int launch_series(int dtype, SeriesKind kind, const Geometry& g, int top, int ar
     if ((kind != kSeriesLog || rows.fresh) && rows.batch < 148)
         slices = std::max<int64_t>(1, std::min<int64_t>({16, 296 / rows.batch, units / (2 * threads)}));
     const dim3 grid((unsigned)slices, (unsigned)std::min<int64_t>(rows.batch, 65535), 1);
-    if (smem > 48 * 1024)
-        RPYB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int rc = allow_shared_memory(fn, smem, kSeriesSmem)) return rc;
     fn<<<grid, (unsigned)threads, smem, stream>>>(a);
     RPYB_CUDA(cudaGetLastError());
     return RPYB_OK;

@@ -33,6 +33,7 @@ constexpr int64_t kSortWindow = 128;
 constexpr int64_t kSortEntries = 8;   // entries a row from which rows are sorted
 constexpr uint32_t kColBits = 20;
 constexpr int64_t kMaxTab = 4096;
+constexpr int64_t kMapRoom = 100 * 1024;   // shared memory of a block when two fit an SM
 
 struct MapArgs {
     const double* tab;
@@ -152,8 +153,7 @@ int launch_map(const MapArgs& a, T* y, const T* x, cudaStream_t s)
 {
     auto fn = packed_map_kernel<T, RB, STAGED>;
     const size_t smem = (size_t)a.ntab * 8 + (STAGED ? (size_t)RB * a.n_cols * sizeof(T) : 0);
-    if (smem > 48 * 1024)
-        RPYB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int rc = allow_shared_memory(fn, smem, 2 * kMapRoom)) return rc;
     const int64_t blocks = (a.batch + RB - 1) / RB;
     if (blocks > 0x7fffffff) return fail(RPYB_E_UNSUPPORTED, "batch too large");
     // few rows: blocks share a row block's groups
@@ -170,7 +170,7 @@ int launch_map_rows(const MapArgs& a, T* y, const T* x, cudaStream_t s)
     // As many rows a block as leave room for two blocks an SM and blocks for
     // every SM; a row that fits only alone is staged alone, a longer one read
     // where it is.
-    const int64_t row = (int64_t)a.n_cols * sizeof(T), room = 100 * 1024 - a.ntab * 8;
+    const int64_t row = (int64_t)a.n_cols * sizeof(T), room = kMapRoom - a.ntab * 8;
     const int64_t want = std::max<int64_t>(1, a.batch / 296);
     if (8 * row <= room && want >= 8) return launch_map<T, 8, true>(a, y, x, s);
     if (4 * row <= room && want >= 4) return launch_map<T, 4, true>(a, y, x, s);
