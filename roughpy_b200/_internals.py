@@ -110,6 +110,8 @@ class SparseMatrix:
         used, self._used = self._used, True
         if not used and self.nnz * batch < (1 << 21):
             return None
+        if ("packed", str(device)) not in self._dev and torch.cuda.is_current_stream_capturing():
+            return None   # no upload in a capture: the CSR arrays of an earlier call serve
         return self.device_packed(device)
 
     def device_packed(self, device):
