@@ -120,9 +120,9 @@ class SparseMatrix:
         key = ("packed", str(device))
         if key not in self._dev:
             data = np.ascontiguousarray(self.data, dtype=np.float64)
+            indptr, indices = (np.ascontiguousarray(a) for a in (self.indptr, self.indices))
             layout = (ctypes.c_int64 * 3)()
-            args = (*self.shape, self.indptr.ctypes.data, self.indices.ctypes.data,
-                    data.ctypes.data)
+            args = (*self.shape, indptr.ctypes.data, indices.ctypes.data, data.ctypes.data)
             size = int(_lib.lib.rpyb_sparse_pack(*args, None, 0, layout))
             if size >= 0:
                 block = np.empty(max(size, 1), dtype=np.uint8)
