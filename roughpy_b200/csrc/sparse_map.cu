@@ -340,10 +340,10 @@ RPYB_API int64_t rpyb_sparse_pack(int64_t n_rows, int64_t n_cols, const int64_t*
 {
     if (n_rows < 0 || n_cols < 0) return fail(RPYB_E_INVALID, "negative size");
     if (!indptr || !layout) return fail(RPYB_E_INVALID, "null pointer");
+    // a row that ends before it begins is empty, as in rpyb_sparse_map
     for (int64_t r = 0; r < n_rows; ++r)
-        if (indptr[r + 1] < indptr[r]) return fail(RPYB_E_INVALID, "indptr must not decrease");
-    if (indptr[n_rows] > indptr[0] && (!indices || !values))
-        return fail(RPYB_E_INVALID, "null pointer");
+        if (indptr[r + 1] > indptr[r] && (!indices || !values))
+            return fail(RPYB_E_INVALID, "null pointer");
     PackedMap m;
     try {
         if (!block) {

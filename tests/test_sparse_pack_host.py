@@ -48,3 +48,14 @@ def test_packed_entries(rows, cols, per_row, layout):
     want = SparseMatrix(indptr, indices, data, (rows, cols)).todense()
     got = unpack(SparseMatrix(layout(indptr), layout(indices), layout(data), (rows, cols)))
     assert np.array_equal(got, want)
+
+
+def test_rows_that_end_before_they_begin_are_empty():
+    """As the CSR kernel has it, which serves a matrix's first small call."""
+    indptr = np.array([0, 3, 1, 4, 4], dtype=np.int64)
+    indices = np.array([0, 2, 4, 1], dtype=np.int64)
+    data = np.array([1.0, -2.0, 0.5, 3.0])
+    want = np.zeros((4, 5))
+    want[0, [0, 2, 4]] = data[:3]
+    want[2, [2, 4, 1]] = data[1:]
+    assert np.array_equal(unpack(SparseMatrix(indptr, indices, data, (4, 5))), want)
