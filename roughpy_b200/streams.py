@@ -193,6 +193,15 @@ def _dissect_batch(infs, sups, tols):
     return k[:m], p[:m], off
 
 
+def _interval_ends(infs, sups):
+    """Both ends as dense float64 vectors; every interval needs its sup (more are ignored)."""
+    infs = np.ascontiguousarray(infs, dtype=np.float64).reshape(-1)
+    sups = np.ascontiguousarray(sups, dtype=np.float64).reshape(-1)
+    if sups.shape[0] < infs.shape[0]:
+        raise ValueError(f"{infs.shape[0]} interval starts but {sups.shape[0]} ends")
+    return infs, sups
+
+
 class _StreamQueries:
     """Query front end shared by the stream classes (the reference's
     Stream::log_signature / signature / signature_derivative and its Python
@@ -233,15 +242,13 @@ class _StreamQueries:
     def log_signature_batch(self, infs, sups, resolution=None, chunk=16384):
         """Log-signatures (Hall coordinates, float64) of many clopen intervals."""
         resolution = _resolution_arg(resolution)
-        infs = np.asarray(infs, dtype=np.float64).reshape(-1)
-        sups = np.asarray(sups, dtype=np.float64).reshape(-1)
+        infs, sups = _interval_ends(infs, sups)
         return self._batch(infs, sups, resolution, chunk, self.lie_basis.size(), False)
 
     def signature_batch(self, infs, sups, resolution=None, chunk=16384):
         """Signatures exp(l2t(log_signature)) (float64) of many clopen intervals."""
         resolution = _resolution_arg(resolution)
-        infs = np.asarray(infs, dtype=np.float64).reshape(-1)
-        sups = np.asarray(sups, dtype=np.float64).reshape(-1)
+        infs, sups = _interval_ends(infs, sups)
         return self._batch(infs, sups, resolution, chunk, self.tensor_basis.size(), True)
 
     def _batch(self, infs, sups, resolution, chunk, cols, sig):
@@ -520,12 +527,11 @@ class LieIncrementStream(_StreamQueries):
     def _query(self, infs, sups, resolution, logsig=True, sig=False, out=None):
         """One rpyb_dyadic_query over clopen intervals; float64 device outputs (`out` where
         given and one of them is asked for)."""
+        infs, sups = _interval_ends(infs, sups)
         tr = self._build_tree()
-        infs = np.ascontiguousarray(infs, dtype=np.float64).reshape(-1)
         if (self.auto_range_table and not tr.range_table and infs.shape[0] >= 1024
                 and tr.rows >= 8192):
             self.build_range_table()
-        sups = np.ascontiguousarray(sups, dtype=np.float64).reshape(-1)
         n = infs.shape[0]
         L, T = self.lie_basis.size(), self.tensor_basis.size()
         if out is not None:
@@ -663,8 +669,7 @@ class PiecewiseAbelianStream(_StreamQueries):
                    support, device)
 
     def _query(self, infs, sups, resolution, logsig=True, sig=False, out=None):
-        infs = np.ascontiguousarray(infs, dtype=np.float64).reshape(-1)
-        sups = np.ascontiguousarray(sups, dtype=np.float64).reshape(-1)
+        infs, sups = _interval_ends(infs, sups)
         n = infs.shape[0]
         L, T = self.lie_basis.size(), self.tensor_basis.size()
         if out is not None:
