@@ -32,7 +32,7 @@ namespace rpyb {
 namespace {
 
 constexpr int64_t kChainSmem = 226 * 1024;
-constexpr int kChainThreads = 512;   // most threads a block
+constexpr int kChainThreads = 1024;   // most threads a block
 
 struct ChainArgs {
     int64_t T = 0;
@@ -116,7 +116,7 @@ __device__ __forceinline__ void project_log(const ChainArgs& a, const double* xs
 }
 
 template <typename TS, int D>
-__global__ void __launch_bounds__(kChainThreads, 2)
+__global__ void __launch_bounds__(kChainThreads, 1)
 chain_products_kernel(const ChainArgs a)
 {
     constexpr int F = chain_first<D>();
@@ -394,14 +394,8 @@ static void set_projection(ChainArgs& a, const LieMapsDev& maps, double* lie, in
 static int run_chain(int src_mode, const Geometry& g, const ChainArgs& a, cudaStream_t s)
 {
     const size_t smem = (size_t)chain_words(g.size(), g.db[g.depth]) * 8;
-    // threads: one per top-level unit up to what gives an SM 1024 threads over
-    // the blocks its shared memory holds
     const int F = g.width == 2 ? 3 : g.width == 3 ? 2 : 1;
-    const int64_t units = g.depth >= F ? g.pw[g.depth - F] : g.pw[g.depth];
-    const int64_t per_sm = std::max<int64_t>(1, std::min<int64_t>(16, kChainSmem / (int64_t)(smem + 1024)));
-    int64_t threads = std::min<int64_t>({(units + 31) / 32 * 32,
-                                         std::max<int64_t>(64, 1024 / per_sm / 32 * 32), kChainThreads});
-    threads = std::max<int64_t>(threads, 32);
+    const int64_t threads = row_block_threads(g, g.depth, F, smem, kChainSmem, a.n, kChainThreads);
     const unsigned grid = (unsigned)std::min<int64_t>(a.n, 1 << 20);
     ChainFn fn = src_mode == RPYB_F64 ? chain_fn<double>(g.width) : chain_fn<float>(g.width);
     if (int rc = allow_shared_memory(fn, smem, kChainSmem)) return rc;

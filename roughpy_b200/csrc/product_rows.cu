@@ -383,16 +383,6 @@ RowArgs row_args(const Geometry& g, int top, const ProductRows& rows)
     return a;
 }
 
-// threads a block: one per unit up to what gives an SM 1024 threads over the
-// blocks its shared memory holds
-int64_t row_threads(int64_t units, size_t smem)
-{
-    const int64_t per_sm = std::max<int64_t>(1, std::min<int64_t>(16, kRowSmem / (int64_t)(smem + 1024)));
-    const int64_t t = std::min<int64_t>({(units + 31) / 32 * 32,
-                                         std::max<int64_t>(64, 1024 / per_sm / 32 * 32), kRowThreads});
-    return std::max<int64_t>(t, 32);
-}
-
 // whether the spec is the whole truncated product of whole rows
 bool whole_product(const ProductSpec& spec, const ProductRows& rows)
 {
@@ -428,12 +418,18 @@ int launch_product_rows(int dtype, const Geometry& g, const ProductSpec& spec,
     const int F = g.width == 2 ? 3 : g.width == 3 ? 2 : 1;
     const size_t smem = (size_t)(2 * stage_room((int)g.db[a.top]) * 8);
     const int64_t units = a.top >= F ? g.pw[a.top - F] : g.pw[a.top];
-    const int64_t threads = row_threads(units, smem);
+    int64_t threads = row_block_threads(g, a.top, F, smem, kRowSmem, rows.batch, kRowThreads);
     // fewer rows than SMs: blocks share a row's top level (not in place, where
     // one block would write lower levels that another still has to stage)
     int64_t slices = 1;
-    if (!in_place && rows.batch < 148)
-        slices = std::max<int64_t>(1, std::min<int64_t>({16, 296 / rows.batch, units / (2 * threads)}));
+    if (!in_place && rows.batch < 148) {
+        // (every block stages the lower levels: with enough threads to have
+        // them all in flight at once)
+        const int64_t least = std::max<int64_t>(128, g.db[a.top] / 8);
+        slices = std::max<int64_t>(1, std::min<int64_t>({16, 148 / rows.batch, units / least}));
+        if (slices > 1)
+            threads = std::min<int64_t>(threads, (units + 32 * slices - 1) / (32 * slices) * 32);
+    }
     const dim3 grid((unsigned)slices, (unsigned)std::min<int64_t>(rows.batch, 65535), 1);
     if (int rc = allow_shared_memory(fn, smem, kRowSmemMost)) return rc;
     fn<<<grid, (unsigned)threads, smem, stream>>>(a);
@@ -460,7 +456,7 @@ int launch_product_slabs(int dtype, const Geometry& g, const ProductSpec& spec,
     else
         fn = spec.accumulate ? slab_fn<float, float, true>(g.width) : slab_fn<float, float, false>(g.width);
     const size_t smem = (size_t)(2 * stage_room((int)g.db[a.top - 1]) * 8);
-    const int64_t threads = row_threads(g.pw[a.top - 2], smem);
+    const int64_t threads = row_block_threads(g, a.top - 1, 1, smem, kRowSmem, rows.batch * g.width, kRowThreads);
     if (int rc = allow_shared_memory(fn, smem, kRowSmemMost)) return rc;
     const dim3 grid((unsigned)g.width, (unsigned)std::min<int64_t>(rows.batch, 65535), 1);
     // the top level first: in place, the lower levels it reads are still the old ones

@@ -2,6 +2,7 @@
 // shared by the series, row-resident product and chain kernels.
 #pragma once
 
+#include <algorithm>
 #include <type_traits>
 
 #include "common.cuh"
@@ -103,6 +104,27 @@ __device__ __forceinline__ void with_level(int k, Fn&& f)
         if (k == KMAX) f(std::integral_constant<int, KMAX>{});
         else with_level<F, KMAX - 1>(k, f);
     }
+}
+
+// Threads of a block that has a whole row of top level `top` to itself, its
+// units owning the first F letters.  An SM gets 1024 threads over the blocks it
+// will hold: those that fit in its shared memory (`room` bytes) or, with fewer
+// rows, its share of them.  A block has no use for more than one thread a unit
+// of the top level, or of all levels where SMs are not full anyway.  (Counting
+// only the blocks that fit left SMs idle below a dozen rows each: (5,5) float32
+// x 148 accumulating took 15.1 us with 64 threads a row, 4.9 with 544.)
+inline int64_t row_block_threads(const Geometry& g, int top, int F, size_t smem, int64_t room,
+                                 int64_t rows, int64_t most)
+{
+    const int64_t resident =
+        std::max<int64_t>(1, std::min<int64_t>({16, room / (int64_t)(smem + 1024), (rows + 147) / 148}));
+    int64_t units = resident < 16 && F > 1 ? 32 : 0;   // the short levels' task
+    for (int k = resident < 16 ? F : std::max(F, top); k <= top; ++k)
+        units += (g.pw[k - F] + 31) / 32 * 32;
+    // whole warps; eleven or twelve blocks of two warps are fewer than ten of three
+    int64_t share = std::max<int64_t>(64, 1024 / resident / 32 * 32);
+    if (share == 64 && 1024 / resident >= 85) share = 96;
+    return std::max<int64_t>(32, std::min<int64_t>({units, share, most}));
 }
 
 // Room for n words staged by stage_words, in float64 words (16-byte multiple).

@@ -36,6 +36,7 @@ namespace {
 
 // dynamic shared memory a block may take (227 KB less the static part)
 constexpr int64_t kSeriesSmem = 226 * 1024;
+constexpr int kSeriesThreads = 1024;   // most threads a block
 
 struct SeriesArgs {
     int width, top, arg_max;
@@ -66,7 +67,7 @@ constexpr int series_max_top()
 // highest level first (the levels shorter than the owned letters are the last
 // task), so that a step's critical path is a few units whatever the depth.
 template <typename T, SeriesKind KIND, int D, int F>
-__global__ void __launch_bounds__(512, 2)
+__global__ void __launch_bounds__(kSeriesThreads, 1)
 series_kernel(const SeriesArgs a)
 {
     constexpr int DD = D > 0 ? D : 1;
@@ -324,12 +325,8 @@ int launch_series(int dtype, SeriesKind kind, const Geometry& g, int top, int ar
     SeriesFn fn = dtype == RPYB_F64 ? series_fn<double>(kind, g.width)
                                     : series_fn<float>(kind, g.width);
     const size_t smem = (size_t)(3 * g.db[top] * 8);
-    // threads: one per top-level unit up to what gives an SM about 1024
-    // threads over the blocks its shared memory holds (small rows: one warp)
     const int64_t units = top >= first ? g.pw[top - first] : g.pw[top];
-    const int64_t per_sm = std::max<int64_t>(1, std::min<int64_t>(16, kSeriesSmem / (int64_t)(smem + 1024)));
-    int64_t threads = std::min<int64_t>({(units + 31) / 32 * 32, std::max<int64_t>(64, 1024 / per_sm / 32 * 32), 512});
-    threads = std::max<int64_t>(threads, 32);
+    const int64_t threads = row_block_threads(g, top, first, smem, kSeriesSmem, rows.batch, kSeriesThreads);
     // fewer rows than SMs: blocks of one row share its top level (each
     // computes the lower levels for itself).  Not for a log whose incoming
     // out[0] every block would have to read before one of them writes it.
