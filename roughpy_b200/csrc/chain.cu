@@ -170,13 +170,6 @@ chain_products_kernel(const ChainArgs a)
             }
             continue;
         }
-        __syncthreads();   // the previous row's reads of the buffers are done
-        double* const xs = stage_words(row_room, src + a.rows[o0] * a.T, T, tid, B);
-        double* top = xs + TL;
-        double* cur = xs;          // lower levels of the running product
-        double* nxt = low_room;
-        double* fx = nullptr;      // lower levels of the factor
-        if (o0 + 1 < o1) fx = stage_words(x_room[0], src + a.rows[o0 + 1] * a.T, TL, tid, B);
         // factors' top levels start towards L2 three products ahead
         auto prefetch_top = [&](int64_t r) {
             if (r >= o1) return;
@@ -186,12 +179,33 @@ chain_products_kernel(const ChainArgs a)
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(p + l));
         };
         for (int64_t r = o0 + 1; r < o0 + 4; ++r) prefetch_top(r);
+        __syncthreads();   // the previous row's reads of the buffers are done
+        double* const xs = stage_words(row_room, src + a.rows[o0] * a.T, T, tid, B);
+        double* top = xs + TL;
+        double* cur = xs;          // lower levels of the running product
+        double* nxt = low_room;
+        double* fx = nullptr;      // lower levels of the factor
+        if (o0 + 1 < o1) fx = stage_words(x_room[0], src + a.rows[o0 + 1] * a.T, TL, tid, B);
         for (int64_t r = o0 + 1; r < o1; ++r) {
             asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();
             const double* X = fx;
-            if (r + 1 < o1)
-                fx = stage_words(x_room[(r - o0) & 1], src + a.rows[r + 1] * a.T, TL, tid, B);
+            // the next factor's lower levels: float64 by asynchronous copies;
+            // float32, which has to be widened, its first words through
+            // registers across this product, so that it does not begin with
+            // their latency ((8,3), 16 queries of 1024 events with their host
+            // time 28 -> 24 us; two words a thread, more would spill)
+            const TS* ahead = r + 1 < o1 ? src + a.rows[r + 1] * a.T : nullptr;
+            double* const ahead_room = x_room[(r - o0) & 1];
+            constexpr int kHeld = sizeof(TS) == 4 ? 2 : 0;
+            TS held[kHeld + 1];
+            if constexpr (kHeld == 0) {
+                if (ahead) fx = stage_words(ahead_room, ahead, TL, tid, B);
+            } else {
+#pragma unroll
+                for (int j = 0; j < kHeld; ++j)
+                    held[j] = ahead && tid + j * B < TL ? __ldg(ahead + tid + j * B) : TS(0);
+            }
             prefetch_top(r + 3);
             const TS* node = src + a.rows[r] * a.T;
             const double node0 = X[0], c0v = cur[0];
@@ -239,6 +253,16 @@ chain_products_kernel(const ChainArgs a)
                     }
             });
             if (tid == 0) nxt[0] = c0v * node0;
+            if constexpr (kHeld > 0) {
+                if (ahead) {
+#pragma unroll
+                    for (int j = 0; j < kHeld; ++j)
+                        if (tid + j * B < TL) ahead_room[tid + j * B] = (double)held[j];
+                    if (kHeld * B < TL)
+                        stage_words(ahead_room + kHeld * B, ahead + kHeld * B, TL - kHeld * B, tid, B);
+                    fx = ahead_room;
+                }
+            }
             double* t = cur;
             cur = nxt;
             nxt = t;
