@@ -18,7 +18,7 @@
 //
 // A query [a, b) is trimmed to the support (streams/src/stream.cpp:37-71),
 // dissected into maximal dyadic pieces on the host, or on the device for
-// batches of 256 and more (intervals/src/dyadic_interval.cpp:191-224), each piece is mapped to a tree
+// large batches (intervals/src/dyadic_interval.cpp:191-224), each piece is mapped to a tree
 // node, and every query's node signatures are multiplied in order on the
 // device in float64 (float32 nodes enter through the mixed-precision
 // product).  log, then the tensor->Lie map, give the log-signature
@@ -904,9 +904,12 @@ RPYB_API int rpyb_dyadic_query(const rpyb_dyadic_tree* t, int64_t n_queries,
     // Many queries whose shape has the fused kernel are dissected on the device:
     // on the host it takes 0.09 to 0.14 us a query, which was most of the time of
     // 100000 queries at (3,4) (9.35 -> 0.75 ms) and the last millisecond of it at
-    // (6,5) (14.0 -> 13.0 ms); few are as fast here, without the extra launch.
+    // (6,5) (14.0 -> 13.0 ms).  Few are faster here, without the upload and launch
+    // before the products can start.  Host / device on B200: 256 at (3,4) 40 / 49
+    // us, 600 48 / 52; at (6,5) float32 106 / 113 and 173 / 179; with the range
+    // table, whose products are short, (3,4) 256 28 / 26, 512 42 / 30.
     int max_tol = 0;
-    if (n_queries >= 256 && chain_lie_available(g, *t->maps) &&
+    if (n_queries >= (t->tb >= 0 ? 400 : 600) && chain_lie_available(g, *t->maps) &&
         device_dissection(t, n_queries, inf_host, sup_host, resolution, &max_tol))
         return query_on_device(t, n_queries, inf_host, sup_host, resolution, max_tol, out_logsig,
                                ld_logsig, out_sig, ld_sig, s);
