@@ -961,6 +961,30 @@ static bool blocked_accumulates_faster(int dtype, const Geometry& g, const Produ
     return staged > (dtype == RPYB_F32 ? 128 : 72) * 1024;
 }
 
+// Shapes and batches whose rows are better left to the kernels below.
+static bool rows_slower(int dtype, const Geometry& g, const ProductSpec& spec, int64_t batch)
+{
+    if (blocked_accumulates_faster(dtype, g, spec)) return true;
+    const int64_t lower = g.db[spec.khi];   // words a factor has staged
+    // Widths above 8 run with a runtime width, several times the instructions
+    // of a split, and short rows pay where that hides behind memory: rows /
+    // others on B200, (12,3) float32 accumulating x 296 12.6 / 10.4 us, x 600
+    // 16.6 / 19.2.  Longer ones pay earlier, (12,4) float64 x 8 18.5 / 19.5, x
+    // 148 39 / 55, and the longest where an SM has one, (16,4) float32 x 100
+    // 82 / 71, x 148 105 / 138.
+    if (g.width > 8) {
+        if (lower < 800) return batch < (dtype == RPYB_F32 ? 592 : 444);
+        return batch < (lower <= 2000 ? 1 : spec.accumulate ? 148 : 32);
+    }
+    // Staging the lower levels of a few very long rows takes longer than tiles
+    // over many SMs: (2,13) float64 x 8 14.4 / 11.9 us, x 64 14.7 / 16.4; (6,6)
+    // assigning x 8 11.3 / 6.7, x 64 16.0 / 21.2.
+    if (batch < 64 && 2 * lower * 8 > 120 * 1024) return true;
+    // (4,6) float64 accumulating, from eight rows an SM on: x 2000 72.2 / 67.6 us.
+    return dtype == RPYB_F64 && spec.accumulate && g.width == 4 && batch >= 8 * 148 &&
+           lower > 1024 && lower < 4096;
+}
+
 // Where the slab kernel beats the kernels below.  Measured on B200, slabs /
 // others: widths 5 and 7, which have no two-letter blocks, (5,7) x 500 float64
 // 299 / 333 us accumulating and 229 / 319 assigning, (7,6) float32 x 600 308 /
@@ -968,15 +992,17 @@ static bool blocked_accumulates_faster(int dtype, const Geometry& g, const Produ
 // assigning float64, (4,8) x 500 219 / 239 us.  Not: (8,6) float64 904 / 835 us
 // accumulating, (4,8) float32 407 / 351 us, accumulating float64 266 / 252 us.
 // A row is only `width` blocks, so few rows leave SMs idle: (8,6) float32 x 10
-// 37 / 18 us.
+// 37 / 18 us, x 64 91 / 80, (5,7) float32 accumulating x 100 65 / 50, x 200
+// 101 / 91, the same from 444 on.
 static bool slabs_faster(int dtype, const Geometry& g, const ProductSpec& spec, int64_t batch)
 {
-    if (batch < 64) return false;
+    const bool f32 = dtype == RPYB_F32;
+    if (batch < (f32 && g.width != 7 ? 148 : 64)) return false;
     switch (g.width) {
         case 4: return dtype == RPYB_F64 && !spec.accumulate;
-        case 5:
+        case 5: return !f32 || !spec.accumulate || batch >= 444;
         case 7: return true;
-        case 8: return dtype == RPYB_F32;
+        case 8: return f32;
         default: return false;
     }
 }
@@ -986,7 +1012,7 @@ int launch_product(int dtype, const Geometry& g, const ProductSpec& spec,
 {
     if (rows.batch <= 0) return RPYB_OK;
     if (product_rows_enabled(dtype) && product_rows_available(g, spec, rows) &&
-        !blocked_accumulates_faster(dtype, g, spec))
+        !rows_slower(dtype, g, spec, rows.batch))
         return launch_product_rows(dtype, g, spec, rows, false, stream);
     if (product_rows_enabled(dtype) && product_slabs_available(g, spec, rows) &&
         slabs_faster(dtype, g, spec, rows.batch))

@@ -388,8 +388,8 @@ RPYB_API int rpyb_ft_inplace_mul(int dtype, int32_t width, int32_t depth, int64_
     rows.ld_rhs = ld_rhs;
     rows.batch = batch;
     // In place where one block has a whole row: three passes over the rows
-    // instead of five (a row in slabs is a few blocks: not for a few rows).  Rows of the two operands may be the same, but no row
-    // of one may reach into another row of the other.
+    // instead of five.  Rows of the two operands may be the same, but no row of
+    // one may reach into another row of the other.
     const char* l0 = static_cast<const char*>(lhs);
     const char* r0 = static_cast<const char*>(rhs);
     const int64_t l_bytes = ((batch - 1) * ld_lhs + T) * (int64_t)es;
@@ -397,8 +397,14 @@ RPYB_API int rpyb_ft_inplace_mul(int dtype, int32_t width, int32_t depth, int64_
     const bool apart = r0 >= l0 + l_bytes || l0 >= r0 + r_bytes;
     const bool same = l0 == r0 && (ld_lhs == ld_rhs || batch == 1);
     const bool whole = product_rows_available(g, sp, rows);
-    if ((apart || same) && product_rows_enabled(dtype) &&
-        (whole || (batch >= 64 && product_slabs_available(g, sp, rows)))) {
+    // A few long rows are a few blocks, a row to an SM (or its slabs): tiles over
+    // many SMs and a copy are faster.  Measured on B200, in place / copied: (6,6)
+    // float64 x 8 23.4 / 12.0 us, x 32 23.8 / 27.5; (8,5) float32 x 8 12.6 / 9.8;
+    // (16,4) float64 x 32 70 / 51.  Not with seven letters, (7,5) x 8 10.3 / 16.2.
+    const int64_t few = !whole ? 64 : g.width > 8 ? (T > 16384 ? 64 : 8)
+                        : T > 16384 && g.width != 7 ? 32 : 1;
+    if ((apart || same) && product_rows_enabled(dtype) && batch >= few &&
+        (whole || product_slabs_available(g, sp, rows))) {
         rows.out = lhs;
         rows.ld_out = ld_lhs;
         return whole ? launch_product_rows(dtype, g, sp, rows, true, s)
