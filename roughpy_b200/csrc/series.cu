@@ -300,6 +300,17 @@ bool series_available(const Geometry& g, int top)
     return g.width >= 2 && g.width <= 16 && top >= 1 && 3 * g.db[top] * 8 <= kSeriesSmem;
 }
 
+// The longest rows that the runtime width takes, (13..16, 4), where a few of
+// them leave most SMs idle: (16,4) float64, row-resident / launches on B200, log
+// x 8 72 / 35 us, x 64 76 / 70, fmexp x 8 63 / 46, x 64 87 / 134; log of float32 x
+// 32 66 / 78.  Float32 exp and fmexp stay: a launch a step rounds every step to
+// float32.
+bool series_slower(int dtype, SeriesKind kind, const Geometry& g, int top, int64_t batch)
+{
+    if (dtype == RPYB_F32 && kind != kSeriesLog) return false;
+    return g.width > 12 && g.db[top] > 2000 && batch < (dtype == RPYB_F64 && kind == kSeriesLog ? 64 : 32);
+}
+
 int launch_series(int dtype, SeriesKind kind, const Geometry& g, int top, int arg_max,
                   const SeriesRows& rows, cudaStream_t stream)
 {

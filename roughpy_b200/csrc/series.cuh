@@ -20,6 +20,9 @@ struct SeriesRows {
 // Whether series of `top` levels of this shape run in the row-resident kernel.
 bool series_available(const Geometry& g, int top);
 
+// Whether one product launch a step is faster there for this batch.
+bool series_slower(int dtype, SeriesKind kind, const Geometry& g, int top, int64_t batch);
+
 // out <- exp(arg), mult exp(arg) or log(arg), truncated at level `top` (>= 1);
 // levels of arg above arg_max count as zero (log).  The level-0 rules are
 // those of the product-launch drivers: exp writes 1, fmexp the multiplier's

@@ -539,7 +539,7 @@ RPYB_API int rpyb_ft_exp(int dtype, int32_t width, int32_t depth, int64_t batch,
     if (M > 1 &&
         (rc = scratch.get((size_t)(batch * g.size()) * elem_size(dtype), &tmp)))
         return rc;
-    if (series_available(g, M)) {
+    if (series_available(g, M) && !series_slower(dtype, kSeriesExp, g, M, batch)) {
         SeriesRows r;
         r.out = out;
         r.ld_out = ld_out;
@@ -578,7 +578,7 @@ RPYB_API int rpyb_ft_fmexp(int dtype, int32_t width, int32_t depth, int64_t batc
     Scratch scratch(workspace, workspace_bytes, s);
     void* tmp = nullptr;
     if (M > 1 && (rc = scratch.get((size_t)(batch * g.size()) * es, &tmp))) return rc;
-    if (series_available(g, M)) {
+    if (series_available(g, M) && !series_slower(dtype, kSeriesFmexp, g, M, batch)) {
         SeriesRows r;
         r.out = out;
         r.ld_out = ld_out;
@@ -617,7 +617,7 @@ static int log_series(int dtype, int32_t width, int32_t depth, int64_t batch, vo
     void* base = nullptr;
     const int nbuf = (dtype == RPYB_F64) ? 1 : 3;
     if ((rc = scratch.get((size_t)(nbuf * batch * T) * 8, &base))) return rc;
-    if (M >= 1 && series_available(g, M)) {
+    if (M >= 1 && series_available(g, M) && !series_slower(dtype, kSeriesLog, g, M, batch)) {
         SeriesRows r;
         r.out = out;
         r.ld_out = ld_out;
