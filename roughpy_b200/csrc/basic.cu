@@ -75,6 +75,9 @@ struct Letters<D, 0> {
 };
 
 constexpr int kAntipodeThreads = 256;
+// Words of a batch from which its upper levels go through tiles, a launch of
+// their own: below, that costs more than gathering (in 32-bit arithmetic) does.
+constexpr int64_t kAntipodeTiled = int64_t(1) << 19;
 
 // levels 2 L and above: one tile a block
 template <typename T, int D, int L>
@@ -348,7 +351,7 @@ RPYB_API int rpyb_ft_antipode(int dtype, int32_t width, int32_t depth, int64_t b
         const V* x = static_cast<const V*>(arg);
         int64_t words = g.size();
         if constexpr (L > 0) {
-            if (depth >= 2 * L) {
+            if (depth >= 2 * L && batch * words >= kAntipodeTiled) {
                 words = g.db[2 * L];
                 const int64_t tiles = g.db[depth - 2 * L + 1];   // sum of d^(k - 2 L)
                 const unsigned blocks = (unsigned)std::min<int64_t>(batch * tiles, 148 * 4096);
