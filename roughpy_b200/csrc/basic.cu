@@ -125,7 +125,8 @@ antipode_tiles_kernel(T* out, const T* arg, int64_t ld_out, int64_t ld_arg, int6
 // broadcasts or runs and arg as runs, and add their slices by a tree.  Sums
 // are float64 for both element types.
 //
-// Three forms.  Rows of at most 1024 words are a warp's, all tiles in turn
+// Four forms.  Rows of at most 64 words in large batches are a thread's a
+// word.  Rows of at most 1024 words are a warp's, all tiles in turn
 // (one tile a warp where there are few rows).  Longer rows that fit in shared
 // memory are a block's: staged once, read once per level.  Others take a block
 // per tile and re-read the row from L2.  The layout before, one thread per
@@ -207,6 +208,35 @@ __device__ __forceinline__ void adjoint_tile(const AdjointArgs& a, T* __restrict
         T* o = out + a.db[k] + i;
         if (!a.accumulate) *o = (T)sum;
         else if (E > 0) *o = (T)((double)*o + sum);
+    }
+}
+
+// Rows of at most 64 words in batches that fill the GPU: a thread per output
+// word, its terms in turn.  A warp a row would spend a tile, with most lanes
+// idle, on each level: (2,2) float64 x 30000 28.7 -> 3.6 us, (3,3) x 100000 119
+// -> 78, (2,5) x 100000 187 -> 134.
+constexpr int64_t kAdjointWords = 64;
+
+template <typename T>
+__global__ void __launch_bounds__(256)
+adjoint_words_kernel(T* out, const T* op, const T* arg, const AdjointArgs a)
+{
+    const uint32_t size = (uint32_t)a.db[a.out_max + 1];
+    const uint32_t total = (uint32_t)a.batch * size;
+    for (uint32_t g = blockIdx.x * 256u + threadIdx.x; g < total; g += gridDim.x * 256u) {
+        const uint32_t b = g / size, w = g - b * size;
+        int k = 0;
+        while (w >= (uint32_t)a.db[k + 1]) ++k;
+        const int E = (int)a.E[k], n = (int)a.pw[k];
+        const T* o = op + b * a.ld_op;
+        const T* x = arg + b * a.ld_arg + w;   // word w - db[k] of level k, and on
+        double sum = 0.0;
+#pragma unroll 4
+        for (int e = 0; e < E; ++e)
+            sum = fma((double)__ldg(o + e), (double)__ldg(x + e * n), sum);
+        T* y = out + b * a.ld_out + w;
+        if (!a.accumulate) *y = (T)sum;
+        else if (E > 0) *y = (T)((double)*y + sum);
     }
 }
 
@@ -426,6 +456,9 @@ static int adjoint_left_mul(int dtype, int32_t width, int32_t depth, int64_t bat
     // Staged rows leave room for two blocks an SM; one block of a few long
     // rows would leave the chip idle, so there the tiles are spread over it.
     const int64_t T = g.db[out_max + 1];
+    // (and the shortest rows at any batch)
+    const bool words = T <= kAdjointWords && (batch >= 148 * 8 || T <= 8) &&
+                       batch * T < (int64_t(1) << 31);
     const bool warp = T <= 1024;
     const bool stage = !warp && staged <= kAdjointSmem && batch >= 64;
     // columns of a tile: the threads of the kernel that is launched below
@@ -443,6 +476,7 @@ static int adjoint_left_mul(int dtype, int32_t width, int32_t depth, int64_t bat
     int64_t blocks = batch * (a.heavy + (tiles - a.heavy + kAdjointGroup - 1) / kAdjointGroup);
     if (warp) blocks = std::min<int64_t>((batch * (tiles / a.tiles_per_task) + 7) / 8, 148 * 64);
     else if (stage) blocks = std::min<int64_t>(batch, 1 << 20);
+    if (words) blocks = grid_for(batch * T, 256);
     if (blocks > 0x7fffffff) return fail(RPYB_E_UNSUPPORTED, "batch too large");
     auto go = [&](auto kind) -> int {
         using V = decltype(kind);
@@ -450,7 +484,9 @@ static int adjoint_left_mul(int dtype, int32_t width, int32_t depth, int64_t bat
         const V* p = static_cast<const V*>(op);
         const V* x = static_cast<const V*>(arg);
         const unsigned nb = (unsigned)blocks;
-        if (warp) {
+        if (words) {
+            adjoint_words_kernel<V><<<nb, 256, 0, s>>>(o, p, x, a);
+        } else if (warp) {
             adjoint_warp_kernel<V><<<nb, 256, 0, s>>>(o, p, x, a);
         } else if (stage) {
             auto fn = adjoint_block_kernel<V, 256, true>;
