@@ -306,14 +306,21 @@ struct LaneLayout {
     static constexpr int64_t fold_words = P >= 2 ? ipow_c(D, P - 1) : 1;
     static constexpr int64_t NF2 =
         fold_words <= 32 ? 1 : (fold_words > 96 && NT / 32 % 4 == 3 ? 4 : 3);
-    // With no shared ancestors (depth 3 and less) one warp sums the gradient, in
-    // one stage: (8,3) x 512 of 300 takes 0.34 ms, 0.59 in two stages and 1.06
-    // with four warps; (3,3) x 2000 of 100 0.238, 0.246 and 0.228.  Where many
-    // blocks fit either way the last wave decides: (2,3) x 4000 of 100 is 0.35 ms
-    // (0.30 with four).
+    // Two warps in one stage where a second stage has little to overlap: one
+    // shared level (depth 4, from width 3 on) or, in float32 at width 2, two.
+    // Two stages / one of two warps / four warps: (3,4) float64 x 148 of 100
+    // 84 / 73 / 74 us, (7,4) x 148 145 / 136 / 136 and x 2000 0.97 / 0.94 / 1.59 ms,
+    // (2,5) float32 x 2000 0.31 / 0.27 / 0.29 ms.
+    static constexpr bool FEW =
+        P >= 2 && (D == 2 ? sizeof(T) == 4 && P <= 3 : P == 2);
+    // With no shared ancestors (depth 3 and less) the fold warps only sum the
+    // gradient, in one stage.  One is enough beside many lanes, where it leaves
+    // room for more blocks ((8,2) float64 x 512 of 100: 0.12 ms with one, 0.17
+    // with two, 0.32 with four); few lanes wait for it: (3,3) x 1000 0.134 / 0.122 /
+    // 0.124 ms, (2,3) x 2000 0.208 / 0.200 / 0.183.
     static constexpr bool TWO =
-        P >= 2 && !(sizeof(T) == 8 && NT > 512) && fold_words <= 64 * NF2;
-    static constexpr int64_t NF = TWO ? NF2 : (P < 2 ? 1 : 4);
+        P >= 2 && !FEW && !(sizeof(T) == 8 && NT > 512) && fold_words <= 64 * NF2;
+    static constexpr int64_t NF = TWO ? NF2 : FEW ? 2 : P >= 2 || D == 2 ? 4 : D <= 4 ? 2 : 1;
     static constexpr int64_t NTB = NT + 32 * NF + (TWO ? 32 : 0);
     static_assert(NTB <= 1024, "threads of a block");
     static constexpr int MINB = NT == 128 ? 2 : 1;       // blocks an SM the registers are held to
