@@ -903,6 +903,9 @@ struct LaneEntry {
     void (*fn)(BwdArgs) = nullptr;
     int64_t smem = 0;
     int threads = 0;
+    // blocks of four fold warps in one stage, which the slots are counted by
+    // where memory bounds them, and of one warp more (lane_slots)
+    int usual_threads = 0;
     int least_threads = 0;
     int64_t lanes = 0;
     int ckw = 0;
@@ -917,6 +920,7 @@ bool lane_fill(LaneEntry& e)
             e.fn = &signature_backward_lanes<T, D, N>;
             e.smem = LY::bytes;
             e.threads = (int)LY::NTB;
+            e.usual_threads = (int)(LY::NT + 32 * std::min<int64_t>(4, (1024 - LY::NT) / 32));
             e.least_threads = (int)LY::NT + 160;
             e.lanes = LY::W;
             e.ckw = LY::PP + D;
@@ -970,37 +974,36 @@ int64_t lane_slot_bytes(const LaneEntry& e, int64_t max_segments)
     return (max_segments * e.ckw * e.lanes * 8 + 255) / 256 * 256;
 }
 
-// Blocks in flight for the lane kernel (one workspace slot each): as many as
-// fit, or, with `least`, as many as fit of blocks of least_threads, which is
-// the count that a caller's workspace has to hold.
-int64_t lane_slots(const LaneEntry& e, int64_t n_streams, bool least)
+// Blocks in flight for the lane kernel (one workspace slot each), by the
+// threads a block is counted with: as many as fit with the kernel's own; with
+// least_threads the count that a caller's workspace has to hold, which is no
+// more than what blocks of usual_threads and a few more registers come to, so
+// that workspaces sized for those stay large enough.
+int64_t lane_slots(const LaneEntry& e, int64_t n_streams, int threads)
 {
     int dev = 0, sms = 148, occ = 1;
     if (cudaGetDevice(&dev) == cudaSuccess) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (cudaFuncSetAttribute(e.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)e.smem) == cudaSuccess)
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                &occ, e.fn, least ? e.least_threads : e.threads, (size_t)e.smem);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, e.fn, threads, (size_t)e.smem);
         cudaGetLastError();
     }
     return std::min<int64_t>(std::max<int64_t>(1, n_streams), (int64_t)sms * std::max(occ, 1));
 }
 
-// The slots beyond the least are taken while the checkpoints of all of them
-// stay within this (they are 24 MB for 512 streams of 1024 steps at width 8,
-// depth 4; streams of a million steps would take 23 GB).
+// All slots that fit are taken while their checkpoints stay within this (they
+// are 24 MB for 512 streams of 1024 steps at width 8, depth 4), beyond it those
+// of usual_threads (streams of a million steps would take 23 GB).
 constexpr int64_t kLaneScratch = (int64_t)256 << 20;
 
 int64_t lane_workspace(const LaneEntry& e, int64_t n_streams, int64_t segments, bool least)
 {
     const int64_t slot = lane_slot_bytes(e, segments);
-    const int64_t few = lane_slots(e, n_streams, true);
-    if (!least) {
-        const int64_t all = lane_slots(e, n_streams, false);
-        if (all > few && all * slot <= kLaneScratch) return 256 + all * slot;
-    }
-    return 256 + few * slot;
+    if (least) return 256 + lane_slots(e, n_streams, e.least_threads) * slot;
+    const int64_t all = lane_slots(e, n_streams, e.threads);
+    if (all * slot <= kLaneScratch) return 256 + all * slot;
+    return 256 + std::min(all, lane_slots(e, n_streams, e.usual_threads)) * slot;
 }
 
 template <typename T>
@@ -1183,7 +1186,7 @@ RPYB_API int rpyb_signature_backward(int mode, int32_t width, int32_t depth, int
     RPYB_CUDA(cudaMemsetAsync(ws, 0, sizeof(int), s));
     if (lanes) {
         a.slot_bytes = lane_slot_bytes(e, a.max_segments);
-        const int64_t slots = std::min<int64_t>(lane_slots(e, n_streams, false),
+        const int64_t slots = std::min<int64_t>(lane_slots(e, n_streams, e.threads),
                                                 (need - 256) / std::max<int64_t>(a.slot_bytes, 1));
         e.fn<<<(unsigned)slots, e.threads, (size_t)e.smem, s>>>(a);
         RPYB_CUDA(cudaGetLastError());
