@@ -71,15 +71,16 @@ struct SigArgs {
     int64_t ld_out;
     const int64_t* order;
     const int64_t* ends;   // (first row, end row) in processing order, or null: a
-                           // lookup that does not wait for order's
+                           // lookup that does not wait for order's (SINGLE only)
     int64_t n_streams;
     int64_t items_per_stream;
     int64_t total_items;
-    // Items come from a device counter (zeroed before the launch), unless the
-    // grid has a warp for each (`single`): then a warp takes the item of its own
-    // number and the counter is neither zeroed nor read.
+    // Items come from a device counter (zeroed before the launch).  Not in the
+    // SINGLE kernels, whose grid has a warp for each: there a warp takes the item
+    // of its own number.  They are kernels of their own because a branch in the
+    // item loop costs the others up to 15 % ((3,5) float32, 4000 streams of 100
+    // steps, 41.0 -> 47.0 us).
     int* queue;
-    bool single;
     int fold;     // fold interval of the classic compensated mode (steps)
     int fold_chunks;  // split kernel: chunks of kChunk steps between folds
     // output rows: row s of `out` unless dst_row is given, in which case
@@ -225,7 +226,7 @@ __device__ __forceinline__ void fold_word(float& hi, float& lo, float& delta)
 // HS (float mode): the hi words of the top level live in shared memory next to
 // their lo words, leaving only the per-step delta accumulators in registers;
 // this lets one lane own more top words (G = D) within the register file.
-template <bool F64, int D, int N, int G, bool HS>
+template <bool F64, int D, int N, int G, bool HS, bool SINGLE>
 __global__ void __launch_bounds__(kSigWarps * 32, 1)
 signature_kernel(const SigArgs a)
 {
@@ -257,9 +258,12 @@ signature_kernel(const SigArgs a)
 
     while (true) {
         int item = 0;
-        if (lane == 0)
-            item = a.single ? (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) : atomicAdd(a.queue, 1);
-        item = __shfl_sync(0xffffffffu, item, 0);
+        if constexpr (SINGLE) {
+            item = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+        } else {
+            if (lane == 0) item = atomicAdd(a.queue, 1);
+            item = __shfl_sync(0xffffffffu, item, 0);
+        }
         if (item >= a.total_items) break;
 
         const int64_t slot = item / a.items_per_stream;
@@ -281,8 +285,14 @@ signature_kernel(const SigArgs a)
             }
         }
 
-        const int64_t start = a.ends ? a.ends[2 * slot] : a.offsets[s];
-        const int64_t len = (a.ends ? a.ends[2 * slot + 1] : a.offsets[s + 1]) - start;
+        int64_t start = a.offsets[s];
+        int64_t len = a.offsets[s + 1] - start;
+        if constexpr (SINGLE) {
+            if (a.ends) {
+                start = a.ends[2 * slot];
+                len = a.ends[2 * slot + 1] - start;
+            }
+        }
         const T* __restrict__ xs = static_cast<const T*>(a.inc) + start * D;
 
         // ---- state
@@ -364,7 +374,16 @@ signature_kernel(const SigArgs a)
 #pragma unroll
                     for (int g = 0; g < G; ++g) mh[g] = fma_t(am, xg[g], mh[g]);
                 };
-                T x[D], xa[G], ax, am, x1[D], xa1[G], ax1, am1;
+                T x[D], xa[G], ax, am;
+                if constexpr (P == 0) {
+                    // no chains to overlap: (8,2) x 4000 of 100, 90 -> 80 us
+                    for (int j = 0; j < nsteps; ++j) {
+                        chains(j, x, xa, ax, am);
+                        products(x, xa, ax, am);
+                    }
+                    continue;
+                }
+                T x1[D], xa1[G], ax1, am1;
                 chains(0, x, xa, ax, am);
                 int j = 0;
 #pragma unroll 1
@@ -550,7 +569,7 @@ signature_kernel(const SigArgs a)
                 }
             }
         }
-        if (a.single) break;
+        if constexpr (SINGLE) break;
     }
 }
 
@@ -620,7 +639,7 @@ __host__ __device__ constexpr int tmem_cols_for(int nwarps) { return nwarps <= 4
 // (FFMA2), while m64 * X[b] is added in float64 when the chunk's deltas are
 // folded (one DFMA per word per chunk).  Per step and lane the FP32 pipe sees
 // G*D + 2G FMAs, every one of them a useful Horner FMA.
-template <int D, int N, int G, bool TM>
+template <int D, int N, int G, bool TM, bool SINGLE>
 __global__ void __maxnreg__(TM ? RPYB_SIG_TMEM_MAXREG : RPYB_SIG_SPLIT_MAXREG)
 signature_kernel_split(const SigArgs a)
 {
@@ -670,9 +689,12 @@ signature_kernel_split(const SigArgs a)
 
     while (true) {
         int item = 0;
-        if (lane == 0)
-            item = a.single ? (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) : atomicAdd(a.queue, 1);
-        item = __shfl_sync(0xffffffffu, item, 0);
+        if constexpr (SINGLE) {
+            item = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+        } else {
+            if (lane == 0) item = atomicAdd(a.queue, 1);
+            item = __shfl_sync(0xffffffffu, item, 0);
+        }
         if (item >= a.total_items) break;
 
         const int64_t slot = item / a.items_per_stream;
@@ -694,8 +716,14 @@ signature_kernel_split(const SigArgs a)
             }
         }
 
-        const int64_t start = a.ends ? a.ends[2 * slot] : a.offsets[s];
-        const int64_t len = (a.ends ? a.ends[2 * slot + 1] : a.offsets[s + 1]) - start;
+        int64_t start = a.offsets[s];
+        int64_t len = a.offsets[s + 1] - start;
+        if constexpr (SINGLE) {
+            if (a.ends) {
+                start = a.ends[2 * slot];
+                len = a.ends[2 * slot + 1] - start;
+            }
+        }
         const float* __restrict__ xs = static_cast<const float*>(a.inc) + start * D;
 
         double ph[PP];
@@ -968,7 +996,7 @@ signature_kernel_split(const SigArgs a)
                 for (int b = 0; b < D; ++b) o[a.db[N] + mw * D + b] = tv[b];
             }
         }
-        if (a.single) break;
+        if constexpr (SINGLE) break;
     }
     if constexpr (TM) {
         tmem_fence_before();
@@ -1037,6 +1065,7 @@ using SigKernel = void (*)(SigArgs);
 
 struct SigVariant {
     SigKernel fn;
+    SigKernel fn_single;    // where the grid has a warp for every item
     int g;
     int64_t lanes;          // W: lanes per stream
     size_t smem_warp;       // dynamic shared memory per warp (bytes)
@@ -1049,7 +1078,8 @@ SigVariant make_variant()
     constexpr int64_t W = IPow<D, N - 2>::value * (D / G);
     constexpr size_t top = F64 ? 0 : (size_t)(HS ? 2 : 1) * G * D * 32 * 4;
     constexpr size_t stage = (size_t)kChunk * D * (F64 ? 8 : 4);
-    return SigVariant{&signature_kernel<F64, D, N, G, HS>, G, W, top + stage};
+    return SigVariant{&signature_kernel<F64, D, N, G, HS, false>,
+                      &signature_kernel<F64, D, N, G, HS, true>, G, W, top + stage};
 }
 
 template <int D, int N, int G, bool TM = false>
@@ -1058,7 +1088,8 @@ SigVariant make_split_variant()
     constexpr int64_t W = IPow<D, N - 2>::value * (D / G);
     constexpr size_t xsum = ((size_t)D * 8 + 15) / 16 * 16;
     constexpr size_t bytes = (size_t)((TM ? 0 : G * D) + G) * 32 * 8 + xsum + (size_t)kChunk * D * 12;
-    return SigVariant{&signature_kernel_split<D, N, G, TM>, G, W, bytes, TM};
+    return SigVariant{&signature_kernel_split<D, N, G, TM, false>,
+                      &signature_kernel_split<D, N, G, TM, true>, G, W, bytes, TM};
 }
 
 // The split kernel's top level in TMEM at width 8 (RPYB_SIG_TMEM=1).  Off by
@@ -1399,12 +1430,14 @@ int launch_signature_variant(const SigVariant& v, const Geometry& g, int64_t n_i
         const auto key = std::make_tuple(dev, (const void*)v.fn, smem_warp, wpb);
         auto it = chosen.find(key);
         if (it == chosen.end()) {
-            RPYB_CUDA(cudaFuncSetAttribute(v.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)(smem_warp * kSigWarps)));
-            // the whole unified L1/shared array as shared memory: the kernels
-            // stage their state there and read global memory once per chunk
-            RPYB_CUDA(cudaFuncSetAttribute(v.fn, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                           (int)cudaSharedmemCarveoutMaxShared));
+            for (const SigKernel fn : {v.fn, v.fn_single}) {
+                RPYB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)(smem_warp * kSigWarps)));
+                // the whole unified L1/shared array as shared memory: the kernels
+                // stage their state there and read global memory once per chunk
+                RPYB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                               (int)cudaSharedmemCarveoutMaxShared));
+            }
             int best_wpb = wpb, best_per_sm = 0;
             if (wpb == 0) {
                 // warps are independent: the block size only matters for
@@ -1453,9 +1486,9 @@ int launch_signature_variant(const SigVariant& v, const Geometry& g, int64_t n_i
     int64_t blocks = (int64_t)per_sm * device_sm_count();
     blocks = std::min<int64_t>(blocks, (a.total_items + wpb - 1) / wpb);
     if (blocks < 1) blocks = 1;
-    a.single = a.total_items <= blocks * wpb;
-    if (!a.single) RPYB_CUDA(cudaMemsetAsync(queue, 0, sizeof(int), s));
-    v.fn<<<(unsigned)blocks, wpb * 32, smem, s>>>(a);
+    const bool single = a.total_items <= blocks * wpb;
+    if (!single) RPYB_CUDA(cudaMemsetAsync(queue, 0, sizeof(int), s));
+    (single ? v.fn_single : v.fn)<<<(unsigned)blocks, wpb * 32, smem, s>>>(a);
     RPYB_CUDA(cudaGetLastError());
     return RPYB_OK;
 }
