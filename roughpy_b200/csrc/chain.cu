@@ -178,7 +178,9 @@ chain_products_kernel(const ChainArgs a)
             for (int64_t l = (int64_t)tid * 128; l < bytes; l += (int64_t)B * 128)
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(p + l));
         };
-        for (int64_t r = o0 + 1; r < o0 + 4; ++r) prefetch_top(r);
+        // (before a float32 row is waited for, after a float64 one's copies start)
+        if (sizeof(TS) == 4)
+            for (int64_t r = o0 + 1; r < o0 + 4; ++r) prefetch_top(r);
         __syncthreads();   // the previous row's reads of the buffers are done
         double* const xs = stage_words(row_room, src + a.rows[o0] * a.T, T, tid, B);
         double* top = xs + TL;
@@ -186,6 +188,8 @@ chain_products_kernel(const ChainArgs a)
         double* nxt = low_room;
         double* fx = nullptr;      // lower levels of the factor
         if (o0 + 1 < o1) fx = stage_words(x_room[0], src + a.rows[o0 + 1] * a.T, TL, tid, B);
+        if (sizeof(TS) == 8)
+            for (int64_t r = o0 + 1; r < o0 + 4; ++r) prefetch_top(r);
         for (int64_t r = o0 + 1; r < o1; ++r) {
             asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();

@@ -285,14 +285,9 @@ signature_kernel(const SigArgs a)
             }
         }
 
-        int64_t start = a.offsets[s];
-        int64_t len = a.offsets[s + 1] - start;
-        if constexpr (SINGLE) {
-            if (a.ends) {
-                start = a.ends[2 * slot];
-                len = a.ends[2 * slot + 1] - start;
-            }
-        }
+        const bool by_ends = SINGLE && a.ends;
+        const int64_t start = by_ends ? a.ends[2 * slot] : a.offsets[s];
+        const int64_t len = (by_ends ? a.ends[2 * slot + 1] : a.offsets[s + 1]) - start;
         const T* __restrict__ xs = static_cast<const T*>(a.inc) + start * D;
 
         // ---- state
@@ -401,127 +396,127 @@ signature_kernel(const SigArgs a)
                     products(x, xa, ax, am);
                 }
             } else {
-            for (int j = 0; j < nsteps; ++j) {
-            const T* row = xbuf + j * D;
-            T x[D];
-            load_row_smem<T, D>(x, row);
-            T xa[G];                               // the lane's letters of level N-1
-            load_slice<T, G>(xa, row + sub * G);
-            T xc[P > 0 ? P : 1];                   // the lane's path letters
+                for (int j = 0; j < nsteps; ++j) {
+                    const T* row = xbuf + j * D;
+                    T x[D];
+                    load_row_smem<T, D>(x, row);
+                    T xa[G];                               // the lane's letters of level N-1
+                    load_slice<T, G>(xa, row + sub * G);
+                    T xc[P > 0 ? P : 1];                   // the lane's path letters
 #pragma unroll
-            for (int i = 0; i < P; ++i) xc[i] = row[c[i]];
+                    for (int i = 0; i < P; ++i) xc[i] = row[c[i]];
 
-            // pre-step values of the path words: hi + delta, hi being kept as the
-            // rounded value of hi + lo
-            T vp[P > 0 ? P : 1];
+                    // pre-step values of the path words: hi + delta, hi being kept as the
+                    // rounded value of hi + lo
+                    T vp[P > 0 ? P : 1];
 #pragma unroll
-            for (int i = 0; i < P; ++i) vp[i] = ph[i] + pd[i];
+                    for (int i = 0; i < P; ++i) vp[i] = ph[i] + pd[i];
 
-            // ---- level N (top): chain through the path, then the mid words
-            {
-                T acc = T(1);
-                if constexpr (P > 0) {
-                    acc = vp[0] + xc[0] * (T(1) / T(N));
+                    // ---- level N (top): chain through the path, then the mid words
+                    {
+                        T acc = T(1);
+                        if constexpr (P > 0) {
+                            acc = vp[0] + xc[0] * (T(1) / T(N));
 #pragma unroll
-                    for (int i = 2; i <= P; ++i)
-                        acc = fma_t(acc, xc[i - 1] * (T(1) / T(N - i + 1)), vp[i - 1]);
-                }
-                const T accx = acc * (T(1) / T(2));
-#pragma unroll
-                for (int g = 0; g < G; ++g) {
-                    // am = S_{N-1} + acc * x/2; the delta joins the product before the
-                    // (large) hi word
-                    const T am = mh[g] + fma_t(accx, xa[g], md[g]);
-                    if constexpr (PACK) {
-                        // packed f32x2 FMAs: two top words per instruction
-                        const float2 am2 = make_float2(am, am);
-#pragma unroll
-                        for (int h = 0; h < D / 2; ++h) {
-                            const float2 r = __ffma2_rn(am2, make_float2(x[2 * h], x[2 * h + 1]),
-                                                        make_float2(td[g][2 * h], td[g][2 * h + 1]));
-                            td[g][2 * h] = r.x;
-                            td[g][2 * h + 1] = r.y;
+                            for (int i = 2; i <= P; ++i)
+                                acc = fma_t(acc, xc[i - 1] * (T(1) / T(N - i + 1)), vp[i - 1]);
                         }
-                    } else {
+                        const T accx = acc * (T(1) / T(2));
 #pragma unroll
-                        for (int b = 0; b < D; ++b) td[g][b] = fma_t(am, x[b], td[g][b]);
-                    }
-                }
-            }
-            // ---- level N-1 (mid words)
-            {
-                T acc = T(1);
-                if constexpr (P > 0) {
-                    acc = vp[0] + xc[0] * (T(1) / T(N - 1));
+                        for (int g = 0; g < G; ++g) {
+                            // am = S_{N-1} + acc * x/2; the delta joins the product before the
+                            // (large) hi word
+                            const T am = mh[g] + fma_t(accx, xa[g], md[g]);
+                            if constexpr (PACK) {
+                                // packed f32x2 FMAs: two top words per instruction
+                                const float2 am2 = make_float2(am, am);
 #pragma unroll
-                    for (int i = 2; i <= P; ++i)
-                        acc = fma_t(acc, xc[i - 1] * (T(1) / T(N - i)), vp[i - 1]);
-                }
-#pragma unroll
-                for (int g = 0; g < G; ++g) md[g] = fma_t(acc, xa[g], md[g]);
-            }
-            // ---- path levels k = P .. 1
-#pragma unroll
-            for (int k = P; k >= 1; --k) {
-                T upd;
-                if (k == 1) {
-                    upd = xc[0];
-                } else {
-                    T acc = vp[0] + xc[0] * (T(1) / T(k));
-#pragma unroll
-                    for (int i = 2; i <= k - 1; ++i)
-                        acc = fma_t(acc, xc[i - 1] * (T(1) / T(k - i + 1)), vp[i - 1]);
-                    upd = acc * xc[k - 1];
-                }
-                pd[k - 1] += upd;
-            }
-
-            if (++since_fold >= a.fold) {
-                    since_fold = 0;
-                    // Fold the deltas into (hi, lo) with an exact two-sum, then
-                    // renormalise (hi, lo) so that hi is the rounded value: the
-                    // chains read hi + delta.
-#pragma unroll
-                    for (int i = 0; i < P; ++i) fold_word(ph[i], pl[i], pd[i]);
-#pragma unroll
-                    for (int g = 0; g < G; ++g) {
-                        fold_word(mh[g], ml[g], md[g]);
-                        if constexpr (PACK) {
-                            // packed fast two-sum (|hi| >= |delta| except while a word is
-                            // still near zero, where the lost error is second order)
-#pragma unroll
-                            for (int h = 0; h < D / 2; ++h) {
-                                float2* hp = hi_top2 + (g * (D / 2) + h) * 32 + lane;
-                                const float2 hi = HS ? *hp : make_float2(th[g][2 * h], th[g][2 * h + 1]);
-                                const float2 dl = make_float2(td[g][2 * h], td[g][2 * h + 1]);
-                                const float2 sm = __fadd2_rn(hi, dl);
-                                const float2 z = __ffma2_rn(hi, make_float2(-1.f, -1.f), sm);
-                                const float2 er = __ffma2_rn(z, make_float2(-1.f, -1.f), dl);
-                                float2* lp = lo_top2 + (g * (D / 2) + h) * 32 + lane;
-                                *lp = __fadd2_rn(*lp, er);
-                                if constexpr (HS) {
-                                    *hp = sm;
-                                } else {
-                                    th[g][2 * h] = sm.x;
-                                    th[g][2 * h + 1] = sm.y;
+                                for (int h = 0; h < D / 2; ++h) {
+                                    const float2 r = __ffma2_rn(am2, make_float2(x[2 * h], x[2 * h + 1]),
+                                                                make_float2(td[g][2 * h], td[g][2 * h + 1]));
+                                    td[g][2 * h] = r.x;
+                                    td[g][2 * h + 1] = r.y;
                                 }
-                                td[g][2 * h] = 0.f;
-                                td[g][2 * h + 1] = 0.f;
-                            }
-                        } else {
+                            } else {
 #pragma unroll
-                            for (int b = 0; b < D; ++b) {
-                                float sh, e;
-                                two_sum(th[g][b], td[g][b], sh, e);
-                                th[g][b] = sh;
-                                float* lp = lo_top + (g * D + b) * 32 + lane;
-                                *lp = __fadd_rn(*lp, e);
-                                td[g][b] = 0.f;
+                                for (int b = 0; b < D; ++b) td[g][b] = fma_t(am, x[b], td[g][b]);
+                            }
+                        }
+                    }
+                    // ---- level N-1 (mid words)
+                    {
+                        T acc = T(1);
+                        if constexpr (P > 0) {
+                            acc = vp[0] + xc[0] * (T(1) / T(N - 1));
+#pragma unroll
+                            for (int i = 2; i <= P; ++i)
+                                acc = fma_t(acc, xc[i - 1] * (T(1) / T(N - i)), vp[i - 1]);
+                        }
+#pragma unroll
+                        for (int g = 0; g < G; ++g) md[g] = fma_t(acc, xa[g], md[g]);
+                    }
+                    // ---- path levels k = P .. 1
+#pragma unroll
+                    for (int k = P; k >= 1; --k) {
+                        T upd;
+                        if (k == 1) {
+                            upd = xc[0];
+                        } else {
+                            T acc = vp[0] + xc[0] * (T(1) / T(k));
+#pragma unroll
+                            for (int i = 2; i <= k - 1; ++i)
+                                acc = fma_t(acc, xc[i - 1] * (T(1) / T(k - i + 1)), vp[i - 1]);
+                            upd = acc * xc[k - 1];
+                        }
+                        pd[k - 1] += upd;
+                    }
+
+                    if (++since_fold >= a.fold) {
+                        since_fold = 0;
+                        // Fold the deltas into (hi, lo) with an exact two-sum, then
+                        // renormalise (hi, lo) so that hi is the rounded value: the
+                        // chains read hi + delta.
+#pragma unroll
+                        for (int i = 0; i < P; ++i) fold_word(ph[i], pl[i], pd[i]);
+#pragma unroll
+                        for (int g = 0; g < G; ++g) {
+                            fold_word(mh[g], ml[g], md[g]);
+                            if constexpr (PACK) {
+                                // packed fast two-sum (|hi| >= |delta| except while a word is
+                                // still near zero, where the lost error is second order)
+#pragma unroll
+                                for (int h = 0; h < D / 2; ++h) {
+                                    float2* hp = hi_top2 + (g * (D / 2) + h) * 32 + lane;
+                                    const float2 hi = HS ? *hp : make_float2(th[g][2 * h], th[g][2 * h + 1]);
+                                    const float2 dl = make_float2(td[g][2 * h], td[g][2 * h + 1]);
+                                    const float2 sm = __fadd2_rn(hi, dl);
+                                    const float2 z = __ffma2_rn(hi, make_float2(-1.f, -1.f), sm);
+                                    const float2 er = __ffma2_rn(z, make_float2(-1.f, -1.f), dl);
+                                    float2* lp = lo_top2 + (g * (D / 2) + h) * 32 + lane;
+                                    *lp = __fadd2_rn(*lp, er);
+                                    if constexpr (HS) {
+                                        *hp = sm;
+                                    } else {
+                                        th[g][2 * h] = sm.x;
+                                        th[g][2 * h + 1] = sm.y;
+                                    }
+                                    td[g][2 * h] = 0.f;
+                                    td[g][2 * h + 1] = 0.f;
+                                }
+                            } else {
+#pragma unroll
+                                for (int b = 0; b < D; ++b) {
+                                    float sh, e;
+                                    two_sum(th[g][b], td[g][b], sh, e);
+                                    th[g][b] = sh;
+                                    float* lp = lo_top + (g * D + b) * 32 + lane;
+                                    *lp = __fadd_rn(*lp, e);
+                                    td[g][b] = 0.f;
+                                }
                             }
                         }
                     }
                 }
-            }
             }
         }
 
@@ -716,14 +711,9 @@ signature_kernel_split(const SigArgs a)
             }
         }
 
-        int64_t start = a.offsets[s];
-        int64_t len = a.offsets[s + 1] - start;
-        if constexpr (SINGLE) {
-            if (a.ends) {
-                start = a.ends[2 * slot];
-                len = a.ends[2 * slot + 1] - start;
-            }
-        }
+        const bool by_ends = SINGLE && a.ends;
+        const int64_t start = by_ends ? a.ends[2 * slot] : a.offsets[s];
+        const int64_t len = (by_ends ? a.ends[2 * slot + 1] : a.offsets[s + 1]) - start;
         const float* __restrict__ xs = static_cast<const float*>(a.inc) + start * D;
 
         double ph[PP];
