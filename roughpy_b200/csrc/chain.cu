@@ -21,8 +21,10 @@
 // projection, on a 2^14-event float64 tree, against 1.06 ms here, where
 // shared-memory wavefronts (73 % busy) and issue (54 %) bound it, the
 // projection's gathers among them.  100000 such queries: 18.5 -> 14.0 ms with
-// the host's dissection, 13.0 with the device's; 20000 at (5,5), which did not fit the
-// registers, 4.9 -> 2.0 ms.
+// the host's dissection, 12.9 with the device's; 20000 at (5,5), which did not fit
+// the registers, 4.9 -> 2.0 ms.  Up to a few hundred queries are a chain or two
+// an SM, and there the registers were faster: 16 queries of 1024 events at (6,5),
+// with their host time, 50 -> 57 us in float64 and 47 -> 59 in float32.
 #include <algorithm>
 
 #include "row_units.cuh"

@@ -988,7 +988,8 @@ static bool rows_slower(int dtype, const Geometry& g, const ProductSpec& spec, i
 // Where the slab kernel beats the kernels below.  Measured on B200, slabs /
 // others: widths 5 and 7, which have no two-letter blocks, (5,7) x 500 float64
 // 299 / 333 us accumulating and 229 / 319 assigning, (7,6) float32 x 600 308 /
-// 528 us; width 8 float32, (8,6) x 1024 1000 / 1149 and 910 / 1074 us; width 4
+// 528 us; width 8 float32, (8,6) x 1024 in a row 1106 / 1159 us accumulating, and
+// 910 / 1074 assigning; width 4
 // assigning float64, (4,8) x 500 219 / 239 us.  Not: (8,6) float64 904 / 835 us
 // accumulating, (4,8) float32 407 / 351 us, accumulating float64 266 / 252 us.
 // A row is only `width` blocks, so few rows leave SMs idle: (8,6) float32 x 10

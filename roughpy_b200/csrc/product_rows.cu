@@ -241,10 +241,12 @@ product_rows_kernel(const RowArgs a)
 // are staged as float64 as before; L_p's part is as many words as level p - 1,
 // and in that place split_unit sees a product of depth N - 1.  Left over are
 // p = 1, whose right words R_{N-1}[a, rho] are one run, and the streamed ends.
-// Levels below N are a row-resident product of their own.   Measured on B200, (8,6)
-// float32 x 1024 accumulating 1149 -> 1000 us (4.9 TB/s); in place (8,6) float32
-// x 500 1.16 -> 0.47 ms.  What bounds it is the latency of the streamed words at
-// 27 warps an SM: 45 % DRAM, 43 % shared-memory pipe, 41 % issue.
+// Levels below N are a row-resident product of their own.  Measured on B200, (8,6)
+// float32 x 1024 accumulating, calls in a row: 1159 -> 1106 us, at the board's
+// power cap (SM clock 1965 -> 1665 MHz); in bursts of 20, 1006 us (4.9 TB/s).  In
+// place (8,6) float32 x 500 1.16 -> 0.47 ms.  What bounds it is the latency of the
+// streamed words at 27 warps an SM (64 registers a thread): 53 % DRAM, 47 % of the
+// shared-memory wavefronts, 37 % issue.
 template <typename T, typename TR, bool ACCUM, int D>
 __global__ void __launch_bounds__(kRowThreads, 1)
 product_slab_kernel(const RowArgs a)

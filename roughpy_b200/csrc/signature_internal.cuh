@@ -20,8 +20,8 @@ int64_t signature_lanes_per_stream(int mode, int width, int depth, int g);
 // at least 4 bytes.
 int signature_launch(int mode, int width, int depth, int g_lane, int wpb, int64_t n_items,
                      const int64_t* offsets, const void* inc, void* out, int64_t ld_out,
-                     const int64_t* order, const int64_t* ends, const int64_t* dst_row, void* alt, int64_t ld_alt,
-                     int* queue, cudaStream_t s);
+                     const int64_t* order, const int64_t* ends, const int64_t* dst_row, void* alt,
+                     int64_t ld_alt, int* queue, cudaStream_t s);
 
 // Per-stream error report of float32 signatures `out32` against the float64
 // path on the same increments (rpyb_signature_batched's err_out).  ws must
