@@ -24,7 +24,10 @@
 // the host's dissection, 12.9 with the device's; 20000 at (5,5), which did not fit
 // the registers, 4.9 -> 2.0 ms.  Up to a few hundred queries are a chain or two
 // an SM, and there the registers were faster: 16 queries of 1024 events at (6,5),
-// with their host time, 50 -> 57 us in float64 and 47 -> 59 in float32.
+// with their host time, 49 -> 55 us in float64 and 46 -> 61 in float32, whose
+// factors have to be waited for and widened before a product.  (Holding the next
+// factor's words in registers across a product took 3 us off a few float32
+// queries and cost large batches 4 to 7 %.)
 #include <algorithm>
 
 #include "row_units.cuh"
@@ -196,22 +199,8 @@ chain_products_kernel(const ChainArgs a)
             asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();
             const double* X = fx;
-            // the next factor's lower levels: float64 by asynchronous copies;
-            // float32, which has to be widened, its first words through
-            // registers across this product, so that it does not begin with
-            // their latency ((8,3), 16 queries of 1024 events with their host
-            // time 28 -> 24 us; two words a thread, more would spill)
-            const TS* ahead = r + 1 < o1 ? src + a.rows[r + 1] * a.T : nullptr;
-            double* const ahead_room = x_room[(r - o0) & 1];
-            constexpr int kHeld = sizeof(TS) == 4 ? 2 : 0;
-            TS held[kHeld + 1];
-            if constexpr (kHeld == 0) {
-                if (ahead) fx = stage_words(ahead_room, ahead, TL, tid, B);
-            } else {
-#pragma unroll
-                for (int j = 0; j < kHeld; ++j)
-                    held[j] = ahead && tid + j * B < TL ? __ldg(ahead + tid + j * B) : TS(0);
-            }
+            if (r + 1 < o1)
+                fx = stage_words(x_room[(r - o0) & 1], src + a.rows[r + 1] * a.T, TL, tid, B);
             prefetch_top(r + 3);
             const TS* node = src + a.rows[r] * a.T;
             const double node0 = X[0], c0v = cur[0];
@@ -259,16 +248,6 @@ chain_products_kernel(const ChainArgs a)
                     }
             });
             if (tid == 0) nxt[0] = c0v * node0;
-            if constexpr (kHeld > 0) {
-                if (ahead) {
-#pragma unroll
-                    for (int j = 0; j < kHeld; ++j)
-                        if (tid + j * B < TL) ahead_room[tid + j * B] = (double)held[j];
-                    if (kHeld * B < TL)
-                        stage_words(ahead_room + kHeld * B, ahead + kHeld * B, TL - kHeld * B, tid, B);
-                    fx = ahead_room;
-                }
-            }
             double* t = cur;
             cur = nxt;
             nxt = t;
