@@ -33,6 +33,7 @@
 #include <algorithm>
 #include <initializer_list>
 #include <mutex>
+#include <set>
 #include <tuple>
 #include <map>
 #include <string>
@@ -1377,6 +1378,18 @@ int split_fold_chunks()
 
 namespace {
 
+// The shared-memory limit and carveout of a signature kernel.
+int prepare_kernel(SigKernel fn, size_t smem_warp)
+{
+    RPYB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)(smem_warp * kSigWarps)));
+    // the whole unified L1/shared array as shared memory: the kernels stage
+    // their state there and read global memory once per chunk
+    RPYB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                   (int)cudaSharedmemCarveoutMaxShared));
+    return RPYB_OK;
+}
+
 // One launch of a specialised signature kernel over n_items work streams
 // (streams, or the time segments of split streams).  `queue` is a zeroed-on-
 // launch device counter of the workspace.  wpb = 0 chooses the block size by
@@ -1420,14 +1433,7 @@ int launch_signature_variant(const SigVariant& v, const Geometry& g, int64_t n_i
         const auto key = std::make_tuple(dev, (const void*)v.fn, smem_warp, wpb);
         auto it = chosen.find(key);
         if (it == chosen.end()) {
-            for (const SigKernel fn : {v.fn, v.fn_single}) {
-                RPYB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)(smem_warp * kSigWarps)));
-                // the whole unified L1/shared array as shared memory: the kernels
-                // stage their state there and read global memory once per chunk
-                RPYB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                               (int)cudaSharedmemCarveoutMaxShared));
-            }
+            if (int rc = prepare_kernel(v.fn, smem_warp)) return rc;
             int best_wpb = wpb, best_per_sm = 0;
             if (wpb == 0) {
                 // warps are independent: the block size only matters for
@@ -1477,6 +1483,19 @@ int launch_signature_variant(const SigVariant& v, const Geometry& g, int64_t n_i
     blocks = std::min<int64_t>(blocks, (a.total_items + wpb - 1) / wpb);
     if (blocks < 1) blocks = 1;
     const bool single = a.total_items <= blocks * wpb;
+    if (single) {
+        // at the first use: a plan that never needs the kernel does not load it
+        static std::mutex mu;
+        static std::set<std::pair<int, const void*>> ready;
+        int dev = 0;
+        RPYB_CUDA(cudaGetDevice(&dev));
+        std::lock_guard<std::mutex> lk(mu);
+        const auto key = std::make_pair(dev, (const void*)v.fn_single);
+        if (!ready.count(key)) {
+            if (int rc = prepare_kernel(v.fn_single, smem_warp)) return rc;
+            ready.insert(key);
+        }
+    }
     if (!single) RPYB_CUDA(cudaMemsetAsync(queue, 0, sizeof(int), s));
     (single ? v.fn_single : v.fn)<<<(unsigned)blocks, wpb * 32, smem, s>>>(a);
     RPYB_CUDA(cudaGetLastError());
